@@ -94,7 +94,8 @@ int pdhg_restart(pdhg_ctx* ctx, int avg, double f);
 int pdhg_download(pdhg_ctx* ctx, int avg, double f, double* x, double* z);
 /* Gpu::name / Gpu::mem_used. name_out receives at most cap bytes (NUL-terminated). */
 int pdhg_info(pdhg_ctx* ctx, char* name_out, size_t cap, size_t* mem_used);
-/* Total kernels this context has launched (graph replays count their kernels). */
+/* Total kernels this context has launched: graph replays count their kernels, and a launch that takes a whole block of
+ * iterations, an evaluation or the power iteration counts the phases it takes. */
 int64_t pdhg_kernel_launches(const pdhg_ctx* ctx);
 const char* pdhg_last_error(const pdhg_ctx* ctx);
 void pdhg_destroy(pdhg_ctx* ctx);

@@ -27,7 +27,9 @@
 #include "../../include/taral_pdhg.h"
 #include "engine.hpp"
 #include "host.hpp"
+#include "cluster.cuh"
 #include "kernels.cuh"
+#include "resident.cuh"
 #include "scaling.cuh"
 
 namespace taral {
@@ -120,12 +122,14 @@ int forced_row_split() {
 
 std::vector<int4> build_row_blocks(const int64_t* ptr, int rows, int tile, int rows_max) {
     std::vector<int4> out;
-    auto close = [&](int r0, int r1) {  // y: rows | kUniformCandidate when no row is much longer than the mean
+    // y: rows | kUniformCandidate when no row is much longer than the mean | kLongRows when one exceeds kShort
+    auto close = [&](int r0, int r1) {
         int64_t mx = 0;
         for (int r = r0; r < r1; ++r) mx = std::max<int64_t>(mx, ptr[r + 1] - ptr[r]);
         const int64_t nz = ptr[r1] - ptr[r0], mean = (nz + (r1 - r0) - 1) / (r1 - r0);
         const bool uniform = r1 - r0 > 1 && mx > kShort && mx <= 2 * mean + 8;
-        out.push_back(make_int4(r0, (r1 - r0) | (uniform ? kUniformCandidate : 0), int(ptr[r0]), int(ptr[r1])));
+        out.push_back(make_int4(r0, (r1 - r0) | (uniform ? kUniformCandidate : 0) | (mx > kShort ? kLongRows : 0),
+                                int(ptr[r0]), int(ptr[r1])));
     };
     int start = 0, cur_rows = 0;
     int64_t cur_nnz = 0;
@@ -170,6 +174,9 @@ struct DevMat {
     int4* blk = nullptr;
     void* val = nullptr;
     int nblk = 0;
+    int4* rblk = nullptr;  // the blocks of the resident launches (resident.cuh): blk, or smaller ones
+    int rnblk = 0;
+    std::vector<int> hptr;  // host copy of ptr, until the set-up ends
 };
 
 template <class T>
@@ -232,6 +239,7 @@ struct Engine final : EngineBase {
         if (!blk.empty())
             CK(cudaMemcpyAsync(d.blk, blk.data(), blk.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
         d.val = upload(a.val, size_t(a.nnz));
+        d.hptr = std::move(p32);
         return d;
     }
 
@@ -338,6 +346,7 @@ struct Engine final : EngineBase {
             CK(cudaMemcpyAsync(d.blk, blk.data(), blk.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
         d.val = alloc<T>(size_t(d.nnz));
         CK(cudaStreamSynchronize(st));  // the host vectors may be released after return
+        d.hptr = std::move(p32);
         return d;
     }
     // Set-up from the column-wise model with the scaling on the device (scaling.cuh): the host builds the unscaled
@@ -425,18 +434,22 @@ struct Engine final : EngineBase {
         pv = zeros<T>(n), pw = zeros<T>(m), pu = zeros<T>(n);
         hbuf = alloc<double>(size_t(std::max(m, n)));
         d_in = alloc<double>(size_t(std::max(m, n)));
-        part = zeros<double>(size_t(296) * 5 * 2);
+        part = zeros<double>(size_t(kEvalCtas) * 5 * 4);
         out = zeros<double>(32);
         pst = zeros<double>(4);
         tickets = zeros<unsigned>(4);
         pdone = zeros<int>(1);
+        rbar = zeros<unsigned>(kBarrierStride + 1), rerr = zeros<int>(1);
         hc.assign(hc_ptr, hc_ptr + n), hrl.assign(hrl_ptr, hrl_ptr + m), hru.assign(hru_ptr, hru_ptr + m);
         h_out = static_cast<double*>(pinned_block());
         if (!h_out) throw CudaError{"cudaMallocHost: no pinned host memory for the status reads"};
         h_flag = reinterpret_cast<int*>(h_out + 32);
+        h_out[kResidentDone] = 0;
         CK(cudaStreamSynchronize(st));
         mem_used = alloc_bytes;
         tune();
+        choose_resident();
+        A.hptr = std::vector<int>(), AT.hptr = std::vector<int>();
     }
     ~Engine() override {
         if (ev0) cudaEventDestroy(ev0), cudaEventDestroy(ev1);
@@ -579,6 +592,109 @@ struct Engine final : EngineBase {
         spmv(AT, z, ATz);
     }
 
+    // ------------------------------------------------------------------ resident launches (resident.cuh)
+    static constexpr int kBarrierStride = 64;  // the two barrier counters and the ticket on lines of their own
+    unsigned* rbar = nullptr;
+    int* rerr = nullptr;
+    int resident_ctas = 0;  // CTAs of a resident launch, 0: the phase kernels
+    bool resident_iterates = false;  // iteration blocks too (every tile has a team of its own), not only evaluations
+    int cluster_ctas = 0;   // CTAs of the LP's cluster (cluster.cuh), 0: not on one cluster
+    size_t cluster_smem = 0;
+    ClusterLp<T>* d_lp = nullptr;
+    int rparity = 0;
+    void choose_resident() {
+        resident_ctas = 0, resident_iterates = false;
+        if (!use_graph || pdl || A.nblk == 0 || AT.nblk == 0) return;
+        int dev, sms, coop, mode = -1;
+        CK(cudaGetDevice(&dev));
+        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+        if (const char* e = std::getenv("TARAL_RESIDENT")) mode = std::atoi(e);
+        if (mode == 0 || !coop) return;
+        resident_blocks(A, sms), resident_blocks(AT, sms);
+        resident_ctas = std::min(sms, std::max(A.rnblk, AT.rnblk));
+        cluster_ctas = 0;
+        if (A.per_thread || AT.per_thread || tuned[0] == 2 || tuned[1] == 2) return;  // the tuner's choice for the phases
+        resident_iterates = mode >= 1 || std::max(A.rnblk, AT.rnblk) <= kTeams * sms;
+        if (mode == 1 || A.maxrow > kTile || AT.maxrow > kTile || m > kClusterRows || n > kClusterRows) return;
+        // One cluster where its time, about 1 us an iteration + 41 ns a KB of x and z + 40 ns a thousand nonzeros, is below
+        // the grid's 5 us. Measured (grid / cluster, us an iteration): planted 2,000 x 5,000 (25,000 nonzeros) FP32 5.4 /
+        // 3.6, FP64 4.9 / 4.2; 3,000 x 7,500 (37,500) FP32 5.4 / 4.3, FP64 5.1 / 5.9; 4,000 x 10,000 FP64 5.1 / 7.6.
+        const char* cl = std::getenv("TARAL_CLUSTER");
+        if (!cl && int64_t(m + n) * int64_t(sizeof(T)) + A.nnz > 90000) return;
+        for (int q = cl ? std::atoi(cl) : cluster_size(A.nnz); q <= kClusterMax; q *= 2) {
+            std::vector<int> plan;
+            const size_t need = cluster_plan<T>(A.hptr.data(), AT.hptr.data(), m, n, q, plan);
+            if (need > kClusterSmem) continue;
+            cluster_ctas = q, cluster_smem = need;
+            int* d_plan = alloc<int>(plan.size());
+            CK(cudaMemcpyAsync(d_plan, plan.data(), plan.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+            const ClusterLp<T> lp{A.ptr, A.idx, AT.ptr, AT.idx, static_cast<const T*>(A.val), static_cast<const T*>(AT.val),
+                                  m, n, x, z, Ax, ATz, xs, zs, c, l, u, rl, ru, par, d_plan, nullptr};
+            d_lp = alloc<ClusterLp<T>>(1);
+            CK(cudaMemcpyAsync(d_lp, &lp, sizeof lp, cudaMemcpyHostToDevice, st));
+            CK(cudaStreamSynchronize(st));
+            mem_used = alloc_bytes;
+            break;
+        }
+    }
+    // Row blocks for one tile per team where that is possible: the nonzeros spread over all teams (at least 256 a tile,
+    // one a thread), so that an SM's gathers, which L1 takes at about one sector a cycle, are as few as they can be.
+    void resident_blocks(DevMat& d, int sms) {
+        const int teams = sms * kTeams;
+        d.rblk = d.blk, d.rnblk = d.nblk;
+        if (d.nblk > teams) return;
+        const std::vector<int64_t> p(d.hptr.begin(), d.hptr.end());
+        std::vector<int4> list;
+        for (double grow = 1;; grow *= 1.1) {
+            const int tile = int(std::min<double>(kTile, std::max<double>(256, grow * double(d.nnz) / teams)));
+            const int rows = int(std::min<double>(kRowsMax, std::max<double>(64, grow * d.rows / teams)));
+            list = build_row_blocks(p.data(), d.rows, tile, rows);
+            if (int(list.size()) <= teams) break;
+            if (tile == kTile && rows == kRowsMax) return;
+        }
+        d.rblk = alloc<int4>(list.size()), d.rnblk = int(list.size());
+        CK(cudaMemcpyAsync(d.rblk, list.data(), list.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
+        CK(cudaStreamSynchronize(st));
+        mem_used = alloc_bytes;
+    }
+    ResidentArgs<T> resident_args(double* to) const {
+        auto mat = [](const DevMat& d) {
+            return ResidentMat<T>{d.ptr, d.idx, static_cast<const T*>(d.val), d.rblk, d.rnblk};
+        };
+        return {mat(A), mat(AT), m, n, x, z, Ax, ATz, xs, zs, c, l, u, rl, ru, Dr, Dc, xlast, zlast, par, tmp_m, tmp_n,
+                part, to, nullptr, nullptr, tickets + 3, rerr};
+    }
+    // `per_team`, `least`: bytes of shared memory per team and at least. The barrier counters alternate: a launch counts on one, which the
+    // launch before it has zeroed, and zeroes the other.
+    template <class... P, class... Args>
+    void launch_resident(void (*kernel)(const ResidentArgs<T>, P...), size_t per_team, size_t least, ResidentArgs<T> ra, Args... args) {
+        ra.bar = rbar + rparity * (kBarrierStride / 2), ra.other_bar = rbar + (1 - rparity) * (kBarrierStride / 2);
+        rparity = 1 - rparity;
+        const int blocks = std::max(A.rnblk, AT.rnblk);
+        const int teams = std::min(kTeams, (blocks + resident_ctas - 1) / resident_ctas);
+        const size_t smem = std::max(per_team * size_t(teams), least);
+        CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(unsigned(resident_ctas)), cfg.blockDim = dim3(unsigned(kThreads * teams));
+        cfg.dynamicSmemBytes = smem, cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        cfg.attrs = attr, cfg.numAttrs = 1;
+        CK(cudaLaunchKernelEx(&cfg, kernel, ra, static_cast<P>(args)...));
+    }
+    void check_resident() {  // after the synchronisation that waits for a launch writing to h_out
+        CK(cudaGetLastError());
+        const bool done = h_out[kResidentDone] == 1.0;
+        h_out[kResidentDone] = 0;
+        if (done) return;
+        CK(cudaMemsetAsync(rerr, 0, sizeof(int), st));
+        CK(cudaMemsetAsync(rbar, 0, (kBarrierStride + 1) * sizeof(unsigned), st));
+        CK(cudaMemsetAsync(tickets, 0, 4 * sizeof(unsigned), st));
+        throw CudaError{"resident kernel: a grid barrier timed out"};
+    }
+
     // ------------------------------------------------------------------ backend concept
     double power_norm(int iters) override {
         std::vector<double> h(n);
@@ -590,6 +706,20 @@ struct Engine final : EngineBase {
         CK(cudaMemsetAsync(pst, 0, 4 * sizeof(double), st));
         CK(cudaMemsetAsync(pdone, 0, sizeof(int), st));
         launches += 1;
+        if (cluster_ctas > 0) {
+            CK(launch_cluster(k_cluster_power<T, true>, k_cluster_power<T, false>, d_lp, 1, cluster_ctas, cluster_smem, st, iters, pv, h_out));
+            CK(cudaStreamSynchronize(st));
+            launches += 2 * int64_t(h_out[1]);  // the products, as when each is a launch of its own
+            return h_out[0];
+        }
+        if (resident_ctas > 0) {
+            launch_resident(k_resident_power<T>, sizeof(RowSmem<T>), 0,
+                            resident_args(h_out), pv, pw, iters, red_grid(n));
+            CK(cudaStreamSynchronize(st));
+            check_resident();
+            launches += 2 * int64_t(h_out[1]);  // the products, as when each is a launch of its own
+            return h_out[0];
+        }
         T *a = pv, *b = pu;
         // steps queued between checks of the device-side stop flag; an even count, so that every chunk starts with
         // the vectors in the same roles and a chunk captured once replays as a CUDA graph
@@ -668,7 +798,14 @@ struct Engine final : EngineBase {
     }
     void iterate(int steps) override {
         if (steps <= 0) return;
-        if (use_graph && steps == eval_freq) {
+        if (cluster_ctas > 0) {
+            CK(launch_cluster(k_cluster_iterate<T, true>, k_cluster_iterate<T, false>, d_lp, 1, cluster_ctas, cluster_smem, st, steps));
+            launches += 1 + 2 * int64_t(steps);  // the phases, as when each is a launch of its own
+        } else if (resident_iterates) {
+            launch_resident(k_resident_iterate<T>, sizeof(RowSmem<T>), 0,
+                            resident_args(out), steps);
+            launches += 1 + 2 * int64_t(steps);  // the phases, as when each is a launch of its own
+        } else if (use_graph && steps == eval_freq) {
             if (!graph) {
                 cudaGraph_t g;
                 int64_t before = launches;
@@ -710,11 +847,18 @@ struct Engine final : EngineBase {
         std::memcpy(o10, h_out, 10 * sizeof(double));
     }
     void eval_pair(double f, double* cur, double* avg) override {
-        queue_eval(false, 1.0, out);
-        queue_eval(true, f, out + 10);
-        CK(cudaMemcpyAsync(h_out, out, 20 * sizeof(double), cudaMemcpyDeviceToHost, st));
+        if (resident_ctas > 0) {  // the scalars go straight to the pinned status block
+            launch_resident(k_resident_eval<T>,
+                            sizeof(RowSmem<double>), 20 * kEvalCtas * sizeof(double), resident_args(h_out), f, red_grid(m), red_grid(n));
+            launches += 6;  // the phases, as when each is a launch of its own
+        } else {
+            queue_eval(false, 1.0, out);
+            queue_eval(true, f, out + 10);
+            CK(cudaMemcpyAsync(h_out, out, 20 * sizeof(double), cudaMemcpyDeviceToHost, st));
+        }
         CK(cudaStreamSynchronize(st));
         CK(cudaGetLastError());
+        if (resident_ctas > 0) check_resident();
         std::memcpy(cur, h_out, 10 * sizeof(double));
         std::memcpy(avg, h_out + 10, 10 * sizeof(double));
     }
@@ -726,6 +870,12 @@ struct Engine final : EngineBase {
         CK(cudaGetLastError());
     }
     void download(bool avg, double f, double* hx, double* hz) override {
+        if (resident_ctas > 0) {  // a block whose barrier gave up leaves no point to return
+            CK(cudaMemcpyAsync(h_flag, rerr, sizeof(int), cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
+            h_out[kResidentDone] = *h_flag ? 0 : 1;
+            check_resident();
+        }
         if (n) {
             if (avg) k_scale_out<double><<<grid_for(n), 256, 0, st>>>(n, f, xs, hbuf);
             else k_scale_out<T><<<grid_for(n), 256, 0, st>>>(n, 1.0, x, hbuf);

@@ -117,6 +117,17 @@ struct EpiStore {
     __device__ __forceinline__ void finish(int r, int, int, double s, Stage&) const { y[r] = Y(s); }
 };
 
+// The dual prox of one row: v - sigma lo where v / sigma < lo, v - sigma up where v / sigma > up, else 0. The FP64
+// division is a chain of some 390 cycles; v * (1 / sigma) is within 2 ulp of the quotient, so it decides both comparisons
+// unless a bound lies within 4 ulp of it (or the quotient is so small that an ulp is no longer relative): only then is
+// the division done, and the result is the same bits either way. NaN takes the last case both ways.
+__device__ __forceinline__ double dual_prox(double v, double lo, double up, double sigma, double inv_sigma) {
+    double q = v * inv_sigma;
+    const double near = 1e-15 * fabs(q);
+    if (fabs(q - lo) <= near || fabs(q - up) <= near || !(fabs(q) >= 1e-280)) q = v / sigma;
+    return q < lo ? v - sigma * lo : (q > up ? v - sigma * up : 0.0);
+}
+
 // Dual step of one row (gpu/pdhg.cu:178-190 semantics, running sum of z in FP64):
 //   v = z + sigma (2 s - Ax_old);  z = prox: v - sigma*rl if v/sigma < rl, v - sigma*ru if v/sigma > ru, else 0;
 //   Ax_old = s;  zs += z.
@@ -217,6 +228,8 @@ constexpr int kSeg = 8;
 // kMidGroups -- rows of kShort + 1 .. kMid nonzeros are summed by groups of kGroup lanes (four rows per warp, lanes
 //               strided by kGroup, a three-level shuffle tree) instead of a whole warp each. Set by the autotuner.
 constexpr int kMidGroups = 1 << 19;
+// kLongRows -- some row of the block exceeds kShort (build_row_blocks).
+constexpr int kLongRows = 1 << 20;
 constexpr int kMid = 128;
 constexpr int kGroup = 8;
 constexpr int kPolicies = 5;  // row-split policies the autotuners choose from (0 = the hybrid rule)
@@ -625,14 +638,12 @@ __device__ __forceinline__ double row_rel_weight(double lo, double up, double dr
     return 1.0 / (1.0 + b / dr);
 }
 
-// Row part of the KKT evaluation (gpu/pdhg.cu:236-251): out = {PR2S, PR2O, PR2R, DROW, DZ2}.
+// Row part of the KKT evaluation (gpu/pdhg.cu:236-251): v += {PR2S, PR2O, PR2R, DROW, DZ2} over the rows i, i + G,
+// i + 2G, ... below m, in that order (G = the grid's threads); the loads of kEvalBatch rows are issued before their
+// sums, which keep the same order.
 template <class T, class V>
-__global__ void __launch_bounds__(kRedThreads) k_eval_row(int m, double f, const V* __restrict__ Ax,
-                                                          const V* __restrict__ z, const T* __restrict__ rl,
-                                                          const T* __restrict__ ru, const T* __restrict__ Dr,
-                                                          const T* __restrict__ zlast, double* part,
-                                                          unsigned* ticket, double* out) {
-    double v[5] = {0, 0, 0, 0, 0};
+__device__ __forceinline__ void eval_rows(double (&v)[5], int i, int G, int m, double f, const V* Ax, const V* z,
+                                          const T* rl, const T* ru, const T* Dr, const T* zlast) {
     auto add = [&](double ax, double zz, double lo, double up, double dr, double zl) {
         ax *= f, zz *= f;
         double r = ax < lo ? lo - ax : (ax > up ? ax - up : 0), ro = r / dr;
@@ -643,10 +654,6 @@ __global__ void __launch_bounds__(kRedThreads) k_eval_row(int m, double f, const
         double dz = zz - zl;
         v[4] += dz * dz;
     };
-    // each thread takes rows i, i + G, i + 2G, ... (G = the grid's threads) in that order; the loads of kEvalBatch
-    // rows are issued before their sums, which keep the same order
-    const int G = gridDim.x * blockDim.x;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
     for (; i + (kEvalBatch - 1) * G < m; i += kEvalBatch * G) {
         double a[kEvalBatch], zz[kEvalBatch], lo[kEvalBatch], up[kEvalBatch], dr[kEvalBatch], zl[kEvalBatch];
 #pragma unroll
@@ -659,17 +666,22 @@ __global__ void __launch_bounds__(kRedThreads) k_eval_row(int m, double f, const
         for (int e = 0; e < kEvalBatch; ++e) add(a[e], zz[e], lo[e], up[e], dr[e], zl[e]);
     }
     for (; i < m; i += G) add(double(Ax[i]), double(z[i]), rl[i], ru[i], double(Dr[i]), double(zlast[i]));
+}
+template <class T, class V>
+__global__ void __launch_bounds__(kRedThreads) k_eval_row(int m, double f, const V* __restrict__ Ax,
+                                                          const V* __restrict__ z, const T* __restrict__ rl,
+                                                          const T* __restrict__ ru, const T* __restrict__ Dr,
+                                                          const T* __restrict__ zlast, double* part,
+                                                          unsigned* ticket, double* out) {
+    double v[5] = {0, 0, 0, 0, 0};
+    eval_rows(v, int(blockIdx.x * blockDim.x + threadIdx.x), int(gridDim.x * blockDim.x), m, f, Ax, z, rl, ru, Dr, zlast);
     reduce_finish<5>(v, part, ticket, out);
 }
 
-// Column part (gpu/pdhg.cu:253-271): out = {DR2S, DR2O, POBJ, DCOL, DX2}.
+// Column part (gpu/pdhg.cu:253-271): v += {DR2S, DR2O, POBJ, DCOL, DX2}, in the order of eval_rows.
 template <class T, class V>
-__global__ void __launch_bounds__(kRedThreads) k_eval_col(int n, double f, const V* __restrict__ x,
-                                                          const V* __restrict__ ATz, const T* __restrict__ c,
-                                                          const T* __restrict__ l, const T* __restrict__ u,
-                                                          const T* __restrict__ Dc, const T* __restrict__ xlast,
-                                                          double* part, unsigned* ticket, double* out) {
-    double v[5] = {0, 0, 0, 0, 0};
+__device__ __forceinline__ void eval_cols(double (&v)[5], int j, int G, int n, double f, const V* x, const V* ATz,
+                                          const T* c, const T* l, const T* u, const T* Dc, const T* xlast) {
     auto add = [&](double xx, double cj, double atz, double lo, double up, double dc, double xl) {
         xx *= f;
         double d = cj + atz * f, res = 0;
@@ -684,8 +696,6 @@ __global__ void __launch_bounds__(kRedThreads) k_eval_col(int n, double f, const
         double ro = res / dc, dx = xx - xl;
         v[0] += res * res, v[1] += ro * ro, v[4] += dx * dx;
     };
-    const int G = gridDim.x * blockDim.x;  // columns j, j + G, ... in that order, loads batched as in k_eval_row
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
     for (; j + (kEvalBatch - 1) * G < n; j += kEvalBatch * G) {
         double xx[kEvalBatch], cj[kEvalBatch], atz[kEvalBatch], lo[kEvalBatch], up[kEvalBatch], dc[kEvalBatch],
             xl[kEvalBatch];
@@ -699,6 +709,15 @@ __global__ void __launch_bounds__(kRedThreads) k_eval_col(int n, double f, const
         for (int e = 0; e < kEvalBatch; ++e) add(xx[e], cj[e], atz[e], lo[e], up[e], dc[e], xl[e]);
     }
     for (; j < n; j += G) add(double(x[j]), c[j], double(ATz[j]), l[j], u[j], double(Dc[j]), double(xlast[j]));
+}
+template <class T, class V>
+__global__ void __launch_bounds__(kRedThreads) k_eval_col(int n, double f, const V* __restrict__ x,
+                                                          const V* __restrict__ ATz, const T* __restrict__ c,
+                                                          const T* __restrict__ l, const T* __restrict__ u,
+                                                          const T* __restrict__ Dc, const T* __restrict__ xlast,
+                                                          double* part, unsigned* ticket, double* out) {
+    double v[5] = {0, 0, 0, 0, 0};
+    eval_cols(v, int(blockIdx.x * blockDim.x + threadIdx.x), int(gridDim.x * blockDim.x), n, f, x, ATz, c, l, u, Dc, xlast);
     reduce_finish<5>(v, part, ticket, out);
 }
 

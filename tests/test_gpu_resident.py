@@ -1,0 +1,52 @@
+"""Launches that take a whole block of iterations, an evaluation or the power iteration (csrc/resident.cuh: a
+cooperative grid; csrc/cluster.cuh: one thread-block cluster, the LP in its shared memory) against the phase kernels they
+stand for: the same products summed in the same order, so every number is the same bit for bit. TARAL_RESIDENT forces
+a form: 0 phase kernels, 1 the grid; TARAL_CLUSTER the smallest cluster (the LP's data may ask for a larger one)."""
+import numpy as np
+import pytest
+
+import lpgen
+import pdhg
+
+pytestmark = pytest.mark.gpu
+
+CASES = {
+    "one_row": lambda: lpgen.packing(2, seed=1),                     # one row block each, mostly idle teams
+    "general_300x700": lambda: lpgen.general(300, 700, seed=3),      # every row and bound kind, empty rows
+    "packing_2000": lambda: lpgen.packing(2000, seed=3),             # several blocks, short rows
+    "zipf_rows_over_a_tile": lambda: lpgen.planted(3000, 8000, 8, seed=5, zipf=1.1, cap=3000, floor=1),
+    "refinery_2": lambda: lpgen.RefineryBase(2, seed=5).instance(2, lpgen.perturbations(1, 3)[0]),  # rows of 49-112
+    "planted_90k": lambda: lpgen.planted(30_000, 90_000, 12, seed=2),  # more blocks than teams: several tiles a team
+}
+
+
+def _record(lp, precision):
+    e = pdhg.Engine.from_model(lp, precision=precision)
+    norm = e.power_norm(200)
+    e.set_steps(0.7 / norm, 0.9 / norm)
+    e.start()
+    out = [np.array([norm])]
+    for steps, restart in ((64, True), (64, False), (7, None)):  # the last block is not of the evaluation length
+        e.iterate(steps)
+        out += list(e.eval_pair(1.0 / steps))
+        if restart is not None:
+            e.restart(restart, 1.0 / steps)
+    out += [v for avg in (0, 1) for v in e.download(avg, 1.0 / 7)]
+    r, x, z = e.solve(e.bnorm, e.cnorm, tol=1e-6, max_iter=640)
+    e.close()
+    return out + [x, z, np.array([r["iterations"], r["restarts"], r["rel_primal"], r["rel_dual"], r["rel_gap"]])]
+
+
+@pytest.mark.parametrize("precision", [pdhg.FP64, pdhg.FP32], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_resident_launches_change_nothing(engine_lib, monkeypatch, case, precision):
+    lp = CASES[case]()
+    monkeypatch.setenv("TARAL_TUNE", "0")  # both sides on the default row split
+    got = {}
+    for mode, cluster in (("0", "1"), ("1", "1"), ("2", "1"), ("2", "4"), ("2", "16")):
+        monkeypatch.setenv("TARAL_RESIDENT", mode)
+        monkeypatch.setenv("TARAL_CLUSTER", cluster)
+        got[mode + cluster] = _record(lp, precision)
+    for mode in got:
+        for k, (a, b) in enumerate(zip(got["01"], got[mode])):
+            assert np.array_equal(a, b, equal_nan=True), (mode, k, np.max(np.abs(a - b)))
