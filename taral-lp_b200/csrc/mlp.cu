@@ -8,12 +8,17 @@
 //
 // GEMMs: for every layer whose input width is a multiple of 8 (and whose dZ rows are 16-byte multiples: the output
 // gradient of the last layer is stored with its row stride rounded up to 8) all three GEMMs run on the tcgen05 tensor
-// cores through TMA (mlp_tc.cu, gemm_umma): the forward C = H Wt^T with Wt = W^T kept as a bf16 [out][in] copy
-// refreshed whenever the weights change (both operands K-major), dW = H_prev^T dZ (both operands read MN-major) and
-// dH_prev = dZ W^T (dZ K-major, Wt MN-major, K split into slices summed in order). Any other layer uses mma.sync
-// m16n8k16 (bf16 x bf16 -> f32), 128 x 128 x 32 CTA tiles, 8 warps of 64 x 32, operands staged in shared memory and
-// fed with ldmatrix; A may be stored transposed (TA: A = X^T) and B as [N][K] (TB: B = W^T); split-K writes per-slice
-// partials that a second kernel adds in slice order (deterministic).
+// cores through TMA (mlp_tc.cu) from one bf16 copy of W, its rows padded to 8 elements: the forward C = H W (W read
+// MN-major) with bias and activation in its epilogue, dH_prev = dZ W^T (W K-major, K split into slices summed in
+// order) and dW = H_prev^T dZ (both operands MN-major), which in training ends in the Adam step itself, so that the
+// weight gradient never reaches memory. Any other layer uses mma.sync m16n8k16 (bf16 x bf16 -> f32), 128 x 128 x 32 CTA
+// tiles, 8 warps of 64 x 32, operands staged in shared memory and fed with ldmatrix; A may be stored transposed (TA:
+// A = X^T) and B as [N][K] (TB: B = W^T); split-K writes per-slice partials that a second kernel adds in slice order
+// (deterministic).
+//
+// A training step at 64 x 132,001 outputs (68M weights) took 1.5 ms with separate kernels for the transposed copy, the
+// gathered targets, the residual, the column sums, the weight gradients and Adam, and a host synchronisation per step;
+// what bounds it is the 26 bytes per weight of Adam plus two reads of the bf16 copy.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -26,16 +31,22 @@
 #include <vector>
 
 #include "../../include/taral_pdhg.h"
+#include "mlp.cuh"
 
 namespace taral {
 namespace tc {
-int gemm_tc(int M, int N, int K, const void* A, const void* Bt, float* C, int* err, cudaStream_t stream);
+using mlp::AdamStep;
+using mlp::bf16;
+int gemm_partials(int M, int N, int K, const void* A, int lda, int a_mn, const void* B, int ldb, int b_mn, float* ws,
+                  int* slices, int* err, cudaStream_t stream);
+int gemm_layer(int M, int N, int K, const void* A, const void* W, int ldw, const float* b, float* Z, bf16* H, int* err,
+               cudaStream_t stream);
+int gemm_adam(int M, int N, int K, const void* A, int lda, const void* B, int ldb, float* W, float* m, float* v, bf16* Wb,
+              int ldw, const AdamStep& s, int* err, cudaStream_t stream);
 int gemm_umma(int M, int N, int K, const void* A, int lda, int a_mn, const void* B, int ldb, int b_mn, float* C,
               int ldc, int slices, float* ws, int* err, cudaStream_t stream);
 }
 namespace mlp {
-
-using bf16 = __nv_bfloat16;
 
 struct MlpError {
     std::string msg;
@@ -173,13 +184,6 @@ __global__ void k_splitk_sum(size_t count, int slices, const float* __restrict__
     }
 }
 
-__device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_grad(float z) {
-    const float cdf = 0.5f * (1.f + erff(z * 0.70710678118654752f));
-    const float pdf = 0.39894228040143268f * expf(-0.5f * z * z);
-    return cdf + z * pdf;
-}
-
 // Z = C + b; H = bf16(gelu(Z)) (act) or Y = Z (no act, H may be NULL).
 __global__ void k_bias_act(int rows, int cols, const float* __restrict__ C, const float* __restrict__ b,
                            float* __restrict__ Z, bf16* __restrict__ H, int act) {
@@ -191,93 +195,140 @@ __global__ void k_bias_act(int rows, int cols, const float* __restrict__ C, cons
     }
 }
 
-// R = Y - T (FP32), dY = bf16(2 R / (rows * cols)); per-row partial sums of R^2 into part[row].
-__global__ void k_loss_grad(int rows, int cols, int ldy, const float* __restrict__ Y, const float* __restrict__ T,
-                            float* __restrict__ R, bf16* __restrict__ dY, double* __restrict__ part) {
-    const int row = blockIdx.x;
+// A bias vector's Adam step, taken where its gradient is formed (b NULL: the gradient only).
+struct BiasStep {
+    float *b, *m, *v;
+    AdamStep s;
+};
+__device__ __forceinline__ void bias_step(const BiasStep& t, int j, float g, float* db) {
+    db[j] = g;
+    if (t.b) adam_step(t.s, g, t.b[j], t.m[j], t.v[j]);
+}
+
+// A CTA takes COLS columns: threads (x, y) = (column, row modulo blockDim / COLS), rows in chunks of kRowChunk. grad(r)
+// is the gradient at row r of the thread's column, formed by the thread that owns the entry; the columns are then summed
+// in row order by one thread each from shared memory (column_smem bytes), as a loop over the rows would, without reading
+// the gradients back from memory.
+constexpr int kRowChunk = 256;
+constexpr int kLossCols = 32, kHiddenCols = 16;
+inline size_t column_smem(int rows, int cols) { return size_t(std::min(rows, kRowChunk)) * size_t(cols + 1) * sizeof(float); }
+template <int COLS, class Grad>
+__device__ __forceinline__ float column_sums(int rows, bool in, float* sh, Grad grad) {
+    const int tx = threadIdx.x % COLS, ty = threadIdx.x / COLS, step = blockDim.x / COLS;
+    float sum = 0.f;
+    for (int r0 = 0; r0 < rows; r0 += kRowChunk) {
+        const int n = min(kRowChunk, rows - r0);
+        if (in) {
+#pragma unroll 4
+            for (int r = ty; r < n; r += step) sh[r * (COLS + 1) + tx] = grad(r0 + r);
+        }
+        __syncthreads();
+        if (ty == 0 && in) {
+#pragma unroll 8
+            for (int r = 0; r < n; ++r) sum += sh[r * (COLS + 1) + tx];
+        }
+        __syncthreads();
+    }
+    return sum;  // in the threads with y = 0
+}
+
+// The output gradient: with r = Y - T, G = 2 r / (rows cols): dY = bf16(G), db = column sums of G, and the CTA's sum of
+// r^2 in part[CTA]. idx: the row of T that belongs to row r (NULL: r itself).
+__global__ void __launch_bounds__(256) k_loss_grad(int rows, int cols, int ldy, const float* __restrict__ Y,
+                                                   const float* __restrict__ T, const int* __restrict__ idx,
+                                                   bf16* __restrict__ dY, float* __restrict__ db, BiasStep bias,
+                                                   double* __restrict__ part) {
+    extern __shared__ float sh[];
+    __shared__ double warps[8];
+    const int j = blockIdx.x * kLossCols + threadIdx.x % kLossCols;
     const float scale = 2.f / (float(rows) * float(cols));
     double s = 0;
-    for (int j = threadIdx.x; j < cols; j += blockDim.x) {
-        const size_t i = size_t(row) * cols + j;
-        const float r = Y[i] - T[i];
-        R[i] = r * scale;
-        dY[size_t(row) * ldy + j] = __float2bfloat16(r * scale);  // row stride ldy >= cols (padded for TMA)
-        s += double(r) * double(r);
-    }
+    const float g = column_sums<kLossCols>(rows, j < cols, sh, [&](int r) {
+        const size_t t = size_t(idx ? __ldg(idx + r) : r) * cols + j;
+        const float e = __ldg(Y + size_t(r) * cols + j) - __ldg(T + t);
+        dY[size_t(r) * ldy + j] = __float2bfloat16(e * scale);  // row stride ldy >= cols (padded for TMA)
+        s += double(e) * double(e);
+        return e * scale;
+    });
+    if (threadIdx.x < kLossCols && j < cols) bias_step(bias, j, g, db);
     for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-    __shared__ double sh[32];
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+    if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = s;
     __syncthreads();
     if (threadIdx.x == 0) {
         double t = 0;
-        for (int w = 0; w < int(blockDim.x >> 5); ++w) t += sh[w];
-        part[row] = t;
+        for (int w = 0; w < 8; ++w) t += warps[w];
+        part[blockIdx.x] = t;
     }
 }
 
-// db[j] = sum over rows of G[r][j] (fixed order).
-__global__ void k_colsum(int rows, int cols, const float* __restrict__ G, float* __restrict__ db) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < cols; j += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int r = 0; r < rows; ++r) s += G[size_t(r) * cols + j];
-        db[j] = s;
-    }
+// A hidden layer's gradient: dH = the sum of the slices of P in order, dZ = bf16(dH gelu'(Z)), db = column sums of
+// dH gelu'(Z). 1,024 threads on 16 columns: with 64 rows every thread has one entry, whose slices (74 behind the output
+// layer) are its whole latency.
+__global__ void __launch_bounds__(1024) k_hidden_grad(int rows, int cols, int slices, const float* __restrict__ P,
+                                                      const float* __restrict__ Z, bf16* __restrict__ dZ,
+                                                      float* __restrict__ db, BiasStep bias) {
+    extern __shared__ float sh[];
+    const int j = blockIdx.x * kHiddenCols + threadIdx.x % kHiddenCols;
+    const size_t count = size_t(rows) * cols;
+    const float g = column_sums<kHiddenCols>(rows, j < cols, sh, [&](int r) {
+        const size_t at = size_t(r) * cols + j;
+        const float z0 = __ldg(Z + at);
+        float d = 0.f;
+        int z = 0;
+        for (; z + 16 <= slices; z += 16) {
+            float p[16];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) p[e] = __ldg(P + size_t(z + e) * count + at);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) d += p[e];
+        }
+#pragma unroll 8
+        for (; z < slices; ++z) d += __ldg(P + size_t(z) * count + at);
+        const float e = d * gelu_grad(z0);
+        dZ[at] = __float2bfloat16(e);
+        return e;
+    });
+    if (threadIdx.x < kHiddenCols && j < cols) bias_step(bias, j, g, db);
 }
 
-// dZ = dH * gelu'(Z): FP32 copy (for db) and bf16 copy (GEMM operand).
-__global__ void k_gelu_back(size_t n, const float* __restrict__ dH, const float* __restrict__ Z, float* __restrict__ dZf,
-                            bf16* __restrict__ dZ) {
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-        const float g = dH[i] * gelu_grad(Z[i]);
-        dZf[i] = g;
-        dZ[i] = __float2bfloat16(g);
-    }
-}
 
 __global__ void k_to_bf16(size_t n, const float* __restrict__ src, bf16* __restrict__ dst) {
     for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
         dst[i] = __float2bfloat16(src[i]);
 }
 
-// Adam on FP32 masters; refreshes the bf16 copy.
-__global__ void k_adam(size_t n, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m1,
-                       float* __restrict__ m2, bf16* __restrict__ wb, float lr, float b1, float b2, float eps, float c1,
-                       float c2) {
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-        const float gi = g[i];
-        const float a = b1 * m1[i] + (1.f - b1) * gi, v = b2 * m2[i] + (1.f - b2) * gi * gi;
-        m1[i] = a, m2[i] = v;
-        const float wi = w[i] - lr * (a / c1) / (sqrtf(v / c2) + eps);
-        w[i] = wi;
-        if (wb) wb[i] = __float2bfloat16(wi);
-    }
+// Adam on row-major FP32 masters with a stored gradient, for a layer whose dW runs on mma.sync; refreshes the bf16 copy
+// (row stride ldb).
+__global__ void k_adam(int rows, int cols, int ldb, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
+                       float* __restrict__ v, bf16* __restrict__ wb, AdamStep s) {
+    for (int r = blockIdx.y; r < rows; r += gridDim.y)
+        for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < cols; j += gridDim.x * blockDim.x) {
+            const size_t at = size_t(r) * cols + j;
+            adam_step(s, g[at], w[at], m[at], v[at]);
+            wb[size_t(r) * ldb + j] = __float2bfloat16(w[at]);
+        }
 }
 
-// Wt[c][r] = W[r][c] for W rows x cols (bf16), through a 32 x 32 shared-memory tile.
-__global__ void k_transpose(int rows, int cols, const bf16* __restrict__ W, bf16* __restrict__ Wt) {
-    __shared__ bf16 t[32][33];
-    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int i = ty; i < 32; i += 8) {
-        const int r = r0 + i, c = c0 + tx;
-        if (r < rows && c < cols) t[i][tx] = W[size_t(r) * cols + c];
-    }
-    __syncthreads();
-    for (int i = ty; i < 32; i += 8) {
-        const int c = c0 + i, r = r0 + tx;
-        if (r < rows && c < cols) Wt[size_t(c) * rows + r] = t[tx][i];
-    }
+// Row-major P (rows x cols) into the masters W (blocked or row-major) and their bf16 copy, and back.
+__global__ void k_set_weights(int rows, int cols, int groups, int ldb, const float* __restrict__ P, float* __restrict__ W,
+                              bf16* __restrict__ wb) {
+    for (int r = blockIdx.y; r < rows; r += gridDim.y)
+        for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < cols; j += gridDim.x * blockDim.x) {
+            const float w = P[size_t(r) * cols + j];
+            W[groups ? blocked_at(r, j, groups) : size_t(r) * cols + j] = w;
+            wb[size_t(r) * ldb + j] = __float2bfloat16(w);
+        }
+}
+__global__ void k_get_weights(int rows, int cols, int groups, const float* __restrict__ W, float* __restrict__ P) {
+    for (int r = blockIdx.y; r < rows; r += gridDim.y)
+        for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < cols; j += gridDim.x * blockDim.x)
+            P[size_t(r) * cols + j] = W[blocked_at(r, j, groups)];
 }
 
-// Gather dataset rows idx[0..rows) into contiguous batch buffers.
-__global__ void k_gather_rows(int rows, int cols, const int* __restrict__ idx, const float* __restrict__ src,
-                              float* __restrict__ dst, bf16* __restrict__ dstb) {
-    const size_t n = size_t(rows) * cols;
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-        const size_t r = i / cols, c = i % cols;
-        const float v = src[size_t(idx[r]) * cols + c];
-        if (dst) dst[i] = v;
-        if (dstb) dstb[i] = __float2bfloat16(v);
-    }
+// The dataset rows idx[0 .. rows) as bf16 operand rows.
+__global__ void k_gather_rows(int cols, const int* __restrict__ idx, const float* __restrict__ src, bf16* __restrict__ dst) {
+    const float* from = src + size_t(idx[blockIdx.x]) * cols;
+    for (int c = threadIdx.x; c < cols; c += blockDim.x) dst[size_t(blockIdx.x) * cols + c] = __float2bfloat16(from[c]);
 }
 
 static int grid1(size_t n) { return int(std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 148 * 16))); }
@@ -286,8 +337,10 @@ struct Layer {
     int in = 0, out = 0;
     float *W = nullptr, *b = nullptr, *gW = nullptr, *gb = nullptr, *mW = nullptr, *vW = nullptr, *mb = nullptr,
           *vb = nullptr;
-    bf16* Wb = nullptr;
-    bf16* Wt = nullptr;  // W^T [out][in] (the tcgen05 forward GEMM's K-major B operand); null: forward on mma.sync
+    bf16* Wb = nullptr;   // W as bf16
+    int ldw = 0;          // row stride of Wb
+    bool tc = false;      // the GEMMs run on tcgen05 (ldw is out rounded up to 16), else on mma.sync (ldw = out)
+    bool fused = false;   // Adam in the epilogue of dW: W, mW, vW blocked (mlp.cuh), else row-major
     float* Z = nullptr;  // pre-activation [batch][out]
     bf16* H = nullptr;   // activation [batch][out] (GEMM operand of the next layer)
 };
@@ -296,11 +349,11 @@ struct Mlp {
     int in_dim = 0, hidden = 0, depth = 0, out_dim = 0, max_batch = 0;
     std::vector<Layer> L;
     bf16* Xb = nullptr;  // input batch
-    float *Xf = nullptr, *Tf = nullptr, *C = nullptr, *R = nullptr, *dHf = nullptr, *dZf = nullptr, *ws = nullptr;
-    bf16 *dYb = nullptr, *dZb = nullptr;
+    float *Xf = nullptr, *Tf = nullptr, *C = nullptr, *ws = nullptr;
+    bf16 *dYb = nullptr, *dZb[2] = {nullptr, nullptr};  // hidden layers' dZ, in turn
     int ldy = 0;  // row stride of dYb: the output width, rounded up to 8 when the last layer's backward runs on tcgen05
     double* part = nullptr;
-    int* d_idx = nullptr;
+    int* d_perm = nullptr;  // an epoch's order of the dataset
     int* d_err = nullptr;  // set by the tcgen05 GEMM when a completion wait gave up
     float *DX = nullptr, *DT = nullptr;  // dataset
     int dcount = 0;
@@ -331,10 +384,13 @@ struct Mlp {
         for (int l = 0; l <= depth; ++l) {
             Layer y;
             y.in = prev, y.out = l < depth ? hidden : out;
-            size_t nw = size_t(y.in) * y.out;
-            y.W = alloc<float>(nw), y.gW = alloc<float>(nw), y.mW = alloc<float>(nw), y.vW = alloc<float>(nw);
-            y.Wb = alloc<bf16>(nw);
-            if (y.in % 8 == 0) y.Wt = alloc<bf16>(nw);
+            y.tc = y.in % 8 == 0;
+            y.ldw = y.tc ? (y.out + 15) / 16 * 16 : y.out;
+            y.fused = y.tc && (l == depth || y.out % 8 == 0);
+            const size_t nw = y.fused ? blocked_size(y.in, y.out) : size_t(y.in) * y.out;
+            y.W = alloc<float>(nw), y.gW = alloc<float>(size_t(y.in) * y.out), y.mW = alloc<float>(nw), y.vW = alloc<float>(nw);
+            y.Wb = alloc<bf16>(size_t(y.in) * y.ldw);
+            MK(cudaMemsetAsync(y.W, 0, nw * sizeof(float), s));  // the padding of the blocks is updated along with them
             y.b = alloc<float>(y.out), y.gb = alloc<float>(y.out), y.mb = alloc<float>(y.out), y.vb = alloc<float>(y.out);
             y.Z = alloc<float>(size_t(mb) * y.out), y.H = alloc<bf16>(size_t(mb) * y.out);
             MK(cudaMemsetAsync(y.mW, 0, nw * sizeof(float), s));
@@ -346,10 +402,10 @@ struct Mlp {
         }
         size_t widest = std::max<size_t>(size_t(out), size_t(hid));
         Xb = alloc<bf16>(size_t(mb) * in), Xf = alloc<float>(size_t(mb) * in), Tf = alloc<float>(size_t(mb) * out);
-        ldy = L[depth].Wt ? (out + 7) / 8 * 8 : out;
-        C = alloc<float>(size_t(mb) * widest), R = alloc<float>(size_t(mb) * out), dYb = alloc<bf16>(size_t(mb) * ldy);
-        dHf = alloc<float>(size_t(mb) * widest), dZf = alloc<float>(size_t(mb) * hid), dZb = alloc<bf16>(size_t(mb) * hid);
-        part = alloc<double>(mb), d_idx = alloc<int>(mb), d_err = alloc<int>(1);
+        ldy = L[depth].tc ? (out + 7) / 8 * 8 : out;
+        C = alloc<float>(size_t(mb) * widest), dYb = alloc<bf16>(size_t(mb) * ldy);
+        for (bf16*& d : dZb) d = alloc<bf16>(size_t(mb) * hid);
+        part = alloc<double>(size_t(loss_ctas())), d_err = alloc<int>(1);
         MK(cudaMemsetAsync(d_err, 0, sizeof(int), s));
         ws_count = size_t(64) * mb * hid;  // split-K partials of dH = dZ W^T (K = out)
         ws = alloc<float>(ws_count);
@@ -379,14 +435,11 @@ struct Mlp {
         MK(cudaGetLastError());
     }
 
-    void refresh_transposes() {  // Wt = Wb^T for the layers whose forward GEMM runs on tcgen05
-        for (Layer& y : L)
-            if (y.Wt) {
-                dim3 grid((y.out + 31) / 32, (y.in + 31) / 32);
-                k_transpose<<<grid, 256, 0, s>>>(y.in, y.out, y.Wb, y.Wt);
-            }
-        MK(cudaGetLastError());
+    static dim3 grid2(const Layer& y) {  // kernels over the entries of a weight matrix
+        return dim3(unsigned(std::min(64, (y.out + 255) / 256)), unsigned(std::min(y.in, 592)));
     }
+
+    int loss_ctas() const { return (out_dim + kLossCols - 1) / kLossCols; }
 
     void check_tc() {  // after a stream synchronisation: did a tcgen05 GEMM give up waiting?
         int e = 0;
@@ -398,79 +451,83 @@ struct Mlp {
         }
     }
 
+    void tc_check(int rc) {
+        if (rc != TARAL_OK) throw MlpError{std::string("tcgen05 GEMM launch: ") + cudaGetErrorString(cudaGetLastError())};
+    }
+
     void forward(int batch) {  // Xb -> L[l].Z, L[l].H ; output Z of the last layer is Y
         const bf16* in = Xb;
         for (int l = 0; l <= depth; ++l) {
             Layer& y = L[l];
-            if (y.Wt) {
-                if (taral::tc::gemm_tc(batch, y.out, y.in, in, y.Wt, C, d_err, s) != TARAL_OK)
-                    throw MlpError{std::string("tcgen05 GEMM launch: ") + cudaGetErrorString(cudaGetLastError())};
+            if (y.tc) {
+                tc_check(taral::tc::gemm_layer(batch, y.out, y.in, in, y.Wb, y.ldw, y.b, y.Z, l < depth ? y.H : nullptr, d_err, s));
             } else {
                 gemm<false, false>(batch, y.out, y.in, in, y.Wb, C);
+                k_bias_act<<<grid1(size_t(batch) * y.out), 256, 0, s>>>(batch, y.out, C, y.b, y.Z, l < depth ? y.H : nullptr,
+                                                                        l < depth ? 1 : 0);
             }
-            k_bias_act<<<grid1(size_t(batch) * y.out), 256, 0, s>>>(batch, y.out, C, y.b, y.Z, l < depth ? y.H : nullptr,
-                                                                    l < depth ? 1 : 0);
             in = y.H;
         }
         MK(cudaGetLastError());
     }
 
-    double backward(int batch) {  // needs forward(batch) and Tf; fills gW, gb; returns the loss
+    // Needs forward(batch); the target of row r is row idx[r] of T (idx NULL: r). step NULL: fills gW, gb. Otherwise the
+    // Adam step is taken on every layer: its dH_prev first, which reads the old weights.
+    void backward(int batch, const float* T, const int* idx, const AdamStep* step) {
+        auto bias = [&](Layer& y) { return step ? BiasStep{y.b, y.mb, y.vb, *step} : BiasStep{}; };
         Layer& top = L[depth];
-        k_loss_grad<<<batch, 256, 0, s>>>(batch, top.out, ldy, top.Z, Tf, R, dYb, part);
+        k_loss_grad<<<loss_ctas(), 256, column_smem(batch, kLossCols), s>>>(batch, top.out, ldy, top.Z, T, idx, dYb, top.gb, bias(top), part);
         const bf16* dZ = dYb;
-        const float* dZfl = R;
         int ldz = ldy;  // row stride of dZ
         for (int l = depth; l >= 0; --l) {
             Layer& y = L[l];
             const bf16* Hprev = l > 0 ? L[l - 1].H : Xb;
-            // tcgen05 when the operands fit TMA (16-byte rows): dW = H_prev^T dZ reads both operands MN-major,
-            // dH_prev = dZ W^T reads dZ K-major and W^T (kept as Wt [out][in]) MN-major; mma.sync otherwise
-            const bool tc = y.Wt && ldz % 8 == 0;
-            if (tc) {
-                if (taral::tc::gemm_umma(y.in, y.out, batch, Hprev, y.in, 1, dZ, ldz, 1, y.gW, y.out, 1, nullptr, d_err, s) !=
-                    TARAL_OK)
-                    throw MlpError{std::string("tcgen05 GEMM launch: ") + cudaGetErrorString(cudaGetLastError())};
-            } else {
-                gemm<true, false>(y.in, y.out, batch, Hprev, dZ, y.gW);              // dW = H_prev^T dZ
-            }
-            k_colsum<<<grid1(y.out), 256, 0, s>>>(batch, y.out, dZfl, y.gb);     // db = sum_b dZ
+            // tcgen05 when the operands fit TMA (16-byte rows): dH_prev = dZ W^T reads both operands K-major, dW = H_prev^T
+            // dZ both MN-major; mma.sync otherwise
+            const bool tc = y.tc && ldz % 8 == 0;
+            bf16* next = dZb[l & 1];
             if (l > 0) {
+                Layer& p = L[l - 1];
+                int slices;
+                const float* partials = ws;
                 if (tc) {
                     const int tiles = ((batch + 127) / 128) * ((y.in + 255) / 256);
                     const size_t per_slice = size_t(batch) * y.in;
-                    const int slices = int(std::max<size_t>(1, std::min<size_t>(std::max(1, 148 / tiles),
-                                                                                ws_count / per_slice)));
-                    if (taral::tc::gemm_umma(batch, y.in, y.out, dZ, ldz, 0, y.Wt, y.in, 1, dHf, y.in, slices, ws, d_err, s) !=
-                        TARAL_OK)
-                        throw MlpError{std::string("tcgen05 GEMM launch: ") + cudaGetErrorString(cudaGetLastError())};
+                    slices = int(std::max<size_t>(1, std::min<size_t>(std::max(1, 148 / tiles), ws_count / per_slice)));
+                    tc_check(taral::tc::gemm_partials(batch, y.in, y.out, dZ, ldz, 0, y.Wb, y.ldw, 0, ws, &slices, d_err, s));
                 } else {
-                    int slices = std::max(1, std::min(64, y.out / 2048));
-                    gemm<false, true>(batch, y.in, y.out, dZ, y.Wb, dHf, slices);    // dH_prev = dZ W^T
+                    gemm<false, true>(batch, y.in, y.out, dZ, y.Wb, C, std::max(1, std::min(64, y.out / 2048)));
+                    slices = 1, partials = C;
                 }
-                Layer& p = L[l - 1];
-                k_gelu_back<<<grid1(size_t(batch) * p.out), 256, 0, s>>>(size_t(batch) * p.out, dHf, p.Z, dZf, dZb);
-                dZ = dZb, dZfl = dZf, ldz = p.out;
+                k_hidden_grad<<<(p.out + kHiddenCols - 1) / kHiddenCols, 1024, column_smem(batch, kHiddenCols), s>>>(batch, p.out, slices, partials, p.Z, next, p.gb, bias(p));
             }
+            if (y.fused && step) {
+                tc_check(taral::tc::gemm_adam(y.in, y.out, batch, Hprev, y.in, dZ, ldz, y.W, y.mW, y.vW, y.Wb, y.ldw, *step, d_err, s));
+            } else {
+                if (tc) tc_check(taral::tc::gemm_umma(y.in, y.out, batch, Hprev, y.in, 1, dZ, ldz, 1, y.gW, y.out, 1, nullptr, d_err, s));
+                else gemm<true, false>(y.in, y.out, batch, Hprev, dZ, y.gW);  // dW = H_prev^T dZ
+                if (step) {
+                    k_adam<<<grid2(y), 256, 0, s>>>(y.in, y.out, y.ldw, y.W, y.gW, y.mW, y.vW, y.Wb, *step);
+                }
+            }
+            dZ = next, ldz = hidden;
         }
-        std::vector<double> h(batch);
-        MK(cudaMemcpyAsync(h.data(), part, batch * sizeof(double), cudaMemcpyDeviceToHost, s));
+        MK(cudaGetLastError());
+    }
+
+    double loss(int batch) {  // of the last backward(batch); synchronises
+        std::vector<double> h(static_cast<size_t>(loss_ctas()));
+        MK(cudaMemcpyAsync(h.data(), part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
         MK(cudaStreamSynchronize(s));
         double t = 0;
         for (double v : h) t += v;
-        return t / (double(batch) * top.out);
+        return t / (double(batch) * L[depth].out);
     }
 
-    void adam(float lr) {
+    AdamStep next_step(float lr) {
         ++steps;
-        const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-        float c1 = 1.f - std::pow(b1, float(steps)), c2 = 1.f - std::pow(b2, float(steps));
-        for (Layer& y : L) {
-            size_t nw = size_t(y.in) * y.out;
-            k_adam<<<grid1(nw), 256, 0, s>>>(nw, y.W, y.gW, y.mW, y.vW, y.Wb, lr, b1, b2, eps, c1, c2);
-            k_adam<<<grid1(y.out), 256, 0, s>>>(y.out, y.b, y.gb, y.mb, y.vb, nullptr, lr, b1, b2, eps, c1, c2);
-        }
-        refresh_transposes();
+        const float b1 = 0.9f, b2 = 0.999f;
+        return {lr, b1, b2, 1e-8f, 1.f - std::pow(b1, float(steps)), 1.f - std::pow(b2, float(steps))};
     }
 
     void load_input(int batch, const float* x_host) {
@@ -527,13 +584,13 @@ extern "C" int taral_mlp_set_params(taral_mlp* h, const float* params) {
         const float* p = params;
         for (auto& y : m.L) {
             size_t nw = size_t(y.in) * y.out;
-            MK(cudaMemcpyAsync(y.W, p, nw * sizeof(float), cudaMemcpyHostToDevice, m.s));
-            taral::mlp::k_to_bf16<<<taral::mlp::grid1(nw), 256, 0, m.s>>>(nw, y.W, y.Wb);
+            MK(cudaMemcpyAsync(y.gW, p, nw * sizeof(float), cudaMemcpyHostToDevice, m.s));  // gW: the row-major form
+            taral::mlp::k_set_weights<<<m.grid2(y), 256, 0, m.s>>>(y.in, y.out, y.fused ? taral::mlp::blocked_groups(y.out) : 0,
+                                                                   y.ldw, y.gW, y.W, y.Wb);
             p += nw;
             MK(cudaMemcpyAsync(y.b, p, y.out * sizeof(float), cudaMemcpyHostToDevice, m.s));
             p += y.out;
         }
-        m.refresh_transposes();
         MK(cudaStreamSynchronize(m.s));
     })
 }
@@ -545,7 +602,9 @@ extern "C" int taral_mlp_get_params(taral_mlp* h, float* params) {
         float* p = params;
         for (auto& y : m.L) {
             size_t nw = size_t(y.in) * y.out;
-            MK(cudaMemcpyAsync(p, y.W, nw * sizeof(float), cudaMemcpyDeviceToHost, m.s));
+            if (y.fused)
+                taral::mlp::k_get_weights<<<m.grid2(y), 256, 0, m.s>>>(y.in, y.out, taral::mlp::blocked_groups(y.out), y.W, y.gW);
+            MK(cudaMemcpyAsync(p, y.fused ? y.gW : y.W, nw * sizeof(float), cudaMemcpyDeviceToHost, m.s));
             p += nw;
             MK(cudaMemcpyAsync(p, y.b, y.out * sizeof(float), cudaMemcpyDeviceToHost, m.s));
             p += y.out;
@@ -574,7 +633,8 @@ extern "C" int taral_mlp_gradients(taral_mlp* h, int batch, const float* x, cons
         m.load_input(batch, x);
         MK(cudaMemcpyAsync(m.Tf, target, size_t(batch) * m.out_dim * sizeof(float), cudaMemcpyHostToDevice, m.s));
         m.forward(batch);
-        double l = m.backward(batch);
+        m.backward(batch, m.Tf, nullptr, nullptr);
+        const double l = m.loss(batch);
         m.check_tc();
         if (loss) *loss = l;
         if (grads) {
@@ -599,6 +659,7 @@ extern "C" int taral_mlp_set_dataset(taral_mlp* h, int count, const float* x, co
         m.DX = m.alloc<float>(size_t(count) * m.in_dim), m.DT = m.alloc<float>(size_t(count) * m.out_dim);
         MK(cudaMemcpyAsync(m.DX, x, size_t(count) * m.in_dim * sizeof(float), cudaMemcpyHostToDevice, m.s));
         MK(cudaMemcpyAsync(m.DT, target, size_t(count) * m.out_dim * sizeof(float), cudaMemcpyHostToDevice, m.s));
+        m.d_perm = m.alloc<int>(size_t(count));
         MK(cudaStreamSynchronize(m.s));
         m.dcount = count;
     })
@@ -616,17 +677,15 @@ extern "C" int taral_mlp_train(taral_mlp* h, int epochs, int batch, float lr, ui
         for (int e = 0; e < epochs; ++e) {
             for (int i = 0; i < m.dcount; ++i) perm[i] = i;
             std::shuffle(perm.begin(), perm.end(), rng);
+            MK(cudaMemcpyAsync(m.d_perm, perm.data(), perm.size() * sizeof(int), cudaMemcpyHostToDevice, m.s));
             for (int b0 = 0; b0 + batch <= m.dcount; b0 += batch) {
-                MK(cudaMemcpyAsync(m.d_idx, perm.data() + b0, batch * sizeof(int), cudaMemcpyHostToDevice, m.s));
-                taral::mlp::k_gather_rows<<<taral::mlp::grid1(size_t(batch) * m.in_dim), 256, 0, m.s>>>(
-                    batch, m.in_dim, m.d_idx, m.DX, m.Xf, m.Xb);
-                taral::mlp::k_gather_rows<<<taral::mlp::grid1(size_t(batch) * m.out_dim), 256, 0, m.s>>>(
-                    batch, m.out_dim, m.d_idx, m.DT, m.Tf, nullptr);
+                taral::mlp::k_gather_rows<<<batch, 128, 0, m.s>>>(m.in_dim, m.d_perm + b0, m.DX, m.Xb);
                 m.forward(batch);
-                loss = m.backward(batch);
-                m.adam(lr);
+                const taral::mlp::AdamStep step = m.next_step(lr);
+                m.backward(batch, m.DT, m.d_perm + b0, &step);
             }
         }
+        loss = m.loss(batch);  // the last step's
         m.check_tc();
         if (last_loss) *last_loss = loss;
     })

@@ -65,3 +65,39 @@ def test_mlp_training_reduces_loss(engine_lib):
     net.set_dataset(x, t)
     last = net.train(epochs=40, batch=64, lr=2e-3, seed=1)
     assert last < 0.1 * l0, (l0, last)
+
+
+@pytest.mark.parametrize("dims,batch", [
+    ((256, 64, 2, 901), 16),   # tcgen05 throughout, ragged output width
+    ((24, 40, 1, 33), 130),    # more rows than one tile, widths below a tile
+    ((20, 24, 1, 50), 8),      # input width not a multiple of 8: the first layer on mma.sync
+    ((16, 12, 2, 70), 9),      # hidden width not a multiple of 8: products on both paths in one network
+    ((16, 16, 1, 40), 300),    # rows in more than one chunk of the column sums
+])
+def test_mlp_training_step_is_adam_on_the_gradients(engine_lib, dims, batch):
+    """Every step of train() on one batch moves each parameter by Adam's step on what gradients() reports for it. The
+    weights' gradients come from the same products, so the difference is rounding: a few ulp of the step, and the bias
+    corrections 1 - b^t formed in FP32 (an ulp of 0.999^t is 6e-5 of 1 - 0.999^t, 3e-5 of the step), plus an ulp of the
+    parameter."""
+    net = pdhg.Mlp(*dims, max_batch=batch)
+    net.init(3)
+    rng = np.random.default_rng(4)
+    x = rng.standard_normal((batch, dims[0])).astype(np.float32)
+    t = rng.standard_normal((batch, dims[3])).astype(np.float32)
+    net.set_dataset(x, t)
+    lr, b1, b2 = 1e-3, np.float64(np.float32(0.9)), np.float64(np.float32(0.999))
+    w = net.get_params().astype(np.float64)
+    m, v = np.zeros_like(w), np.zeros_like(w)
+    for step in range(1, 4):
+        before, grads = net.gradients(x, t)
+        loss = net.train(epochs=1, batch=batch, lr=lr, seed=step)
+        assert abs(loss - before) <= 1e-5 * abs(before)  # rows in another order
+        g = grads.astype(np.float64)
+        m, v = b1 * m + (1 - b1) * g, b2 * v + (1 - b2) * g * g
+        c1, c2 = (np.float64(np.float32(1) - np.float32(b) ** np.float32(step)) for b in (b1, b2))
+        expected = w - lr * (m / c1) / (np.sqrt(v / c2) + 1e-8)
+        w = net.get_params().astype(np.float64)
+        # the shuffled rows change the summation order of the gradients: 1e-5 of a gradient's size moves a step by
+        # at most lr * 1e-5 * max|g| / (|g| + eps)
+        slack = lr * np.minimum(2.0, 1e-5 * np.max(np.abs(g)) / (np.abs(g) + 1e-8))
+        assert np.all(np.abs(w - expected) <= lr * 1e-4 + slack + 1.3e-7 * np.abs(expected)), step
