@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "../../include/taral_pdhg.h"
+#include "cluster.cuh"
 #include "engine.hpp"
 #include "host.hpp"
 #include "kernels.cuh"
@@ -248,19 +249,38 @@ __global__ void __launch_bounds__(kThreads) k_pack_eval(const int4* __restrict__
     }
 }
 
-// One warp per instance: kkt[inst*10 + k] = sum of its pack blocks' partials, in block order (deterministic).
-__global__ void k_eval_finish(int ninst, const int2* __restrict__ where, const int* __restrict__ rr,
-                              const int* __restrict__ cr, const double* __restrict__ prow,
-                              const double* __restrict__ pcol, const int* __restrict__ active, double* kkt) {
-    const int inst = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (inst >= ninst || !active[inst] || lane >= 10) return;
-    const int2 pt = where[inst];  // {pack, slot}
+// Sums of `count` consecutive partials of K values each, in order: the CTA loads a chunk of them at once, then thread k
+// < K adds the chunk's values k one after another (a thread that also loads them pays the load latency per partial: 120 us
+// for the 450 blocks of a 12-period refinery LP, against 9 us). stride: doubles between the partials of one slot.
+constexpr int kFinishThreads = 128, kFinishChunk = 256;
+template <int K>
+__device__ __forceinline__ double ordered_sum(const double* part, size_t stride, int count, double (*sh)[K]) {
     double s = 0;
-    if (lane < 5)
-        for (int b = rr[pt.x]; b < rr[pt.x + 1]; ++b) s += prow[(size_t(b) * 8 + pt.y) * 5 + lane];
-    else
-        for (int b = cr[pt.x]; b < cr[pt.x + 1]; ++b) s += pcol[(size_t(b) * 8 + pt.y) * 5 + lane - 5];
-    kkt[inst * 10 + lane] = s;
+    for (int b0 = 0; b0 < count; b0 += kFinishChunk) {
+        const int n = min(kFinishChunk, count - b0);
+        for (int i = threadIdx.x; i < n * K; i += kFinishThreads) sh[i / K][i % K] = part[size_t(b0 + i / K) * stride + i % K];
+        __syncthreads();
+        if (int(threadIdx.x) < K) {
+#pragma unroll 8
+            for (int i = 0; i < n; ++i) s += sh[i][threadIdx.x];
+        }
+        __syncthreads();
+    }
+    return s;  // in threads 0 .. K - 1
+}
+
+// One CTA per instance: kkt[inst*10 + k] = sum of its pack blocks' partials, in block order (deterministic).
+__global__ void __launch_bounds__(kFinishThreads) k_eval_finish(const int2* __restrict__ where, const int* __restrict__ rr,
+                                                                const int* __restrict__ cr, const double* __restrict__ prow,
+                                                                const double* __restrict__ pcol,
+                                                                const int* __restrict__ active, double* kkt) {
+    __shared__ double sh[kFinishChunk][5];
+    const int inst = blockIdx.x;
+    if (!active[inst]) return;
+    const int2 pt = where[inst];  // {pack, slot}
+    const double r = ordered_sum<5>(prow + (size_t(rr[pt.x]) * 8 + pt.y) * 5, 40, rr[pt.x + 1] - rr[pt.x], sh);
+    const double c = ordered_sum<5>(pcol + (size_t(cr[pt.x]) * 8 + pt.y) * 5, 40, cr[pt.x + 1] - cr[pt.x], sh);
+    if (threadIdx.x < 5) kkt[inst * 10 + threadIdx.x] = r, kkt[inst * 10 + 5 + threadIdx.x] = c;
 }
 
 // The schedule's decision after a block (schedule.hpp, judge_block) for every running instance, one thread each.
@@ -373,21 +393,27 @@ __global__ void __launch_bounds__(kThreads) k_pack_pow_part(const int4* __restri
     }
 }
 
-__global__ void k_pow_update(int ninst, const int2* __restrict__ where, const int* __restrict__ cr,
-                             const double* __restrict__ part, double* est, double* scale, int* active, int it) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ninst || !active[i]) return;
-    const int2 pt = where[i];
-    double s = 0;
-    for (int b = cr[pt.x]; b < cr[pt.x + 1]; ++b) s += part[size_t(b) * 8 + pt.y];
-    double prev = est[i];
+// One CTA per distinct matrix: the step of its first instance {pack, slot, instance}; its blocks of the power lists are
+// range[k] .. range[k + 1] - 1. taken: the steps so far (on the device, so that a captured chunk of steps replays).
+__global__ void __launch_bounds__(kFinishThreads) k_pow_update(const int4* __restrict__ first, const int* __restrict__ range,
+                                                               const double* __restrict__ part, double* est, double* scale,
+                                                               int* active, int* taken) {
+    __shared__ double sh[kFinishChunk][1];
+    const int4 f = first[blockIdx.x];
+    const int inst = f.z;
+    if (!active[inst]) return;
+    const int b0 = range[blockIdx.x], b1 = range[blockIdx.x + 1];
+    const double s = ordered_sum<1>(part + size_t(b0) * 8 + f.y, 8, b1 - b0, sh);
+    if (threadIdx.x) return;
+    const int it = taken[blockIdx.x]++;
+    const double prev = est[inst];
     if (s <= 0) {
-        est[i] = 0, active[i] = 0;
+        est[inst] = 0, active[inst] = 0;
         return;
     }
-    double e = sqrt(sqrt(s));
-    est[i] = e, scale[i] = 1 / sqrt(s);
-    if (it >= 10 && fabs(e - prev) <= 1e-7 * e) active[i] = 0;
+    const double e = sqrt(sqrt(s));
+    est[inst] = e, scale[inst] = 1 / sqrt(s);
+    if (it >= 10 && fabs(e - prev) <= 1e-7 * e) active[inst] = 0;
 }
 
 template <class T>
@@ -500,6 +526,21 @@ struct Batch final : BatchBase {
     // row-chunk lists of the width-1 packs for k_rowthread_batch: one warp per kChunk rows of one instance
     int nA1r = 0, nT1r = 0;
     int4 *A1_rc = nullptr, *Ae1_rc = nullptr, *T1_rc = nullptr, *Te1_rc = nullptr;
+    // The power iteration runs on the first instance of every distinct matrix: block lists of those alone (their packs),
+    // [0] A, [1] A^T, and the columns' blocks in evaluation order.
+    struct PowerLists {
+        int n1 = 0, np = 0;
+        int4 *blk1 = nullptr, *ext1 = nullptr, *blkp = nullptr, *extp = nullptr;
+    } pw_lists[2];
+    int npw_ev = 0;
+    int4 *pw_ev = nullptr, *pwe_ev = nullptr, *pw_first = nullptr;
+    int *pw_range = nullptr, *pw_taken = nullptr;
+    cudaGraphExec_t pgraph = nullptr;  // a chunk of power-iteration steps
+    // small instances, each on one cluster (cluster.cuh): all of them, and the first of every distinct matrix
+    int cluster_ctas = 0;
+    size_t cluster_smem = 0;
+    ClusterLp<T> *d_lps = nullptr, *d_first_lps = nullptr;
+    double* d_norms = nullptr;
     std::vector<int4> h_a1r, h_ae1r, h_t1r, h_te1r, c_a1r, c_ae1r, c_t1r, c_te1r;
     std::vector<int4> h_a1, h_ap, h_t1, h_tp;  // host copies of the iteration block lists (autotuner)
     std::vector<int4> h_ae1, h_ae, h_te1, h_te;  // and of their extensions (instance or pack of each entry)
@@ -547,6 +588,7 @@ struct Batch final : BatchBase {
     }
     ~Batch() override {
         if (graph) cudaGraphExecDestroy(graph);
+        if (pgraph) cudaGraphExecDestroy(pgraph);
         for (void* p : allocs) cudaFreeAsync(p, s);
         if (s) cudaStreamSynchronize(s);
         if (h_count) cudaFreeHost(h_count);
@@ -808,6 +850,7 @@ struct Batch final : BatchBase {
         h_a1 = a1_it, h_ap = a_it, h_t1 = t1_it, h_tp = t_it;
         h_ae1 = ae1_it, h_ae = ae_it, h_te1 = te1_it, h_te = te_it;
         slot_inst = put(hslot), d_where = put(where);
+        power_lists(t_ev, te_ev, hcr);
         // 5. upload
         A_it = put(a_it), Ae_it = put(ae_it), T_it = put(t_it), Te_it = put(te_it);
         A_ev = put(a_ev), Ae_ev = put(ae_ev), T_ev = put(t_ev), Te_ev = put(te_ev);
@@ -849,11 +892,85 @@ struct Batch final : BatchBase {
         for (int i = 0; i < count; ++i) models.push_back(md + i);
         mark("vectors+lists");
         tune();
+        choose_cluster();
         mark("tune");
         if (std::getenv("TARAL_TIMING")) {
             std::fprintf(stderr, "taral: batch set-up");
             for (const auto& mk : marks) std::fprintf(stderr, " %s %.3f", mk.first, mk.second);
             std::fprintf(stderr, " s\n");
+        }
+    }
+
+    void power_lists(const std::vector<int4>& t_ev, const std::vector<int4>& te_ev, const std::vector<int>& hcr) {
+        std::vector<char> first_of(size_t(ninst), 0), pack_of(packs.size(), 0);
+        for (int i : first_inst) first_of[size_t(i)] = 1, pack_of[size_t(where[size_t(i)].x)] = 1;
+        auto pick = [&](const std::vector<int4>& blk, const std::vector<int4>& ext, const std::vector<char>& keep, int4*& db, int4*& de) {
+            std::vector<int4> b, e;
+            for (size_t k = 0; k < blk.size(); ++k)
+                if (keep[size_t(ext[k].x)]) b.push_back(blk[k]), e.push_back(ext[k]);
+            db = put(b), de = put(e);
+            return int(b.size());
+        };
+        pw_lists[0].n1 = pick(h_a1, h_ae1, first_of, pw_lists[0].blk1, pw_lists[0].ext1), pw_lists[0].np = pick(h_ap, h_ae, pack_of, pw_lists[0].blkp, pw_lists[0].extp);
+        pw_lists[1].n1 = pick(h_t1, h_te1, first_of, pw_lists[1].blk1, pw_lists[1].ext1), pw_lists[1].np = pick(h_tp, h_te, pack_of, pw_lists[1].blkp, pw_lists[1].extp);
+        std::vector<int4> ev, eve, first;
+        std::vector<int> range{0};
+        for (int k = 0; k < distinct; ++k) {
+            const int i = first_inst[size_t(k)];
+            const int2 at = where[size_t(i)];
+            for (int b = hcr[size_t(at.x)]; b < hcr[size_t(at.x) + 1]; ++b) ev.push_back(t_ev[size_t(b)]), eve.push_back(te_ev[size_t(b)]);
+            first.push_back(make_int4(at.x, at.y, i, 0)), range.push_back(int(ev.size()));
+        }
+        npw_ev = int(ev.size());
+        pw_ev = put(ev), pwe_ev = put(eve), pw_first = put(first), pw_range = put(range), pw_taken = alloc<int>(size_t(distinct));
+    }
+
+    // Small instances on one cluster each (cluster.cuh): where the launch's waves of clusters, at about 0.9 us an iteration
+    // + 0.33 us a thousand nonzeros of a CTA (+ 1 us for the cluster's barriers and exchange), take less than the phase
+    // kernels' 7.5 us + 8 us a million products. Measured, FP64: 40 instances of 151 x 347 (1,400 nonzeros) 1.4 against 9 us.
+    void choose_cluster() {
+        const char* res = std::getenv("TARAL_RESIDENT");
+        if (pdl || (res && std::atoi(res) == 0) || forced_row_split() > 0 || std::getenv("TARAL_ROWTHREAD")) return;
+        if (std::getenv("TARAL_ROWSPLIT") || packs.size() != size_t(ninst)) return;
+        int64_t most = 0;
+        for (const auto& sh : mats) {
+            if (sh->maxrowA > kTile || sh->maxrowT > kTile || sh->S.m > kClusterRows || sh->S.n > kClusterRows) return;
+            if (sh->S.m == 0 || sh->S.n == 0) return;
+            most = std::max(most, sh->nnz);
+        }
+        int dev, sms;
+        BK(cudaGetDevice(&dev));
+        BK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        std::vector<std::vector<int>> plans(mats.size());
+        for (int q = cluster_size(most); q <= 8; q *= 2) {
+            const double waves = std::ceil(double(ninst) * q / double(q > 1 ? 128 : sms));
+            const double cluster = waves * (0.9 + 0.33e-3 * double(most) / q + (q > 1 ? 1.0 : 0.0));
+            if (cluster > 7.5 + 8e-6 * double(nnz_total)) return;
+            size_t need = 0;
+            for (size_t k = 0; k < mats.size() && need <= kClusterSmem; ++k) {
+                const Shared& sh = *mats[k];
+                const std::vector<int> ap(sh.S.A.ptr.begin(), sh.S.A.ptr.end()), tp(sh.S.AT.ptr.begin(), sh.S.AT.ptr.end());
+                need = std::max(need, cluster_plan<T>(ap.data(), tp.data(), sh.S.m, sh.S.n, q, plans[k]));
+            }
+            if (need > kClusterSmem) continue;
+            std::vector<int*> d_plan;
+            for (const auto& p : plans) d_plan.push_back(put(p));
+            std::vector<ClusterLp<T>> lps, firsts;
+            for (int i = 0; i < ninst; ++i) {
+                const Shared& sh = *mats[size_t(mat_of[size_t(i)])];
+                const Pack& pk = packs[size_t(where[size_t(i)].x)];
+                const int rb = pk.rbase, cb = pk.cbase;
+                ClusterLp<T> lp{Aptr + sh.pbaseA, Aidx, Tptr + sh.pbaseT, Tidx, Aval, Tval, sh.S.m, sh.S.n, x + cb, z + rb, Ax + rb,
+                                ATz + cb, xs + cb, zs + rb, c + cb, l + cb, u + cb, rl + rb, ru + rb, par + 2 * i, pv + cb,
+                                d_plan[size_t(mat_of[size_t(i)])], running + i};
+                lps.push_back(lp);
+                lp.active = nullptr;
+                if (first_inst[size_t(mat_of[size_t(i)])] == i) firsts.push_back(lp);  // in the order of the matrices
+            }
+            d_lps = put(lps), d_first_lps = put(firsts), d_norms = alloc<double>(2 * mats.size());
+            cluster_ctas = q, cluster_smem = need;
+            mem_used = alloc_bytes;
+            return;
         }
     }
 
@@ -1005,7 +1122,7 @@ struct Batch final : BatchBase {
             if (nA) k_pack_eval<T, double, true><<<nA, kThreads, 0, s>>>(A_ev, Ae_ev, slot_inst, act, fi, tmpM, zs, rl, ru, nullptr, Dr, zlast, partA);
             if (nT) k_pack_eval<T, double, false><<<nT, kThreads, 0, s>>>(T_ev, Te_ev, slot_inst, act, fi, xs, tmpN, l, u, c, Dc, xlast, partT);
         }
-        k_eval_finish<<<(ninst + 7) / 8, 256, 0, s>>>(ninst, d_where, rr, cr, partA, partT, act, dst);
+        k_eval_finish<<<ninst, kFinishThreads, 0, s>>>(d_where, rr, cr, partA, partT, act, dst);
         launches += 3;
     }
     // The iteration lists of the running instances only. A stopped instance's CTAs would return at once, but in the
@@ -1064,10 +1181,15 @@ struct Batch final : BatchBase {
     }
 
     void block(int steps) {
-        if (nT) k_pack_xupd<T><<<nT, kThreads, 0, s>>>(T_ev, Te_ev, slot_inst, running, x, ATz, c, l, u, par, xs), ++launches;
-        for (int k = 0; k < steps; ++k) {
-            spmv_A(x, EpiRow<T>{Ax, z, zs, rl, ru, par}, running, pdl);
-            spmv_T(z, EpiCol<T>{ATz, x, xs, c, l, u, par, k + 1 < steps ? 1 : 0}, running, pdl);
+        if (cluster_ctas > 0) {
+            BK(launch_cluster(k_cluster_iterate<T, true>, k_cluster_iterate<T, false>, d_lps, ninst, cluster_ctas, cluster_smem, s, steps));
+            launches += 1 + 2 * int64_t(steps);  // the phases, as when each is a launch of its own
+        } else {
+            if (nT) k_pack_xupd<T><<<nT, kThreads, 0, s>>>(T_ev, Te_ev, slot_inst, running, x, ATz, c, l, u, par, xs), ++launches;
+            for (int k = 0; k < steps; ++k) {
+                spmv_A(x, EpiRow<T>{Ax, z, zs, rl, ru, par}, running, pdl);
+                spmv_T(z, EpiCol<T>{ATz, x, xs, c, l, u, par, k + 1 < steps ? 1 : 0}, running, pdl);
+            }
         }
         int g = (ninst + 255) / 256;
         k_advance<<<g, 256, 0, s>>>(ninst, st, steps);
@@ -1081,6 +1203,55 @@ struct Batch final : BatchBase {
         products(rflag);
         k_count<<<1, 256, 0, s>>>(ninst, running, count);
         launches += 7;
+    }
+
+    // Up to 200 power steps on the first instance of every distinct matrix, 8 at a time between looks at the device-side
+    // stop flags; with graphs a chunk is captured once for the batch's lifetime (its lists never change).
+    void power_iteration() {
+        constexpr int chunk = 8;  // even: the vectors end a chunk in their starting roles
+        BK(cudaMemsetAsync(pw_taken, 0, size_t(distinct) * sizeof(int), s));
+        auto steps = [&] {
+            T *a = pv, *b = pu;
+            for (int k = 0; k < chunk; ++k) {
+                power_spmv(0, a, pw), power_spmv(1, pw, b);
+                if (npw_ev) k_pack_pow_part<T><<<npw_ev, kThreads, 0, s>>>(pw_ev, pwe_ev, slot_inst, pactive, b, partT);
+                k_pow_update<<<distinct, kFinishThreads, 0, s>>>(pw_first, pw_range, partT, est, pscale, pactive, pw_taken);
+                if (npw_ev) k_pack_pow_scale<T><<<npw_ev, kThreads, 0, s>>>(pw_ev, pwe_ev, slot_inst, pactive, pscale, b);
+                launches += 3;
+                std::swap(a, b);
+            }
+            k_count<<<1, 256, 0, s>>>(ninst, pactive, count), ++launches;
+        };
+        for (int it = 0; it < 200; it += chunk) {
+            if (!opt.graph) {
+                steps();
+            } else {
+                const int64_t before = launches;
+                if (!pgraph) {
+                    cudaGraph_t gr;
+                    BK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+                    steps();
+                    BK(cudaStreamEndCapture(s, &gr));
+                    BK(cudaGraphInstantiate(&pgraph, gr, 0));
+                    BK(cudaGraphDestroy(gr));
+                    per_pgraph = launches - before;
+                }
+                BK(cudaGraphLaunch(pgraph, s));
+                launches = before + per_pgraph;
+            }
+            BK(cudaMemcpyAsync(h_count, count, sizeof(int), cudaMemcpyDeviceToHost, s));
+            BK(cudaStreamSynchronize(s));
+            if (*h_count == 0) break;
+        }
+    }
+    int64_t per_pgraph = 0;
+    void power_spmv(int phase, const T* xin, T* y) {
+        const PowerLists& q = pw_lists[phase];
+        const int *ptr = phase ? Tptr : Aptr, *idx = phase ? Tidx : Aidx;
+        const T* val = phase ? Tval : Aval;
+        const EpiStore<T> e{y};
+        if (q.n1) launch(k_rowblock_batch<T, T, EpiStore<T>, true>, q.n1, false, ptr, idx, val, xin, (const int4*)q.blk1, (const int4*)q.ext1, (const int*)pactive, e);
+        if (q.np) k_pack_spmv<T, T, EpiStore<T>><<<q.np, kThreads, 0, s>>>(ptr, idx, val, xin, q.blkp, q.extp, slot_inst, pactive, e), ++launches;
     }
 
     void cancel() override {
@@ -1115,26 +1286,21 @@ struct Batch final : BatchBase {
             if (rep[size_t(mat_of[i])] < 0) rep[size_t(mat_of[i])] = i, first[size_t(i)] = 1;
         BK(cudaMemcpyAsync(pactive, first.data(), ninst * sizeof(int), cudaMemcpyHostToDevice, s));
         BK(cudaMemsetAsync(est, 0, ninst * sizeof(double), s));
-        T *a = pv, *b = pu;
-        int g = (ninst + 255) / 256;
-        for (int it = 0; it < 200;) {
-            int end = std::min(200, it + 8);
-            for (; it < end; ++it) {
-                spmv_A(a, EpiStore<T>{pw}, pactive);
-                spmv_T(pw, EpiStore<T>{b}, pactive);
-                if (nT) k_pack_pow_part<T><<<nT, kThreads, 0, s>>>(T_ev, Te_ev, slot_inst, pactive, b, partT);
-                k_pow_update<<<g, 256, 0, s>>>(ninst, d_where, cr, partT, est, pscale, pactive, it);
-                if (nT) k_pack_pow_scale<T><<<nT, kThreads, 0, s>>>(T_ev, Te_ev, slot_inst, pactive, pscale, b);
-                launches += 3;
-                std::swap(a, b);
-            }
-            k_count<<<1, 256, 0, s>>>(ninst, pactive, count);
-            BK(cudaMemcpyAsync(h_count, count, sizeof(int), cudaMemcpyDeviceToHost, s));
-            BK(cudaStreamSynchronize(s));
-            if (*h_count == 0) break;
-        }
+        const int g = (ninst + 255) / 256;
         std::vector<double> norms(ninst);
-        BK(cudaMemcpyAsync(norms.data(), est, ninst * sizeof(double), cudaMemcpyDeviceToHost, s));
+        if (cluster_ctas > 0) {
+            BK(launch_cluster(k_cluster_power<T, true>, k_cluster_power<T, false>, d_first_lps, distinct, cluster_ctas, cluster_smem, s, 200, d_norms));
+            std::vector<double> got(2 * size_t(distinct));
+            BK(cudaMemcpyAsync(got.data(), d_norms, got.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
+            BK(cudaStreamSynchronize(s));
+            for (int k = 0; k < distinct; ++k) {
+                norms[size_t(first_inst[size_t(k)])] = got[2 * size_t(k)];
+                launches += 2 * int64_t(got[2 * size_t(k) + 1]);  // the products, as when each is a launch of its own
+            }
+        } else {
+            power_iteration();
+            BK(cudaMemcpyAsync(norms.data(), est, ninst * sizeof(double), cudaMemcpyDeviceToHost, s));
+        }
         BK(cudaStreamSynchronize(s));
         for (int i = 0; i < ninst; ++i) norms[size_t(i)] = norms[size_t(rep[size_t(mat_of[i])])];
         double power_s = since(t0);
@@ -1193,7 +1359,7 @@ struct Batch final : BatchBase {
         int64_t it = 0;
         // TARAL_COMPACT=0 keeps the full iteration lists; TARAL_TRACE=1 prints the running count per block
         const char* ce = std::getenv("TARAL_COMPACT");
-        const bool compact = !(ce && std::atoi(ce) == 0);
+        const bool compact = !(ce && std::atoi(ce) == 0) && cluster_ctas == 0;  // a cluster launch takes its LPs as they are
         const bool trace = std::getenv("TARAL_TRACE") != nullptr;
         int live_lists = ninst;  // running instances when the lists were last built
         std::vector<int> live(static_cast<size_t>(ninst));

@@ -34,7 +34,8 @@ struct ClusterLp {
     double *xs, *zs;
     const T *c, *l, *u, *rl, *ru;
     const double* par;
-    const int* plan;    // the slices, see ClusterPlan
+    const T* v0;        // the power iteration's start
+    const int* plan;    // the CTAs' headers (ClusterCta) and what they refer to, see cluster_plan
     const int* active;  // NULL, or the LP is left alone when *active == 0
 };
 
@@ -261,7 +262,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster_iterate(const Cl
 // shuffle tree, then 8 groups, then all of them: the CTAs and warps of k_power_sumsq. v stays unnormalised in the copies;
 // the factor is applied where it is gathered.
 template <class T, bool MANY>
-__global__ void __launch_bounds__(kClusterThreads, 1) k_cluster_power(const ClusterLp<T>* __restrict__ lps, int ctas, int iters, const T* v0, double* out) {
+__global__ void __launch_bounds__(kClusterThreads, 1) k_cluster_power(const ClusterLp<T>* __restrict__ lps, int ctas, int iters, double* out) {
     extern __shared__ __align__(16) unsigned char raw[];
     __shared__ double sums[kClusterRows / 256 + 1], total;
     const ClusterLp<T> p = lps[blockIdx.x / ctas];
@@ -277,7 +278,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster_power(const Clus
     double* squares = reinterpret_cast<double*>(raw + o.squares);
     const int groups = (p.n + 31) / 32, blocks = (p.n + 255) / 256;
     lp_barrier<MANY>();
-    for (int j = tid; j < p.n; j += kClusterThreads) v[where[j]] = v0[j];  // every CTA fills its own copy
+    for (int j = tid; j < p.n; j += kClusterThreads) v[where[j]] = p.v0[j];  // every CTA fills its own copy
     __syncthreads();
     double est = 0, f = 0;
     int it = 0;

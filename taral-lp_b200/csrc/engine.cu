@@ -630,7 +630,7 @@ struct Engine final : EngineBase {
             int* d_plan = alloc<int>(plan.size());
             CK(cudaMemcpyAsync(d_plan, plan.data(), plan.size() * sizeof(int), cudaMemcpyHostToDevice, st));
             const ClusterLp<T> lp{A.ptr, A.idx, AT.ptr, AT.idx, static_cast<const T*>(A.val), static_cast<const T*>(AT.val),
-                                  m, n, x, z, Ax, ATz, xs, zs, c, l, u, rl, ru, par, d_plan, nullptr};
+                                  m, n, x, z, Ax, ATz, xs, zs, c, l, u, rl, ru, par, pv, d_plan, nullptr};
             d_lp = alloc<ClusterLp<T>>(1);
             CK(cudaMemcpyAsync(d_lp, &lp, sizeof lp, cudaMemcpyHostToDevice, st));
             CK(cudaStreamSynchronize(st));
@@ -707,7 +707,7 @@ struct Engine final : EngineBase {
         CK(cudaMemsetAsync(pdone, 0, sizeof(int), st));
         launches += 1;
         if (cluster_ctas > 0) {
-            CK(launch_cluster(k_cluster_power<T, true>, k_cluster_power<T, false>, d_lp, 1, cluster_ctas, cluster_smem, st, iters, pv, h_out));
+            CK(launch_cluster(k_cluster_power<T, true>, k_cluster_power<T, false>, d_lp, 1, cluster_ctas, cluster_smem, st, iters, h_out));
             CK(cudaStreamSynchronize(st));
             launches += 2 * int64_t(h_out[1]);  // the products, as when each is a launch of its own
             return h_out[0];

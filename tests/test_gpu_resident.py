@@ -2,6 +2,8 @@
 cooperative grid; csrc/cluster.cuh: one thread-block cluster, the LP in its shared memory) against the phase kernels they
 stand for: the same products summed in the same order, so every number is the same bit for bit. TARAL_RESIDENT forces
 a form: 0 phase kernels, 1 the grid; TARAL_CLUSTER the smallest cluster (the LP's data may ask for a larger one)."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -50,3 +52,27 @@ def test_resident_launches_change_nothing(engine_lib, monkeypatch, case, precisi
     for mode in got:
         for k, (a, b) in enumerate(zip(got["01"], got[mode])):
             assert np.array_equal(a, b, equal_nan=True), (mode, k, np.max(np.abs(a - b)))
+
+
+@pytest.mark.parametrize("precision", [pdhg.FP64, pdhg.FP32], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("shape", ["one_cta", "several_ctas", "shared_matrix"])
+def test_batch_clusters_change_nothing(engine_lib, monkeypatch, shape, precision):
+    """A batch of small LPs on one cluster each against the batch's phase kernels: the same norms, iterations and points,
+    bit for bit, through restarts, instances that stop at different blocks and a final partial block."""
+    if shape == "shared_matrix":  # instances of one matrix with their own costs and bounds
+        base = lpgen.general(200, 450, seed=5)
+        rng = np.random.default_rng(1)
+        lps = [dataclasses.replace(base, cost=base.cost * rng.uniform(0.8, 1.2, base.n)) for _ in range(5)]
+    else:
+        m, n = (120, 300) if shape == "one_cta" else (900, 2100)
+        lps = [lpgen.general(m + 7 * k, n + 11 * k, seed=k) for k in range(5)] + [lpgen.transport(12, 17, seed=2)]
+    got = []
+    for mode in ("0", "2"):
+        monkeypatch.setenv("TARAL_RESIDENT", mode)
+        b = pdhg.Batch(lps, tol=1e-5, max_iter=1000, precision=precision)
+        got.append(b.solve() + b.solve())  # the second solve replays the captured launches
+        b.close()
+    for (r0, x0, y0), (r1, x1, y1) in zip((got[0][:3], got[0][3:]), (got[1][:3], got[1][3:])):
+        for a, c in zip(r0, r1):
+            assert (a["status"], a["iterations"], a["restarts"], a["norm_a"]) == (c["status"], c["iterations"], c["restarts"], c["norm_a"])
+        assert all(np.array_equal(p, q) for p, q in zip(x0 + y0, x1 + y1))
