@@ -22,6 +22,7 @@
 #include <memory>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/taral_pdhg.h"
@@ -29,6 +30,7 @@
 #include "engine.hpp"
 #include "host.hpp"
 #include "kernels.cuh"
+#include "panels.cuh"
 #include "scaling.cuh"
 #include "solve.hpp"
 
@@ -473,6 +475,7 @@ struct Shared {  // one distinct scaled matrix
     int64_t nnzbase = 0, nnz = 0;
     int dr_off = 0, dc_off = 0;  // offsets of this matrix's Dr / Dc in the device scaling scratch
     int maxrowA = 0, maxrowT = 0;  // longest row of A and of A^T
+    PanelPlan panels[2];           // of A and of A^T, until they are uploaded
 };
 
 uint64_t fnv(const void* p, size_t n, uint64_t h) {  // FNV-1a over 8-byte words, then the tail bytes
@@ -669,10 +672,18 @@ struct Batch final : BatchBase {
                 });
             for (auto& t : th) t.join();
         };
+        // panels (panels.cuh) for every matrix, both ways, or for none
+        nnz_total = 0;
+        for (int i = 0; i < count; ++i) nnz_total += md[i].col_ptr[md[i].n];
+        const bool panels_ok = panels_allowed();
         par_for(distinct, [&](int k) {
             Shared& sh = *mats[k];
             const taral_model& mk = md[first_inst[k]];
             model_matrices(mk, sh.S.A, sh.S.AT, 1);
+            if (panels_ok) {
+                sh.panels[0] = build_panels(sh.S.A.ptr.data(), sh.S.A.idx.data(), mk.m, mk.n, kPanelTarget, kBatchPanelCols, 1);
+                if (!sh.panels[0].empty()) sh.panels[1] = build_panels(sh.S.AT.ptr.data(), sh.S.AT.idx.data(), mk.n, mk.m, kPanelTarget, kBatchPanelCols, 1);
+            }
             sh.S.m = mk.m, sh.S.n = mk.n, sh.nnz = int64_t(sh.S.A.idx.size());
         });
         mark("transposes");
@@ -729,6 +740,7 @@ struct Batch final : BatchBase {
                 k_narrow<T><<<g, 256, 0, s>>>(nzb, va, Aval);
                 k_narrow<T><<<g, 256, 0, s>>>(nzb, vt, Tval);
             }
+            put_panels();
             std::vector<double> hdr(static_cast<size_t>(drn)), hdc(static_cast<size_t>(dcn));
             if (drn) BK(cudaMemcpyAsync(hdr.data(), dr, size_t(drn) * sizeof(double), cudaMemcpyDeviceToHost, s));
             if (dcn) BK(cudaMemcpyAsync(hdc.data(), dc, size_t(dcn) * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -851,6 +863,7 @@ struct Batch final : BatchBase {
         h_ae1 = ae1_it, h_ae = ae_it, h_te1 = te1_it, h_te = te_it;
         slot_inst = put(hslot), d_where = put(where);
         power_lists(t_ev, te_ev, hcr);
+        panel_lists(std::vector<int>(size_t(count), 1));
         // 5. upload
         A_it = put(a_it), Ae_it = put(ae_it), T_it = put(t_it), Te_it = put(te_it);
         A_ev = put(a_ev), Ae_ev = put(ae_ev), T_ev = put(t_ev), Te_ev = put(te_ev);
@@ -899,6 +912,103 @@ struct Batch final : BatchBase {
             for (const auto& mk : marks) std::fprintf(stderr, " %s %.3f", mk.first, mk.second);
             std::fprintf(stderr, " s\n");
         }
+    }
+
+    // ------------------------------------------------------------------ panels
+    // Every phase of a batch on panels of the distinct matrices, kPW instances that share a matrix to a CTA. On 48
+    // refinery scenarios of 12 matrices (22.6M products a phase, FP32) a row phase takes @ROW us (row blocks 72), a column
+    // phase @COL (55). From a million nonzeros over the instances, where panels fill the SMs. TARAL_PANELS=0: none.
+    static constexpr int kPW = sizeof(T) == 4 ? 4 : 2;
+    static constexpr int kPanelTarget = 24576, kBatchPanelCols = 4096;
+    PanelMat<T> panels[2];
+    int npanels[2] = {0, 0};
+    PanelSize panel_most[2];
+    std::vector<int> first_panel[2];                       // of every matrix, and the end
+    PanelWork<kPW>* panel_work[2] = {nullptr, nullptr};    // the running instances' CTAs
+    PanelWork<1>* panel_first[2] = {nullptr, nullptr};     // the power iteration's
+    int npanel_work[2] = {0, 0};
+    bool panels_allowed() const {
+        const char* e = std::getenv("TARAL_PANELS");
+        const char* pack = std::getenv("TARAL_BATCH_PACK");
+        if ((e && std::atoi(e) == 0) || (pack && std::atoi(pack) > 1) || pdl || std::getenv("TARAL_ROWSPLIT") || std::getenv("TARAL_ROWTHREAD"))
+            return false;
+        return nnz_total >= (int64_t(1) << 20) || (e && std::atoi(e) > 0);
+    }
+    void put_panels() {  // the plans of all matrices one after another, filled from the scaled values
+        for (const auto& sh : mats)
+            if (sh->panels[0].empty() || sh->panels[1].empty()) return;
+        for (int k = 0; k < 2; ++k) {
+            PanelPlan all;
+            for (size_t q = 0; q < mats.size(); ++q) {
+                Shared& sh = *mats[q];
+                PanelPlan& p = sh.panels[k];
+                first_panel[k].push_back(int(all.panels.size()));
+                all.append(p, k ? sh.pbaseT : sh.pbaseA);
+                p = PanelPlan();
+            }
+            first_panel[k].push_back(int(all.panels.size()));
+            Four<T>* val = alloc<Four<T>>(size_t(all.groups) * 32);
+            Places* place = alloc<Places>(size_t(all.groups) * 32);
+            T* lval = alloc<T>(size_t(all.long_entries));
+            auto* lplace = alloc<unsigned short>(size_t(all.long_entries));
+            panels[k] = {put(all.panels), put(all.slice), put(all.order), put(all.cols), val, place, put(all.longrow), lval, lplace};
+            npanels[k] = int(all.panels.size()), panel_most[k] = all.most;
+            k_panel_fill<T><<<npanels[k], kThreads, 0, s>>>(panels[k].panels, panels[k].slice, panels[k].order, panels[k].cols,
+                                                            panels[k].longrow, k ? Tptr : Aptr, k ? Tidx : Aidx, k ? Tval : Aval, val,
+                                                            place, lval, lplace);
+            BK(cudaGetLastError());
+        }
+    }
+    // The CTAs of the instances with live[i], matrix by matrix: a panel, then the groups of instances that use it.
+    void panel_lists(const std::vector<int>& live) {
+        if (npanels[0] == 0) return;
+        std::vector<std::vector<int>> users(mats.size());
+        for (int i = 0; i < ninst; ++i)
+            if (live[size_t(i)]) users[size_t(mat_of[size_t(i)])].push_back(i);
+        for (int k = 0; k < 2; ++k) {
+            std::vector<PanelWork<kPW>> work;
+            std::vector<PanelWork<1>> first;
+            auto entry = [&](auto& w, int at, int i) {
+                const Shared& sh = *mats[size_t(mat_of[size_t(i)])];
+                const Pack& q = packs[size_t(where[size_t(i)].x)];
+                w.inst[at] = i, w.row[at] = k ? q.cbase - sh.pbaseT : q.rbase - sh.pbaseA, w.gather[at] = k ? q.rbase : q.cbase;
+            };
+            for (size_t q = 0; q < mats.size(); ++q)
+                for (int p = first_panel[k][q]; p < first_panel[k][q + 1]; ++p) {
+                    for (size_t u = 0; u < users[q].size(); u += kPW) {
+                        PanelWork<kPW> w;
+                        w.panel = p;
+                        for (int t = 0; t < kPW; ++t) {
+                            w.inst[t] = -1, w.row[t] = 0, w.gather[t] = 0;
+                            if (u + size_t(t) < users[q].size()) entry(w, t, users[q][u + size_t(t)]);
+                        }
+                        work.push_back(w);
+                    }
+                    PanelWork<1> f;
+                    f.panel = p, entry(f, 0, first_inst[q]);
+                    first.push_back(f);
+                }
+            if (!panel_work[k]) {  // every instance is live: the longest lists
+                panel_work[k] = put(work), panel_first[k] = put(first);
+            } else if (!work.empty()) {
+                BK(cudaMemcpyAsync(panel_work[k], work.data(), work.size() * sizeof(work[0]), cudaMemcpyHostToDevice, s));
+                BK(cudaStreamSynchronize(s));
+            }
+            npanel_work[k] = int(work.size());
+        }
+    }
+    // One phase on panels, if this batch has them; false: the row blocks'.
+    template <class X, class E>
+    bool panel_phase(int k, const X* xin, const E& e, const int* act) {
+        if constexpr (std::is_same<X, T>::value) {
+            if (npanels[0] == 0) return false;
+            if (npanel_work[k] == 0) return true;
+            BK(launch_panels(panels[k], npanel_work[k], panel_most[k], xin, (const PanelWork<kPW>*)panel_work[k], act,
+                             panel_step(e), s));
+            ++launches;
+            return true;
+        }
+        return false;
     }
 
     void power_lists(const std::vector<int4>& t_ev, const std::vector<int4>& te_ev, const std::vector<int>& hcr) {
@@ -987,6 +1097,7 @@ struct Batch final : BatchBase {
         const int forced = forced_row_split();
         int forced_thread = -1;
         if (const char* e = std::getenv("TARAL_ROWTHREAD")) forced_thread = std::atoi(e) != 0 ? 1 : 0;
+        if (npanels[0]) return;  // the phases run on panels
         const bool timing = forced < 0 && forced_thread < 0;
         if (timing && nnz_total < (int64_t(1) << 20)) return;  // small: timings are noise
         std::vector<int> ones(size_t(ninst), 1);
@@ -1089,6 +1200,7 @@ struct Batch final : BatchBase {
     bool pdl = false;  // TARAL_PDL=1 (set at build)
     template <class X, class E>
     void spmv_A(const X* xin, const E& e, const int* act, bool programmatic = false) {
+        if (panel_phase(0, xin, e, act)) return;
         if (thread1[0] && nA1r)
             launch(k_rowthread_batch<T, X, E>, (nA1r + 7) / 8, programmatic, nA1r, (const int*)Aptr, (const int*)Aidx,
                    (const T*)Aval, xin, (const int4*)A1_rc, (const int4*)Ae1_rc, act, e);
@@ -1099,6 +1211,7 @@ struct Batch final : BatchBase {
     }
     template <class X, class E>
     void spmv_T(const X* xin, const E& e, const int* act, bool programmatic = false) {
+        if (panel_phase(1, xin, e, act)) return;
         if (thread1[1] && nT1r)
             launch(k_rowthread_batch<T, X, E>, (nT1r + 7) / 8, programmatic, nT1r, (const int*)Tptr, (const int*)Tidx,
                    (const T*)Tval, xin, (const int4*)T1_rc, (const int4*)Te1_rc, act, e);
@@ -1171,12 +1284,14 @@ struct Batch final : BatchBase {
         pick(h_a1r, h_ae1r, true, c_a1r, c_ae1r), pick(h_t1r, h_te1r, true, c_t1r, c_te1r);
         upload_lists(c_a1, c_ae1, c_ap, c_ae, c_t1, c_te1, c_tp, c_te);
         upload_chunks(c_a1r, c_ae1r, c_t1r, c_te1r);
+        panel_lists(live);
         compacted = true;
     }
     void restore_lists() {
         if (!compacted) return;
         upload_lists(h_a1, h_ae1, h_ap, h_ae, h_t1, h_te1, h_tp, h_te);
         upload_chunks(h_a1r, h_ae1r, h_t1r, h_te1r);
+        panel_lists(std::vector<int>(size_t(ninst), 1));
         compacted = false;
     }
 
@@ -1246,6 +1361,12 @@ struct Batch final : BatchBase {
     }
     int64_t per_pgraph = 0;
     void power_spmv(int phase, const T* xin, T* y) {
+        if (npanels[0]) {
+            BK(launch_panels(panels[phase], npanels[phase], panel_most[phase], xin, (const PanelWork<1>*)panel_first[phase],
+                             (const int*)pactive, PanelStore<T>{y}, s));
+            ++launches;
+            return;
+        }
         const PowerLists& q = pw_lists[phase];
         const int *ptr = phase ? Tptr : Aptr, *idx = phase ? Tidx : Aidx;
         const T* val = phase ? Tval : Aval;

@@ -22,6 +22,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/taral_pdhg.h"
@@ -29,6 +30,7 @@
 #include "host.hpp"
 #include "cluster.cuh"
 #include "kernels.cuh"
+#include "panels.cuh"
 #include "resident.cuh"
 #include "scaling.cuh"
 
@@ -152,7 +154,7 @@ static int grid_for(int64_t k) {  // elementwise kernels: grid-stride, at most 8
     return int(std::max<int64_t>(1, std::min<int64_t>((k + 255) / 256, 148 * 8)));
 }
 static int red_grid(int64_t k) {  // reductions: fixed grid per size, so the partial-sum order is fixed
-    return int(std::max<int64_t>(1, std::min<int64_t>((k + 255) / 256, 296)));
+    return int(std::max<int64_t>(1, std::min<int64_t>((k + 255) / 256, kRedCtas)));
 }
 
 struct CudaError {
@@ -258,7 +260,48 @@ struct Engine final : EngineBase {
         begin(m_, n_, freq, flags);
         A = upload(hA), AT = upload(hAT);
         nnz = hA.nnz;
+        PanelPlan panels_a, panels_t;
+        plan_panels({hA.rows, hA.ptr, hA.idx, hA.val}, {hAT.rows, hAT.ptr, hAT.idx, hAT.val}, flags, panels_a, panels_t);
+        put_panels(0, A, panels_a), put_panels(1, AT, panels_t);
+        CK(cudaStreamSynchronize(st));  // the plans are released
         finish_init(hc_ptr, hl, hu, hrl_ptr, hru_ptr, hDr, hDc);
+    }
+    // Panels (panels.cuh) for A and A^T, both or neither, from 1.5M nonzeros in FP64 and 3M in FP32: a panel's latency is
+    // about 7 us. Refinery LPs, us an iteration with row blocks / panels: 1.1M nonzeros FP64 15.1 / 17.0, FP32 11.8 / 16.0;
+    // 2.3M FP64 31.3 / 20.9, FP32 16.3 / 18.4; 3.4M FP64 42.0 / 31.6, FP32 23.3 / 21.3. Panels of half an SM's share of the nonzeros, 8,192 to 16,384: smaller ones
+    // reread too many columns, larger ones leave SMs idle. TARAL_PANELS=0: none (tests).
+    PanelMat<T> panels[2];
+    int npanels[2] = {0, 0};
+    PanelSize panel_most[2];
+    void plan_panels(const CsrRef& a, const CsrRef& at, unsigned flags, PanelPlan& pa, PanelPlan& pt) {
+        const char* e = std::getenv("TARAL_PANELS");
+        const bool forced = e && std::atoi(e) > 0;  // whatever the size
+        if ((e && !forced) || (flags & TARAL_FLAG_NO_GRAPH) || std::getenv("TARAL_PDL") || forced_row_split() >= 0 ||
+            std::getenv("TARAL_ROWTHREAD") || (a.nnz() < (sizeof(T) == 4 ? 3000000 : 1500000) && !forced))
+            return;
+        const int target = int(std::min<int64_t>(16384, std::max<int64_t>(8192, a.nnz() / (148 * 2) * 21 / 20)));
+        pa = build_panels(a.ptr, a.idx, a.rows, at.rows, target, kPanelCols, host_threads());
+        if (!pa.empty()) pt = build_panels(at.ptr, at.idx, at.rows, a.rows, target, kPanelCols, host_threads());
+        if (pa.empty() || pt.empty()) pa = PanelPlan(), pt = PanelPlan();
+    }
+    void put_panels(int which, const DevMat& d, const PanelPlan& p) {
+        if (p.empty()) return;
+        auto put = [&](const auto& v) {
+            using U = typename std::decay_t<decltype(v)>::value_type;
+            U* to = alloc<U>(v.size());
+            if (!v.empty()) CK(cudaMemcpyAsync(to, v.data(), v.size() * sizeof(U), cudaMemcpyHostToDevice, st));
+            return to;
+        };
+        Four<T>* val = alloc<Four<T>>(size_t(p.groups) * 32);
+        Places* place = alloc<Places>(size_t(p.groups) * 32);
+        T* lval = alloc<T>(size_t(p.long_entries));
+        auto* lplace = alloc<unsigned short>(size_t(p.long_entries));
+        panels[which] = {put(p.panels), put(p.slice), put(p.order), put(p.cols), val, place, put(p.longrow), lval, lplace};
+        npanels[which] = int(p.panels.size()), panel_most[which] = p.most;
+        const PanelMat<T>& q = panels[which];
+        k_panel_fill<T><<<npanels[which], kThreads, 0, st>>>(q.panels, q.slice, q.order, q.cols, q.longrow, d.ptr, d.idx,
+                                                             static_cast<const T*>(d.val), val, place, lval, lplace);
+        CK(cudaGetLastError());
     }
     // Internal row order (contexts built from a model whose rows are of both kinds, short (<= kShort nonzeros)
     // and long): rows sorted by ascending length (stable). The row phase's blocks then hold rows of similar length,
@@ -361,7 +404,10 @@ struct Engine final : EngineBase {
         // indices renumbered), so both phases sum exactly as before
         Csr hAp;
         Entries<int32_t> at_idx;
-        const bool reorder = order_rows(hA, mAT, hAp, at_idx);
+        // panels keep the model's row order, in which neighbouring rows share columns
+        PanelPlan panels_a, panels_t;
+        plan_panels(ref(hA), mAT, flags, panels_a, panels_t);
+        const bool reorder = panels_a.empty() && order_rows(hA, mAT, hAp, at_idx);
         const CsrRef uA = ref(reorder ? hAp : hA);
         CsrRef uAT = mAT;
         if (reorder) uAT.idx = at_idx.data();
@@ -400,6 +446,7 @@ struct Engine final : EngineBase {
             k_narrow<T><<<g, 256, 0, st>>>(nz, va, static_cast<T*>(A.val));
             k_narrow<T><<<g, 256, 0, st>>>(nz, vt, static_cast<T*>(AT.val));
         }
+        put_panels(0, A, panels_a), put_panels(1, AT, panels_t);
         if (m) CK(cudaMemcpyAsync(P.Dr.data(), dr, size_t(m) * sizeof(double), cudaMemcpyDeviceToHost, st));
         if (n) CK(cudaMemcpyAsync(P.Dc.data(), dc, size_t(n) * sizeof(double), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
@@ -484,7 +531,7 @@ struct Engine final : EngineBase {
         int which = 0;
         for (DevMat* d : {&A, &AT}) {
             const int slot = which++;
-            if (d->nblk == 0) continue;
+            if (d->nblk == 0 || npanels[slot]) continue;
             const bool small = d->nnz < (int64_t(1) << 20);  // timings are noise
             const bool short_rows = d->maxrow <= kShort;      // every row on the thread path of policy 0
             // the thread-per-row kernel: bit-identical with short rows; otherwise (FP32, rows up to kMid) it sums
@@ -575,6 +622,16 @@ struct Engine final : EngineBase {
     template <class X, class E>
     void rowblock(const DevMat& a, const X* xin, const E& epi, const int* skip = nullptr, bool programmatic = false) {
         if (a.nblk == 0) return;
+        const int which = &a == &AT ? 1 : 0;
+        if constexpr (std::is_same<X, T>::value) {
+            if (npanels[which]) {  // `skip` only spares work
+                const PanelWork<1>* whole = nullptr;
+                CK(launch_panels(panels[which], npanels[which], panel_most[which], xin, whole, nullptr,
+                                 panel_step(epi), st));
+                ++launches;
+                return;
+            }
+        }
         if (a.per_thread)
             launch(k_rowthread<T, X, E>, (a.rows + kThreads - 1) / kThreads, programmatic, a.rows,
                    (const int*)a.ptr, (const int*)a.idx, static_cast<const T*>(a.val), xin, skip, epi);
@@ -614,7 +671,8 @@ struct Engine final : EngineBase {
         resident_blocks(A, sms), resident_blocks(AT, sms);
         resident_ctas = std::min(sms, std::max(A.rnblk, AT.rnblk));
         cluster_ctas = 0;
-        if (A.per_thread || AT.per_thread || tuned[0] == 2 || tuned[1] == 2) return;  // the tuner's choice for the phases
+        // the tuner's choice for the phases, or panels
+        if (A.per_thread || AT.per_thread || tuned[0] == 2 || tuned[1] == 2 || npanels[0]) return;
         resident_iterates = mode >= 1 || std::max(A.rnblk, AT.rnblk) <= kTeams * sms;
         if (mode == 1 || A.maxrow > kTile || AT.maxrow > kTile || m > kClusterRows || n > kClusterRows) return;
         // One cluster where its time, about 1 us an iteration + 41 ns a KB of x and z + 40 ns a thousand nonzeros, is below
@@ -712,7 +770,7 @@ struct Engine final : EngineBase {
             launches += 2 * int64_t(h_out[1]);  // the products, as when each is a launch of its own
             return h_out[0];
         }
-        if (resident_ctas > 0) {
+        if (resident_ctas > 0 && npanels[0] == 0) {
             launch_resident(k_resident_power<T>, sizeof(RowSmem<T>), 0,
                             resident_args(h_out), pv, pw, iters, red_grid(n));
             CK(cudaStreamSynchronize(st));

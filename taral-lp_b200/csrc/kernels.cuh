@@ -23,6 +23,7 @@ constexpr int kThreads = 256;  // threads per CTA in every SpMV-shaped kernel
 constexpr int kTile = 2044;    // nonzeros staged per row block: with the 16-byte alignment slack, 512 quads
 constexpr int kRowsMax = 256;  // rows per row block (one epilogue row per thread)
 constexpr int kRedThreads = 256;
+constexpr int kRedCtas = 296;  // most CTAs of a reduction
 // Resident CTAs per SM the row-block kernels are compiled for, by product type: 8 (32 registers) with float
 // products; 5 (48 registers) with double products, whose staging registers would otherwise spill to local memory
 // (measured on the bench LP's row phase in FP64: 55.7 us at 8 CTAs with spills, 40.2 us at 5 without).
@@ -618,10 +619,16 @@ __device__ __forceinline__ void reduce_finish(double (&v)[K], double* part, unsi
     if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     __syncthreads();
     if (last) {
+        // the partials are loaded all at once, then added in CTA order by a thread per value (a thread that also loads them
+        // waits for every load: 9.6 us a reduction at 126 CTAs, 4 us so)
+        __shared__ double all[kRedCtas * K];
         __threadfence();
+        for (unsigned i = threadIdx.x; i < gridDim.x * K; i += blockDim.x) all[i] = __ldcg(part + i);
+        __syncthreads();
         if (threadIdx.x < K) {
             double s = 0;
-            for (unsigned b = 0; b < gridDim.x; ++b) s += __ldcg(part + b * K + threadIdx.x);
+#pragma unroll 8
+            for (unsigned b = 0; b < gridDim.x; ++b) s += all[b * K + threadIdx.x];
             out[threadIdx.x] = s;
         }
         if (threadIdx.x == 0) *ticket = 0;

@@ -1,0 +1,472 @@
+// Products with matrices whose rows share columns: panels of rows with the columns they use in shared memory.
+//
+// What bounds the row-block kernels (kernels.cuh) on such a matrix -- a multi-period model, where the rows of a period use
+// the columns of that period -- is neither HBM (6-12 % busy) nor the arithmetic but L1: a warp's 32 gathered entries lie in
+// about 28 cache lines, one tag lookup each, whether they hit or not. Shared memory serves 32 random words in 3-4 cycles.
+//   panel  -- consecutive rows (kPanelRows at most) and the sorted list of the columns they use (kPanelCols at most). A
+//             CTA copies those entries of the gathered vector to shared memory once and gathers there.
+//   slices -- the panel's rows of at most kShort nonzeros, sorted by descending length, in groups of 32: a lane per row,
+//             its entries in order, four at a time, stored so that a warp reads 32 x 16 (or 32) bytes of values and 32 x 8
+//             bytes of 16-bit positions in the column list. Rows are filled up with zero values at a position that
+//             holds zero.
+//   long   -- longer rows, a warp each with its lanes strided; four sums at a time (4 / W rows of W instances) share one
+//             shuffle tree whose first two levels split them between the lanes (6 exchanges instead of 20).
+//   W      -- instances that share the matrix (batches): their entries of one column are neighbours in shared memory, one
+//             gather serves all W, and the panel's matrix entries and column list are read once for them.
+// Every row's products and summation order are those of the row blocks (block_sums), so the results are the same bits; the
+// sums go through shared memory, so that the fused step reads and writes its vectors in row order.
+#pragma once
+#include <algorithm>
+#include <cstdint>
+#include <vector>
+
+#include "host.hpp"
+#include "kernels.cuh"
+
+namespace taral {
+
+constexpr int kPanelRows = 1024, kPanelCols = 6144;
+constexpr int kPanelThreads = 512;
+struct Panel {
+    int row0, rows;      // rows of the matrix
+    int slice0, slices;  // slices of 32 short rows
+    int long0, nlong;    // longer rows
+    int col0, cols;      // the column list
+};
+// Device arrays of one matrix (or of several, one after another): entries of slice s at (slice[s].x + k) * 32 + lane, k <
+// slice[s].y; order[32 s + lane]: the lane's row in its panel, 0xffff: none. Long row q = {first entry in lval / lplace,
+// entries, row in its panel, -}.
+template <class T>
+struct alignas(16) Four {
+    T v[4];
+};
+struct alignas(8) Places {
+    unsigned short p[4];
+};
+template <class T>
+struct PanelMat {
+    const Panel* panels;
+    const int2* slice;
+    const unsigned short* order;
+    const int* cols;
+    const Four<T>* val;
+    const Places* place;
+    const int4* longrow;
+    const T* lval;
+    const unsigned short* lplace;
+};
+// A CTA's work in a batch: a panel and up to W instances; row shifts and gather offsets as for k_rowblock_batch.
+template <int W>
+struct alignas(16) PanelWork {
+    int panel, inst[W], row[W], gather[W];
+};
+
+// Fused steps on a row's sum, with the constants of its instance formed once per CTA (scale: two doubles per instance):
+// load the row's operands, then apply.
+template <class Y>
+struct PanelStore {
+    Y* y;
+    struct Ops {};
+    __device__ __forceinline__ double2 scale(int) const { return make_double2(0, 0); }
+    __device__ __forceinline__ Ops load(int) const { return {}; }
+    __device__ __forceinline__ void apply(int r, double s, double2, const Ops&) const { y[r] = Y(s); }
+};
+template <class T>
+struct PanelRow {  // EpiRow, the division by sigma as in dual_prox
+    T *Ax, *z;
+    double* zs;
+    const T *rl, *ru;
+    const double* par;
+    struct Ops { T z, ax, rl, ru; double zs; };
+    __device__ __forceinline__ double2 scale(int inst) const { return make_double2(par[2 * inst + 1], 1.0 / par[2 * inst + 1]); }
+    __device__ __forceinline__ Ops load(int r) const { return {z[r], Ax[r], rl[r], ru[r], zs[r]}; }
+    __device__ __forceinline__ void apply(int r, double s, double2 k, const Ops& o) const {
+        const T st = T(s);
+        const T zn = T(dual_prox(double(o.z) + k.x * (2.0 * double(st) - double(o.ax)), double(o.rl), double(o.ru), k.x, k.y));
+        Ax[r] = st, z[r] = zn, zs[r] = o.zs + double(zn);
+    }
+};
+template <class T>
+struct PanelCol {  // EpiCol
+    T *ATz, *x;
+    double* xs;
+    const T *c, *l, *u;
+    const double* par;
+    int upd;
+    struct Ops { T x, c, l, u; double xs; };
+    __device__ __forceinline__ double2 scale(int inst) const { return make_double2(par[2 * inst], 0); }
+    __device__ __forceinline__ Ops load(int r) const {
+        if (!upd) return {T(0), T(0), T(0), T(0), 0.0};
+        return {x[r], c[r], l[r], u[r], xs[r]};
+    }
+    __device__ __forceinline__ void apply(int r, double s, double2 k, const Ops& o) const {
+        const T st = T(s);
+        ATz[r] = st;
+        if (upd) {
+            const T xn = T(clampv(double(o.x) - k.x * (double(o.c) + double(st)), double(o.l), double(o.u)));
+            x[r] = xn, xs[r] = o.xs + double(xn);
+        }
+    }
+};
+
+template <class X, int W>
+constexpr size_t panel_smem(int cols, int rows, int nlong) {
+    return (size_t(cols) + 1) * W * sizeof(X) + 16 + (size_t(rows) * W + 1) * sizeof(double) + size_t(nlong) * sizeof(int4);
+}
+
+// A lane's entries of R long rows q .. q + R - 1 (below end): STRIDES strides of 32 from entry k of each.
+template <class T, int R, int STRIDES>
+struct LongRows {
+    T m[R][STRIDES];
+    unsigned c[R][STRIDES / 2];  // places, two to a register
+    __device__ __forceinline__ int place(int r, int e) const { return int(e & 1 ? c[r][e / 2] >> 16 : c[r][e / 2] & 0xffff); }
+    __device__ __forceinline__ void load(const PanelMat<T>& a, const int4* heads, int q, int end, int none, int k) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int2 h = q + r < end ? *reinterpret_cast<const int2*>(heads + q + r) : make_int2(0, 0);
+#pragma unroll
+            for (int e = 0; e < STRIDES; ++e) {
+                const bool in = k + 32 * e < h.y;
+                m[r][e] = in ? __ldg(a.lval + h.x + k + 32 * e) : T(0);
+                const unsigned p = in ? __ldg(a.lplace + h.x + k + 32 * e) : unsigned(none);  // the entry that holds zero
+                c[r][e / 2] = e & 1 ? c[r][e / 2] | p << 16 : p;
+            }
+        }
+    }
+};
+
+// One CTA per panel (work NULL: panel blockIdx.x, one instance) or per work item. A panel's latency is what a phase of a
+// single LP takes, so every load that does not need the gathered entries is issued before the copy of those is waited for:
+// the first long rows of each warp here, and in the loop the next ones before the current are summed.
+template <class T, class X, int W, class E>
+__global__ void __launch_bounds__(kPanelThreads, 2) k_panel(const PanelMat<T> a, const X* __restrict__ xin,
+                                                            const PanelWork<W>* __restrict__ work,
+                                                            const int* __restrict__ active, E epi) {
+    using P = typename ProdT<T, X>::type;
+    constexpr int kWarps = kPanelThreads / 32, R = 4 / W, STRIDES = W == 4 ? 4 : 2;
+    extern __shared__ __align__(16) unsigned char raw[];
+    __shared__ double2 scale[W];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const Panel p = a.panels[work ? work[blockIdx.x].panel : int(blockIdx.x)];
+    const int* list = a.cols + p.col0;
+    constexpr int kAtOnce = 4;
+    int c0[kAtOnce];  // the first columns this thread copies
+#pragma unroll
+    for (int i = 0; i < kAtOnce; ++i) c0[i] = tid + i * kPanelThreads < p.cols ? __ldg(list + tid + i * kPanelThreads) : -1;
+    X* xs = reinterpret_cast<X*>(raw);
+    double* sums = reinterpret_cast<double*>(raw + ((size_t(p.cols + 1) * W * sizeof(X) + 15) & ~size_t(15)));
+    int4* heads = reinterpret_cast<int4*>(sums + (size_t(p.rows) * W + 1) / 2 * 2);
+    for (int q = tid; q < p.nlong; q += kPanelThreads) heads[q] = __ldg(a.longrow + p.long0 + q);
+    // a warp's long rows are consecutive
+    const int per = ((p.nlong + kWarps - 1) / kWarps + R - 1) / R * R, lq0 = warp * per, lq1 = min(p.nlong, lq0 + per);
+    LongRows<T, R, STRIDES> rows;
+    int gather[W];
+    bool on[W];
+    if (work) {
+        int any = 0;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            const int i = work[blockIdx.x].inst[w];
+            on[w] = i >= 0 && (!active || active[i]);
+            gather[w] = work[blockIdx.x].gather[w], any |= on[w];
+            if (tid == w) scale[w] = on[w] ? epi.scale(i) : make_double2(0, 0);
+        }
+        if (!any) return;  // the same for the whole CTA
+    } else {
+        on[0] = true, gather[0] = 0;
+        if (tid == 0) scale[0] = epi.scale(0);
+    }
+    __syncthreads();
+    {
+        X g[kAtOnce][W];
+#pragma unroll
+        for (int i = 0; i < kAtOnce; ++i)
+#pragma unroll
+            for (int w = 0; w < W; ++w) g[i][w] = c0[i] >= 0 && on[w] ? __ldg(xin + gather[w] + c0[i]) : X(0);
+        rows.load(a, heads, lq0, lq1, p.cols, lane);
+#pragma unroll
+        for (int i = 0; i < kAtOnce; ++i)
+            if (c0[i] >= 0)
+#pragma unroll
+                for (int w = 0; w < W; ++w) xs[(tid + i * kPanelThreads) * W + w] = g[i][w];
+    }
+#pragma unroll 4
+    for (int i = tid + kAtOnce * kPanelThreads; i < p.cols; i += kPanelThreads) {
+        const int c = __ldg(list + i);
+#pragma unroll
+        for (int w = 0; w < W; ++w) xs[i * W + w] = on[w] ? __ldg(xin + gather[w] + c) : X(0);
+    }
+    if (tid < W) xs[p.cols * W + tid] = X(0);
+    __syncthreads();
+    // long rows: R at a time, four sums per lane
+    for (int q0 = lq0; q0 < lq1; q0 += R) {
+        LongRows<T, R, STRIDES> now = rows;
+        rows.load(a, heads, q0 + R, lq1, p.cols, lane);  // the next rows' entries, while these are summed
+        double v[4] = {0, 0, 0, 0};
+        int longest = 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) longest = max(longest, q0 + r < lq1 ? heads[q0 + r].y : 0);
+        for (int k = lane;; now.load(a, heads, q0, lq1, p.cols, k)) {
+#pragma unroll
+            for (int e = 0; e < STRIDES; ++e)
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+#pragma unroll
+                    for (int w = 0; w < W; ++w) v[r * W + w] += double(mul_rn(P(now.m[r][e]), P(xs[now.place(r, e) * W + w])));
+            k += 32 * STRIDES;
+            if (k - lane >= longest) break;
+        }
+        // each lane keeps two of the four sums, then one; a sum's tree is that of xor 16, 8, 4, 2, 1
+        const bool hi = lane & 16, odd = lane & 8;
+        double s0 = hi ? v[2] : v[0], s1 = hi ? v[3] : v[1];
+        s0 += __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], 16);
+        s1 += __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], 16);
+        double s = odd ? s1 : s0;
+        s += __shfl_xor_sync(0xffffffffu, odd ? s0 : s1, 8);
+        for (int off = 4; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+        const int which = lane >> 3, r = which / W, w = which % W;
+        if ((lane & 7) == 0 && q0 + r < lq1) sums[w * p.rows + heads[q0 + r].z] = s;
+    }
+    // slices, the last warps first: the first ones have the most long rows
+    for (int s = kWarps - 1 - warp; s < p.slices; s += kWarps) {
+        const int2 sl = __ldg(a.slice + p.slice0 + s);
+        const int local = a.order[32 * (p.slice0 + s) + lane];
+        const Four<T>* val = a.val + size_t(sl.x) * 32 + lane;
+        const Places* place = a.place + size_t(sl.x) * 32 + lane;
+        double sum[W];
+#pragma unroll
+        for (int w = 0; w < W; ++w) sum[w] = 0;
+        constexpr int G = W > 1 && sizeof(T) == 4 ? 4 : 2;  // groups of four entries in flight
+        for (int k = 0; k < sl.y; k += G) {
+            Four<T> v[G];
+            Places c[G];
+#pragma unroll
+            for (int g = 0; g < G; ++g)
+                if (k + g < sl.y) v[g] = val[32 * (k + g)], c[g] = place[32 * (k + g)];
+#pragma unroll
+            for (int g = 0; g < G; ++g)
+                if (k + g < sl.y) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const X* from = xs + int(c[g].p[e]) * W;
+#pragma unroll
+                        for (int w = 0; w < W; ++w) sum[w] += double(mul_rn(P(v[g].v[e]), P(from[w])));
+                    }
+                }
+        }
+        if (local < p.rows) {
+#pragma unroll
+            for (int w = 0; w < W; ++w) sums[w * p.rows + local] = sum[w];
+        }
+    }
+    __syncthreads();
+    int shift[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) shift[w] = p.row0 + (work ? work[blockIdx.x].row[w] : 0);
+    for (int t = tid; t < p.rows; t += kPanelThreads) {
+        typename E::Ops ops[W];
+#pragma unroll
+        for (int w = 0; w < W; ++w)
+            if (on[w]) ops[w] = epi.load(shift[w] + t);
+#pragma unroll
+        for (int w = 0; w < W; ++w)
+            if (on[w]) epi.apply(shift[w] + t, sums[w * p.rows + t], scale[w], ops[w]);
+    }
+}
+
+// The slices' entries from the CSR matrix (a CTA per panel): values, and positions in the panel's column list found by
+// bisection in shared memory.
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_panel_fill(const Panel* __restrict__ panels, const int2* __restrict__ slice,
+                                                         const unsigned short* __restrict__ order, const int* __restrict__ cols,
+                                                         const int4* __restrict__ longrow, const int* __restrict__ ptr,
+                                                         const int* __restrict__ idx, const T* __restrict__ val,
+                                                         Four<T>* out, Places* place, T* lval, unsigned short* lplace) {
+    __shared__ int list[kPanelCols];
+    const Panel p = panels[blockIdx.x];
+    for (int i = threadIdx.x; i < p.cols; i += kThreads) list[i] = cols[p.col0 + i];
+    __syncthreads();
+    auto find = [&](int want) {
+        int lo = 0, hi = p.cols - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (list[mid] < want) lo = mid + 1;
+            else hi = mid;
+        }
+        return (unsigned short)lo;
+    };
+    const int lane = threadIdx.x & 31;
+    for (int q = threadIdx.x >> 5; q < p.nlong; q += kThreads / 32) {
+        const int4 row = longrow[p.long0 + q];
+        const int b = ptr[p.row0 + row.z];
+        for (int k = lane; k < row.y; k += 32) lval[row.x + k] = val[b + k], lplace[row.x + k] = find(idx[b + k]);
+    }
+    for (int s = threadIdx.x >> 5; s < p.slices; s += kThreads / 32) {
+        const int2 sl = slice[p.slice0 + s];
+        const int local = order[32 * (p.slice0 + s) + lane];
+        const int b = local < p.rows ? ptr[p.row0 + local] : 0, len = local < p.rows ? ptr[p.row0 + local + 1] - b : 0;
+        for (int k = 0; k < sl.y; ++k) {
+            Four<T> v;
+            Places c;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int at = 4 * k + e;
+                if (at >= len) {
+                    v.v[e] = T(0), c.p[e] = (unsigned short)p.cols;
+                    continue;
+                }
+                v.v[e] = val[b + at], c.p[e] = find(idx[b + at]);
+            }
+            out[(size_t(sl.x) + k) * 32 + lane] = v, place[(size_t(sl.x) + k) * 32 + lane] = c;
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------ host side
+struct PanelSize {  // the largest panel's columns, rows and long rows
+    int cols = 0, rows = 0, nlong = 0;
+    void cover(const PanelSize& o) { cols = std::max(cols, o.cols), rows = std::max(rows, o.rows), nlong = std::max(nlong, o.nlong); }
+};
+struct PanelPlan {
+    std::vector<Panel> panels;
+    std::vector<int2> slice;
+    std::vector<unsigned short> order;
+    std::vector<int4> longrow;
+    std::vector<int> cols;
+    int groups = 0;             // entry groups of 32 lanes x 4
+    int long_entries = 0;
+    int64_t padded = 0;         // entries stored
+    PanelSize most;
+    bool empty() const { return panels.empty(); }
+    void append(const PanelPlan& p, int row_shift) {
+        for (Panel h : p.panels) {
+            h.row0 += row_shift, h.slice0 += int(slice.size()), h.long0 += int(longrow.size()), h.col0 += int(cols.size());
+            panels.push_back(h);
+        }
+        for (int2 q : p.slice) slice.push_back(make_int2(q.x + groups, q.y));
+        for (int4 q : p.longrow) longrow.push_back(make_int4(q.x + long_entries, q.y, q.z, 0));
+        order.insert(order.end(), p.order.begin(), p.order.end());
+        cols.insert(cols.end(), p.cols.begin(), p.cols.end());
+        groups += p.groups, long_entries += p.long_entries, padded += p.padded;
+        most.cover(p.most);
+    }
+};
+
+// Panels of about `target` nonzeros and at most max_cols columns for the rows [first, last); empty where a single row uses
+// more columns than that.
+template <class I>
+PanelPlan panels_of(const I* ptr, const int32_t* idx, int first, int last, int cols, int target, int max_cols) {
+    PanelPlan plan;
+    std::vector<int> seen(size_t(cols), 0), list;
+    int stamp = 0, low = 0, high = 0;
+    auto unique = [&](int r0, int r1) {  // columns of the rows [r0, r1) into list, unsorted, all of them in [low, high]
+        list.clear(), ++stamp, low = cols, high = -1;
+        for (I k = ptr[r0]; k < ptr[r1]; ++k) {
+            const int c = idx[k];
+            if (seen[size_t(c)] != stamp) seen[size_t(c)] = stamp, list.push_back(c), low = std::min(low, c), high = std::max(high, c);
+        }
+    };
+    auto len = [&](int r) { return int(ptr[r + 1] - ptr[r]); };
+    std::vector<int> by, shorter, count(size_t(kShort) + 2);
+    for (int r0 = first; r0 < last;) {
+        int r1 = r0;
+        while (r1 < last && r1 - r0 < kPanelRows && (r1 == r0 || ptr[r1 + 1] - ptr[r0] <= I(target))) ++r1;
+        for (unique(r0, r1); int(list.size()) > max_cols; unique(r0, r1)) {  // too many columns: half the rows
+            if (r1 - r0 == 1) return PanelPlan();
+            r1 = r0 + (r1 - r0) / 2;
+        }
+        Panel p{};
+        p.row0 = r0, p.rows = r1 - r0, p.slice0 = int(plan.slice.size()), p.col0 = int(plan.cols.size()), p.cols = int(list.size());
+        p.long0 = int(plan.longrow.size());
+        if (int64_t(high) - low < 16 * int64_t(list.size())) {  // in column order: the marks of the range
+            for (int c = low; c <= high; ++c)
+                if (seen[size_t(c)] == stamp) plan.cols.push_back(c);
+        } else {
+            std::sort(list.begin(), list.end());
+            plan.cols.insert(plan.cols.end(), list.begin(), list.end());
+        }
+        // long rows in row order, the others by descending length (stable counting sort)
+        shorter.clear(), std::fill(count.begin(), count.end(), 0);
+        for (int r = r0; r < r1; ++r) {
+            const int l = len(r);
+            if (l > kShort) {
+                plan.longrow.push_back(make_int4(plan.long_entries, l, r - r0, 0));
+                plan.long_entries += l, plan.padded += l;
+            } else {
+                shorter.push_back(r), ++count[size_t(kShort - l) + 1];
+            }
+        }
+        p.nlong = int(plan.longrow.size()) - p.long0;
+        for (size_t l = 1; l < count.size(); ++l) count[l] += count[l - 1];
+        by.resize(shorter.size());
+        for (int r : shorter) by[size_t(count[size_t(kShort - len(r))]++)] = r;
+        for (size_t t = 0; t < by.size(); t += 32) {
+            const int width = (len(by[t]) + 3) / 4;
+            plan.slice.push_back(make_int2(plan.groups, width));
+            plan.groups += width, plan.padded += 128 * int64_t(width);
+            for (size_t l = t; l < t + 32; ++l) plan.order.push_back(l < by.size() ? (unsigned short)(by[l] - r0) : 0xffff);
+        }
+        p.slices = int(plan.slice.size()) - p.slice0;
+        plan.most.cover({p.cols, p.rows, p.nlong});
+        plan.panels.push_back(p);
+        r0 = r1;
+    }
+    return plan;
+}
+
+// Panels for the CSR rows on `threads` host threads (max_cols <= kPanelCols), or none where they do not pay: the column
+// lists must hold at most a third as many columns as the panels hold nonzeros (a list and its entries of x cost about as
+// much to read as they save otherwise), and padding at most 40 % of the nonzeros.
+template <class I>
+PanelPlan build_panels(const I* ptr, const int32_t* idx, int rows, int cols, int target, int max_cols, int threads) {
+    PanelPlan plan;
+    if (rows == 0 || ptr[rows] == ptr[0]) return plan;
+    for (int r = 0; r < rows; ++r)
+        if (ptr[r + 1] - ptr[r] > I(kTile)) return plan;  // summed by a whole CTA in the row blocks
+    const int64_t all = int64_t(ptr[rows] - ptr[0]);
+    auto pays = [](const PanelPlan& p, int64_t nnz) { return nnz >= 3 * int64_t(p.cols.size()) && 10 * p.padded <= 14 * nnz; };
+    {  // a look at a few rows first: most matrices without shared columns are refused here
+        PanelPlan look;
+        int64_t nnz = 0;
+        for (int q = 0; q < 4; ++q) {
+            const int r0 = int(int64_t(rows) * q / 4);
+            int r1 = r0;
+            while (r1 < rows && ptr[r1] - ptr[r0] < I(target)) ++r1;
+            const PanelPlan p = panels_of(ptr, idx, r0, r1, cols, target, max_cols);
+            if (p.empty()) return plan;
+            look.append(p, 0), nnz += int64_t(ptr[r1] - ptr[r0]);
+        }
+        if (!pays(look, nnz)) return plan;
+    }
+    threads = int(std::max<int64_t>(1, std::min<int64_t>(threads, all / (8 * int64_t(target)))));
+    std::vector<PanelPlan> part(static_cast<size_t>(threads));
+    split_ranges(threads, threads, [&](int, int64_t q0, int64_t q1) {
+        for (int64_t q = q0; q < q1; ++q) {
+            auto cut = [&](int64_t k) {
+                return k >= threads ? rows : int(std::lower_bound(ptr, ptr + rows, ptr[0] + I(all * k / threads)) - ptr);
+            };
+            part[size_t(q)] = panels_of(ptr, idx, cut(q), cut(q + 1), cols, target, max_cols);
+        }
+    });
+    for (const PanelPlan& p : part) plan.append(p, 0);
+    int covered = 0;
+    for (const Panel& p : plan.panels) covered += p.rows;
+    return covered == rows && pays(plan, all) ? plan : PanelPlan();
+}
+
+// The panel counterparts of the row blocks' fused steps.
+template <class Y> PanelStore<Y> panel_step(const EpiStore<Y>& e) { return {e.y}; }
+template <class T> PanelRow<T> panel_step(const EpiRow<T>& e) { return {e.Ax, e.z, e.zs, e.rl, e.ru, e.par}; }
+template <class T> PanelCol<T> panel_step(const EpiCol<T>& e) { return {e.ATz, e.x, e.xs, e.c, e.l, e.u, e.par, e.upd}; }
+
+template <class T, int W, class E>
+cudaError_t launch_panels(const PanelMat<T>& a, int ctas, const PanelSize& most, const T* xin, const PanelWork<W>* work,
+                          const int* active, const E& step, cudaStream_t st) {
+    const size_t smem = panel_smem<T, W>(most.cols, most.rows, most.nlong);
+    const cudaError_t e = cudaFuncSetAttribute(k_panel<T, T, W, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e != cudaSuccess) return e;
+    k_panel<T, T, W, E><<<ctas, kPanelThreads, smem, st>>>(a, xin, work, active, step);
+    return cudaGetLastError();
+}
+
+}  // namespace taral

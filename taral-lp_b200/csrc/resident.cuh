@@ -338,7 +338,7 @@ __device__ __forceinline__ void team_sums(double (&v)[K], const Team& t, double*
 // and the current point's partial sums, a barrier, the average's partial sums; the CTA that finishes last adds the
 // partials. The partials are those of k_eval_row / k_eval_col at gr / gc CTAs -- a team takes their CTAs one after
 // another -- and are added in the same order, so the scalars are the same bits. `out` may be pinned host memory.
-constexpr int kEvalCtas = 296;  // most CTAs of one reduction (red_grid)
+constexpr int kEvalCtas = kRedCtas;
 template <class T>
 __global__ void __launch_bounds__(kThreads * kTeams, 1) k_resident_eval(const ResidentArgs<T> a, double f, int gr, int gc) {
     extern __shared__ __align__(16) unsigned char raw[];

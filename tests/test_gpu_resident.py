@@ -22,6 +22,13 @@ CASES = {
 }
 
 
+PANEL_CASES = {
+    "refinery_2": CASES["refinery_2"],      # long rows and slices, panels over several periods
+    "dense_columns": lambda: lpgen.planted(40, 900, 5, seed=3),   # A: 40 rows of ~112 on 900 columns; A^T: 900 rows of 5 on 40
+    "transport_9x30": lambda: lpgen.transport(9, 30, seed=4),
+}
+
+
 def _record(lp, precision):
     e = pdhg.Engine.from_model(lp, precision=precision)
     norm = e.power_norm(200)
@@ -55,6 +62,23 @@ def test_resident_launches_change_nothing(engine_lib, monkeypatch, case, precisi
 
 
 @pytest.mark.parametrize("precision", [pdhg.FP64, pdhg.FP32], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("case", sorted(PANEL_CASES))
+def test_panels_change_nothing(engine_lib, monkeypatch, case, precision):
+    """Products by panels (csrc/panels.cuh; TARAL_PANELS=1 takes them at any size where the columns are shared) against
+    the row blocks in the same row order."""
+    lp = PANEL_CASES[case]()
+    monkeypatch.setenv("TARAL_TUNE", "0")
+    monkeypatch.setenv("TARAL_ROWORDER", "0")
+    monkeypatch.setenv("TARAL_RESIDENT", "0")
+    got = []
+    for flag in ("0", "1"):
+        monkeypatch.setenv("TARAL_PANELS", flag)
+        got.append(_record(lp, precision))
+    for k, (a, b) in enumerate(zip(*got)):
+        assert np.array_equal(a, b, equal_nan=True), (k, np.max(np.abs(a - b)))
+
+
+@pytest.mark.parametrize("precision", [pdhg.FP64, pdhg.FP32], ids=["fp64", "fp32"])
 @pytest.mark.parametrize("shape", ["one_cta", "several_ctas", "shared_matrix"])
 def test_batch_clusters_change_nothing(engine_lib, monkeypatch, shape, precision):
     """A batch of small LPs on one cluster each against the batch's phase kernels: the same norms, iterations and points,
@@ -73,6 +97,27 @@ def test_batch_clusters_change_nothing(engine_lib, monkeypatch, shape, precision
         got.append(b.solve() + b.solve())  # the second solve replays the captured launches
         b.close()
     for (r0, x0, y0), (r1, x1, y1) in zip((got[0][:3], got[0][3:]), (got[1][:3], got[1][3:])):
+        for a, c in zip(r0, r1):
+            assert (a["status"], a["iterations"], a["restarts"], a["norm_a"]) == (c["status"], c["iterations"], c["restarts"], c["norm_a"])
+        assert all(np.array_equal(p, q) for p, q in zip(x0 + y0, x1 + y1))
+
+
+@pytest.mark.parametrize("precision", [pdhg.FP64, pdhg.FP32], ids=["fp64", "fp32"])
+def test_batch_panels_change_nothing(engine_lib, monkeypatch, precision):
+    """A batch's phases on panels, several instances to a CTA (7 and 2 of two matrices: full and partly used groups),
+    against the row blocks; instances stop at different blocks, so the lists are rebuilt on the way."""
+    base = lpgen.RefineryBase(2, seed=5)
+    pert = lpgen.perturbations(9, seed=8)
+    lps = [base.instance(2, p) for p in pert[:7]] + [base.instance(1, p) for p in pert[7:]]
+    monkeypatch.setenv("TARAL_TUNE", "0")
+    got = []
+    for flag in ("0", "1"):
+        monkeypatch.setenv("TARAL_PANELS", flag)
+        b = pdhg.Batch(lps, tol=1e-4, max_iter=20_000, precision=precision, time_limit=120)
+        got.append((b.solve(), b.solve()))  # the second solve restores the full lists
+        b.close()
+    assert len({r["iterations"] for r in got[0][0][0]}) > 2
+    for (r0, x0, y0), (r1, x1, y1) in zip(*got):
         for a, c in zip(r0, r1):
             assert (a["status"], a["iterations"], a["restarts"], a["norm_a"]) == (c["status"], c["iterations"], c["restarts"], c["norm_a"])
         assert all(np.array_equal(p, q) for p, q in zip(x0 + y0, x1 + y1))
