@@ -188,8 +188,39 @@ __global__ void __launch_bounds__(kThreads, 6) k_pack_spmv(const int* __restrict
     if (mine) epi.finish(vbase + tid, my_inst, tid, sm.rowsum[tid], st);
 }
 
-// Per-(CTA, slot) partial sums of the row (ROW = true) or column KKT scalars over one pack block, CTAs in
-// evaluation order (gpu/pdhg.cu:236-251 and :253-271); f per instance (1 for the current point).
+// One row's (ROW) or column's terms of the KKT scalars (gpu/pdhg.cu:236-251 and :253-271) at vector index r; f per
+// instance (1 for the current point). Row: a = Ax (or A xs), b = z (or zs); column: a = x (or xs), b = ATz (or A^T zs), c_v =
+// c, lo_v = l, up_v = u.
+template <bool ROW, class T, class V>
+__device__ __forceinline__ void kkt_terms(double (&v)[5], int r, double f, const V* __restrict__ a, const V* __restrict__ b,
+                                          const T* __restrict__ lo_v, const T* __restrict__ up_v,
+                                          const T* __restrict__ c_v, const T* __restrict__ D,
+                                          const T* __restrict__ last) {
+    if (ROW) {
+        double ax = double(a[r]) * f, zz = double(b[r]) * f, lo = lo_v[r], up = up_v[r];
+        double res = ax < lo ? lo - ax : (ax > up ? ax - up : 0), ro = res / double(D[r]);
+        double rr = ro * row_rel_weight(lo, up, double(D[r]));
+        v[0] += res * res, v[1] += ro * ro, v[2] += rr * rr;
+        if (zz > 0 && up < INFINITY) v[3] -= zz * up;
+        if (zz < 0 && lo > -INFINITY) v[3] -= zz * lo;
+        double dz = zz - double(last[r]);
+        v[4] += dz * dz;
+    } else {
+        double xx = double(a[r]) * f, cj = c_v[r], d = cj + double(b[r]) * f, lo = lo_v[r], up = up_v[r], res = 0;
+        v[2] += cj * xx;
+        if (d > 0) {
+            if (lo > -INFINITY) v[3] += d * lo;
+            else res = d;
+        } else if (d < 0) {
+            if (up < INFINITY) v[3] += d * up;
+            else res = -d;
+        }
+        double ro = res / double(D[r]), dx = xx - double(last[r]);
+        v[0] += res * res, v[1] += ro * ro, v[4] += dx * dx;
+    }
+}
+
+// Per-(CTA, slot) partial sums of the KKT scalars over one pack block, CTAs in evaluation order.
 // part[(cta * 8 + slot) * 5 + k].
 template <class T, class V, bool ROW>
 __global__ void __launch_bounds__(kThreads) k_pack_eval(const int4* __restrict__ blk, const int4* __restrict__ ext,
@@ -208,32 +239,7 @@ __global__ void __launch_bounds__(kThreads) k_pack_eval(const int4* __restrict__
     const double f = live && fi ? fi[inst] : 1.0;
     double v[5] = {0, 0, 0, 0, 0};
     if (live)
-        for (int q = tid; q < (nrows << lw); q += kThreads) {
-            const int r = vbase + q;
-            if (ROW) {  // a = Ax (or A xs), b = z (or zs)
-                double ax = double(a[r]) * f, zz = double(b[r]) * f, lo = lo_v[r], up = up_v[r];
-                double res = ax < lo ? lo - ax : (ax > up ? ax - up : 0), ro = res / double(D[r]);
-                double rr = ro * row_rel_weight(lo, up, double(D[r]));
-                v[0] += res * res, v[1] += ro * ro, v[2] += rr * rr;
-                if (zz > 0 && up < INFINITY) v[3] -= zz * up;
-                if (zz < 0 && lo > -INFINITY) v[3] -= zz * lo;
-                double dz = zz - double(last[r]);
-                v[4] += dz * dz;
-            } else {  // a = x (or xs), b = ATz (or A^T zs); c_v = c, lo_v = l, up_v = u
-                double xx = double(a[r]) * f, cj = c_v[r], d = cj + double(b[r]) * f, lo = lo_v[r], up = up_v[r],
-                       res = 0;
-                v[2] += cj * xx;
-                if (d > 0) {
-                    if (lo > -INFINITY) v[3] += d * lo;
-                    else res = d;
-                } else if (d < 0) {
-                    if (up < INFINITY) v[3] += d * up;
-                    else res = -d;
-                }
-                double ro = res / double(D[r]), dx = xx - double(last[r]);
-                v[0] += res * res, v[1] += ro * ro, v[4] += dx * dx;
-            }
-        }
+        for (int q = tid; q < (nrows << lw); q += kThreads) kkt_terms<ROW>(v, vbase + q, f, a, b, lo_v, up_v, c_v, D, last);
     __shared__ double sh[kThreads / 32][8][5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
@@ -249,6 +255,39 @@ __global__ void __launch_bounds__(kThreads) k_pack_eval(const int4* __restrict__
             for (int i = 0; i < kThreads / 32; ++i) s += sh[i][t][k];
         part[(size_t(blockIdx.x) * 8 + t) * 5 + k] = s;
     }
+}
+
+// The same partial sums where every pack has one slot, a warp per block: it takes the block's rows 32 at a time, as the
+// warps of k_pack_eval's CTA do, and adds the 32-row sums in order. Blocks of a multi-period model hold about 45 rows, so a
+// CTA per block is a launch of thousands of CTAs that last as long as their chain of loads (75-85 us for 48 refinery
+// scenarios; a warp per block 19-37 us).
+template <class T, class V, bool ROW>
+__global__ void __launch_bounds__(kThreads) k_warp_eval(int blocks, const int4* __restrict__ blk, const int4* __restrict__ ext,
+                                                         const int* __restrict__ slot_inst,
+                                                         const int* __restrict__ active, const double* __restrict__ fi,
+                                                         const V* __restrict__ a, const V* __restrict__ b,
+                                                         const T* __restrict__ lo_v, const T* __restrict__ up_v,
+                                                         const T* __restrict__ c_v, const T* __restrict__ D,
+                                                         const T* __restrict__ last, double* part) {
+    const int block = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (block >= blocks) return;
+    const int4 e4 = __ldg(ext + block);
+    const int nrows = __ldg(blk + block).y & 0xffff, inst = slot_inst[8 * e4.x];
+    if (inst < 0 || !active[inst]) return;  // nobody reads the partials of a stopped instance
+    const double f = fi ? fi[inst] : 1.0;
+    double total[5] = {0, 0, 0, 0, 0};
+    for (int q0 = 0; q0 < nrows; q0 += 32) {
+        double v[5] = {0, 0, 0, 0, 0};
+        if (q0 + lane < nrows) kkt_terms<ROW>(v, e4.y + q0 + lane, f, a, b, lo_v, up_v, c_v, D, last);
+        for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+            for (int k = 0; k < 5; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], off);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) total[k] += v[k];
+    }
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < 5; ++k) part[size_t(block) * 40 + k] = total[k];
 }
 
 // Sums of `count` consecutive partials of K values each, in order: the CTA loads a chunk of them at once, then thread k
@@ -427,6 +466,45 @@ __global__ void k_pack_pow_scale(const int4* __restrict__ blk, const int4* __res
     const double sc = scale[inst];
     for (int q = threadIdx.x; q < (nrows << lw); q += blockDim.x) v[vbase + q] = T(double(v[vbase + q]) * sc);
 }
+// Both where every pack has one slot: the partial sums by a warp per block (as k_warp_eval), the scaling over the
+// instances' whole vectors (range {first entry, entries} per first instance, blockIdx.y).
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_warp_pow_part(int blocks, const int4* __restrict__ blk, const int4* __restrict__ ext,
+                                                             const int* __restrict__ slot_inst, const int* __restrict__ active,
+                                                             const T* __restrict__ v, double* part) {
+    const int block = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (block >= blocks) return;
+    const int4 e4 = __ldg(ext + block);
+    const int nrows = __ldg(blk + block).y & 0xffff, inst = slot_inst[8 * e4.x];
+    if (inst < 0 || !active[inst]) return;
+    double total = 0;
+    for (int q0 = 0; q0 < nrows; q0 += 32) {
+        const double t = q0 + lane < nrows ? double(v[e4.y + q0 + lane]) : 0.0;
+        double a = 0.0 + t * t;
+        for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+        total += a;
+    }
+    if (lane == 0) part[size_t(block) * 8] = total;
+}
+// The first instances' start vectors (k_power_start for all of them).
+template <class T>
+__global__ void k_power_starts(const int4* __restrict__ first, const int2* __restrict__ range, const int* __restrict__ width,
+                               const double* __restrict__ norm, T* __restrict__ v) {
+    const int2 r = range[blockIdx.y];
+    const int W = width[blockIdx.y], slot = first[blockIdx.y].y;
+    const double nrm = norm[blockIdx.y];
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < r.y; j += gridDim.x * blockDim.x)
+        v[size_t(r.x) + size_t(j) * W + slot] = T(power_entry(unsigned(j)) / nrm);
+}
+template <class T>
+__global__ void k_flat_pow_scale(const int4* __restrict__ first, const int2* __restrict__ range, const int* __restrict__ active,
+                                 const double* __restrict__ scale, T* __restrict__ v) {
+    const int inst = first[blockIdx.y].z;
+    if (!active[inst]) return;
+    const double sc = scale[inst];
+    const int2 r = range[blockIdx.y];
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < r.y; j += gridDim.x * blockDim.x) v[r.x + j] = T(double(v[r.x + j]) * sc);
+}
 
 // Download: out = (avg ? sum * f : point) for every used slot.
 template <class T>
@@ -538,6 +616,9 @@ struct Batch final : BatchBase {
     int npw_ev = 0;
     int4 *pw_ev = nullptr, *pwe_ev = nullptr, *pw_first = nullptr;
     int *pw_range = nullptr, *pw_taken = nullptr;
+    int2* pw_cols = nullptr;    // the columns of the first instances' packs: {first entry, entries of one slot}
+    int* pw_width = nullptr;    // and the packs' widths
+    double* pw_norm = nullptr;  // the start vectors' norms, by matrix
     cudaGraphExec_t pgraph = nullptr;  // a chunk of power-iteration steps
     // small instances, each on one cluster (cluster.cuh): all of them, and the first of every distinct matrix
     int cluster_ctas = 0;
@@ -916,14 +997,15 @@ struct Batch final : BatchBase {
 
     // ------------------------------------------------------------------ panels
     // Every phase of a batch on panels of the distinct matrices, kPW instances that share a matrix to a CTA. On 48
-    // refinery scenarios of 12 matrices (22.6M products a phase, FP32) a row phase takes @ROW us (row blocks 72), a column
-    // phase @COL (55). From a million nonzeros over the instances, where panels fill the SMs. TARAL_PANELS=0: none.
+    // refinery scenarios of 12 matrices (22.6M products a phase, FP32) a row phase takes 42 us (row blocks 72), a column
+    // phase 33 (55). From a million nonzeros over the instances, where panels fill the SMs. TARAL_PANELS=0: none.
     static constexpr int kPW = sizeof(T) == 4 ? 4 : 2;
     static constexpr int kPanelTarget = 24576, kBatchPanelCols = 4096;
     PanelMat<T> panels[2];
     int npanels[2] = {0, 0};
     PanelSize panel_most[2];
-    std::vector<int> first_panel[2];                       // of every matrix, and the end
+    std::vector<Panel> h_panels[2];                        // on the host, and the first of every matrix, and the end
+    std::vector<int> first_panel[2];
     PanelWork<kPW>* panel_work[2] = {nullptr, nullptr};    // the running instances' CTAs
     PanelWork<1>* panel_first[2] = {nullptr, nullptr};     // the power iteration's
     int npanel_work[2] = {0, 0};
@@ -952,7 +1034,7 @@ struct Batch final : BatchBase {
             T* lval = alloc<T>(size_t(all.long_entries));
             auto* lplace = alloc<unsigned short>(size_t(all.long_entries));
             panels[k] = {put(all.panels), put(all.slice), put(all.order), put(all.cols), val, place, put(all.longrow), lval, lplace};
-            npanels[k] = int(all.panels.size()), panel_most[k] = all.most;
+            npanels[k] = int(all.panels.size()), panel_most[k] = all.most, h_panels[k] = all.panels;
             k_panel_fill<T><<<npanels[k], kThreads, 0, s>>>(panels[k].panels, panels[k].slice, panels[k].order, panels[k].cols,
                                                             panels[k].longrow, k ? Tptr : Aptr, k ? Tidx : Aidx, k ? Tval : Aval, val,
                                                             place, lval, lplace);
@@ -977,15 +1059,15 @@ struct Batch final : BatchBase {
                 for (int p = first_panel[k][q]; p < first_panel[k][q + 1]; ++p) {
                     for (size_t u = 0; u < users[q].size(); u += kPW) {
                         PanelWork<kPW> w;
-                        w.panel = p;
+                        w.panel = h_panels[k][size_t(p)];
                         for (int t = 0; t < kPW; ++t) {
-                            w.inst[t] = -1, w.row[t] = 0, w.gather[t] = 0;
-                            if (u + size_t(t) < users[q].size()) entry(w, t, users[q][u + size_t(t)]);
+                            entry(w, t, users[q][u + size_t(t) < users[q].size() ? u + size_t(t) : u]);
+                            if (u + size_t(t) >= users[q].size()) w.inst[t] = -1;
                         }
                         work.push_back(w);
                     }
                     PanelWork<1> f;
-                    f.panel = p, entry(f, 0, first_inst[q]);
+                    f.panel = h_panels[k][size_t(p)], entry(f, 0, first_inst[q]);
                     first.push_back(f);
                 }
             if (!panel_work[k]) {  // every instance is live: the longest lists
@@ -1024,15 +1106,26 @@ struct Batch final : BatchBase {
         pw_lists[0].n1 = pick(h_a1, h_ae1, first_of, pw_lists[0].blk1, pw_lists[0].ext1), pw_lists[0].np = pick(h_ap, h_ae, pack_of, pw_lists[0].blkp, pw_lists[0].extp);
         pw_lists[1].n1 = pick(h_t1, h_te1, first_of, pw_lists[1].blk1, pw_lists[1].ext1), pw_lists[1].np = pick(h_tp, h_te, pack_of, pw_lists[1].blkp, pw_lists[1].extp);
         std::vector<int4> ev, eve, first;
+        std::vector<int2> cols_of;
+        std::vector<int> widths;
+        std::vector<std::pair<int, int>> by_n;  // (columns, matrix)
+        std::vector<double> norms(static_cast<size_t>(distinct));
         std::vector<int> range{0};
         for (int k = 0; k < distinct; ++k) {
             const int i = first_inst[size_t(k)];
             const int2 at = where[size_t(i)];
             for (int b = hcr[size_t(at.x)]; b < hcr[size_t(at.x) + 1]; ++b) ev.push_back(t_ev[size_t(b)]), eve.push_back(te_ev[size_t(b)]);
             first.push_back(make_int4(at.x, at.y, i, 0)), range.push_back(int(ev.size()));
+            cols_of.push_back(make_int2(packs[size_t(at.x)].cbase, mats[size_t(k)]->S.n));
+            widths.push_back(packs[size_t(at.x)].W);
+            by_n.emplace_back(mats[size_t(k)]->S.n, k);
         }
+        std::sort(by_n.begin(), by_n.end());  // the norms are sums over prefixes of one sequence
+        double nn = 0;
+        int done = 0;
+        for (const auto& q : by_n) nn = power_norm2(nn, done, q.first), done = q.first, norms[size_t(q.second)] = std::sqrt(nn);
         npw_ev = int(ev.size());
-        pw_ev = put(ev), pwe_ev = put(eve), pw_first = put(first), pw_range = put(range), pw_taken = alloc<int>(size_t(distinct));
+        pw_ev = put(ev), pwe_ev = put(eve), pw_first = put(first), pw_range = put(range), pw_cols = put(cols_of), pw_width = put(widths), pw_norm = put(norms), pw_taken = alloc<int>(size_t(distinct));
     }
 
     // Small instances on one cluster each (cluster.cuh): where the launch's waves of clusters, at about 0.9 us an iteration
@@ -1224,16 +1317,24 @@ struct Batch final : BatchBase {
         spmv_A(x, EpiStore<T>{Ax}, act);
         spmv_T(z, EpiStore<T>{ATz}, act);
     }
+    template <class V, bool ROW, class... Args>
+    void eval_blocks(int blocks, const int4* blk, const int4* ext, Args... args) {
+        if (blocks == 0) return;
+        if (packs.size() == size_t(ninst))  // one slot each
+            k_warp_eval<T, V, ROW><<<(blocks + 7) / 8, kThreads, 0, s>>>(blocks, blk, ext, slot_inst, args...);
+        else
+            k_pack_eval<T, V, ROW><<<blocks, kThreads, 0, s>>>(blk, ext, slot_inst, args...);
+    }
     void eval_into(double* dst, bool avg, const int* act) {
         const double* fi = avg ? fbuf : nullptr;
         if (!avg) {
-            if (nA) k_pack_eval<T, T, true><<<nA, kThreads, 0, s>>>(A_ev, Ae_ev, slot_inst, act, fi, Ax, z, rl, ru, nullptr, Dr, zlast, partA);
-            if (nT) k_pack_eval<T, T, false><<<nT, kThreads, 0, s>>>(T_ev, Te_ev, slot_inst, act, fi, x, ATz, l, u, c, Dc, xlast, partT);
+            eval_blocks<T, true>(nA, A_ev, Ae_ev, act, fi, Ax, z, rl, ru, (const T*)nullptr, Dr, zlast, partA);
+            eval_blocks<T, false>(nT, T_ev, Te_ev, act, fi, x, ATz, l, u, c, Dc, xlast, partT);
         } else {
             spmv_A(xs, EpiStore<double>{tmpM}, act);
             spmv_T(zs, EpiStore<double>{tmpN}, act);
-            if (nA) k_pack_eval<T, double, true><<<nA, kThreads, 0, s>>>(A_ev, Ae_ev, slot_inst, act, fi, tmpM, zs, rl, ru, nullptr, Dr, zlast, partA);
-            if (nT) k_pack_eval<T, double, false><<<nT, kThreads, 0, s>>>(T_ev, Te_ev, slot_inst, act, fi, xs, tmpN, l, u, c, Dc, xlast, partT);
+            eval_blocks<double, true>(nA, A_ev, Ae_ev, act, fi, tmpM, zs, rl, ru, (const T*)nullptr, Dr, zlast, partA);
+            eval_blocks<double, false>(nT, T_ev, Te_ev, act, fi, xs, tmpN, l, u, c, Dc, xlast, partT);
         }
         k_eval_finish<<<ninst, kFinishThreads, 0, s>>>(d_where, rr, cr, partA, partT, act, dst);
         launches += 3;
@@ -1329,9 +1430,13 @@ struct Batch final : BatchBase {
             T *a = pv, *b = pu;
             for (int k = 0; k < chunk; ++k) {
                 power_spmv(0, a, pw), power_spmv(1, pw, b);
-                if (npw_ev) k_pack_pow_part<T><<<npw_ev, kThreads, 0, s>>>(pw_ev, pwe_ev, slot_inst, pactive, b, partT);
+                const bool single = packs.size() == size_t(ninst);  // one slot each
+                if (npw_ev && single) k_warp_pow_part<T><<<(npw_ev + 7) / 8, kThreads, 0, s>>>(npw_ev, pw_ev, pwe_ev, slot_inst, pactive, b, partT);
+                else if (npw_ev) k_pack_pow_part<T><<<npw_ev, kThreads, 0, s>>>(pw_ev, pwe_ev, slot_inst, pactive, b, partT);
                 k_pow_update<<<distinct, kFinishThreads, 0, s>>>(pw_first, pw_range, partT, est, pscale, pactive, pw_taken);
-                if (npw_ev) k_pack_pow_scale<T><<<npw_ev, kThreads, 0, s>>>(pw_ev, pwe_ev, slot_inst, pactive, pscale, b);
+                if (npw_ev && single)
+                    k_flat_pow_scale<T><<<dim3(unsigned(std::max(1, std::min(64, 592 / distinct))), unsigned(distinct)), kThreads, 0, s>>>(pw_first, pw_cols, pactive, pscale, b);
+                else if (npw_ev) k_pack_pow_scale<T><<<npw_ev, kThreads, 0, s>>>(pw_ev, pwe_ev, slot_inst, pactive, pscale, b);
                 launches += 3;
                 std::swap(a, b);
             }
@@ -1388,17 +1493,7 @@ struct Batch final : BatchBase {
         BK(cudaEventCreate(&e1));
         BK(cudaEventRecord(e0, s));
         // power iteration per instance (gpu/pdhg.cu:416-436)
-        std::vector<double> h(N);
-        for (int i = 0; i < ninst; ++i) {
-            int n = models[i]->n;
-            double nn = 0;
-            std::vector<double> v0(static_cast<size_t>(n));
-            for (int j = 0; j < n; ++j) v0[j] = 0.5 + double((uint32_t(j) * 2654435761u) % 1000u) / 1000.0;
-            for (int j = 0; j < n; ++j) nn += v0[j] * v0[j];
-            for (int j = 0; j < n; ++j) h[xidx(i, j)] = v0[j] / std::sqrt(nn);
-        }
-        BK(cudaMemcpyAsync(dout, h.data(), size_t(N) * sizeof(double), cudaMemcpyHostToDevice, s));
-        k_cast<T><<<std::max(1, std::min((N + 255) / 256, 1184)), 256, 0, s>>>(N, dout, pv);
+        k_power_starts<T><<<dim3(unsigned(std::max(1, std::min(64, 592 / distinct))), unsigned(distinct)), 256, 0, s>>>(pw_first, pw_cols, pw_width, pw_norm, pv);
         // One estimate per distinct matrix: instances that share a matrix share its scaled copy, its row blocks and
         // the deterministic start vector, so their power iterations are the same numbers; only the first instance
         // of each matrix iterates, the others take its estimate.

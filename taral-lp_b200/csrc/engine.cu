@@ -267,8 +267,8 @@ struct Engine final : EngineBase {
         finish_init(hc_ptr, hl, hu, hrl_ptr, hru_ptr, hDr, hDc);
     }
     // Panels (panels.cuh) for A and A^T, both or neither, from 1.5M nonzeros in FP64 and 3M in FP32: a panel's latency is
-    // about 7 us. Refinery LPs, us an iteration with row blocks / panels: 1.1M nonzeros FP64 15.1 / 17.0, FP32 11.8 / 16.0;
-    // 2.3M FP64 31.3 / 20.9, FP32 16.3 / 18.4; 3.4M FP64 42.0 / 31.6, FP32 23.3 / 21.3. Panels of half an SM's share of the nonzeros, 8,192 to 16,384: smaller ones
+    // about 7 us. Refinery LPs, us an iteration with row blocks / panels: 1.1M nonzeros FP64 15.1 / 14.7, FP32 11.7 / 13.6;
+    // 2.3M FP64 31.3 / 19.5, FP32 16.1 / 17.2; 3.4M FP64 42.0 / 27.3, FP32 22.9 / 19.8. Panels of half an SM's share of the nonzeros, 8,192 to 16,384: smaller ones
     // reread too many columns, larger ones leave SMs idle. TARAL_PANELS=0: none (tests).
     PanelMat<T> panels[2];
     int npanels[2] = {0, 0};
@@ -755,12 +755,7 @@ struct Engine final : EngineBase {
 
     // ------------------------------------------------------------------ backend concept
     double power_norm(int iters) override {
-        std::vector<double> h(n);
-        double nn = 0;
-        for (int j = 0; j < n; ++j) h[j] = 0.5 + double((uint32_t(j) * 2654435761u) % 1000u) / 1000.0, nn += h[j] * h[j];
-        for (int j = 0; j < n; ++j) h[j] = h[j] / std::sqrt(nn);
-        if (n) CK(cudaMemcpyAsync(d_in, h.data(), size_t(n) * sizeof(double), cudaMemcpyHostToDevice, st));
-        k_cast<T><<<grid_for(n), 256, 0, st>>>(n, d_in, pv);
+        k_power_start<T><<<grid_for(n), 256, 0, st>>>(n, std::sqrt(power_norm2(0.0, 0, n)), pv);
         CK(cudaMemsetAsync(pst, 0, 4 * sizeof(double), st));
         CK(cudaMemsetAsync(pdone, 0, sizeof(int), st));
         launches += 1;

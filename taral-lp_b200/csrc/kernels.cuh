@@ -802,9 +802,20 @@ __global__ void k_scale_out(int n, double f, const V* __restrict__ src, double* 
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) dst[j] = double(src[j]) * f;
 }
 
+// The power iteration's start (gpu/pdhg.cu:419-423): entry j is (1/2 + ((j * 2654435761) mod 2^32 mod 1000) / 1000) / norm.
+// The norm's sum of squares runs in index order, on the host: nn over the first `from` entries
+// continued to `to`.
+__host__ __device__ inline double power_entry(unsigned j) { return 0.5 + double((j * 2654435761u) % 1000u) / 1000.0; }
+inline double power_norm2(double nn, int from, int to) {
+    for (int j = from; j < to; ++j) {
+        const double h = power_entry(unsigned(j));
+        nn += h * h;
+    }
+    return nn;
+}
 template <class T>
-__global__ void k_cast(int n, const double* __restrict__ src, T* __restrict__ dst) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) dst[j] = T(src[j]);
+__global__ void k_power_start(int n, double norm, T* __restrict__ v) {
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) v[j] = T(power_entry(unsigned(j)) / norm);
 }
 
 }  // namespace taral

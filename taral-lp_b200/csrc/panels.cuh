@@ -55,10 +55,12 @@ struct PanelMat {
     const T* lval;
     const unsigned short* lplace;
 };
-// A CTA's work in a batch: a panel and up to W instances; row shifts and gather offsets as for k_rowblock_batch.
+// A CTA's work in a batch: a panel and up to W instances; row shifts and gather offsets as for k_rowblock_batch. An unused
+// slot has inst -1 and the shifts of slot 0.
 template <int W>
 struct alignas(16) PanelWork {
-    int panel, inst[W], row[W], gather[W];
+    Panel panel;
+    int inst[W], row[W], gather[W];
 };
 
 // Fused steps on a row's sum, with the constants of its instance formed once per CTA (scale: two doubles per instance):
@@ -137,7 +139,8 @@ struct LongRows {
 
 // One CTA per panel (work NULL: panel blockIdx.x, one instance) or per work item. A panel's latency is what a phase of a
 // single LP takes, so every load that does not need the gathered entries is issued before the copy of those is waited for:
-// the first long rows of each warp here, and in the loop the next ones before the current are summed.
+// the first long rows of each warp here, and in the loop the next ones before the current are summed. (More rows in
+// flight per warp spill, and ranges prefetched into L2 compete with the loads: 10% slower each.)
 template <class T, class X, int W, class E>
 __global__ void __launch_bounds__(kPanelThreads, 2) k_panel(const PanelMat<T> a, const X* __restrict__ xin,
                                                             const PanelWork<W>* __restrict__ work,
@@ -147,7 +150,7 @@ __global__ void __launch_bounds__(kPanelThreads, 2) k_panel(const PanelMat<T> a,
     extern __shared__ __align__(16) unsigned char raw[];
     __shared__ double2 scale[W];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const Panel p = a.panels[work ? work[blockIdx.x].panel : int(blockIdx.x)];
+    const Panel p = work ? work[blockIdx.x].panel : a.panels[blockIdx.x];
     const int* list = a.cols + p.col0;
     constexpr int kAtOnce = 4;
     int c0[kAtOnce];  // the first columns this thread copies
@@ -182,7 +185,7 @@ __global__ void __launch_bounds__(kPanelThreads, 2) k_panel(const PanelMat<T> a,
 #pragma unroll
         for (int i = 0; i < kAtOnce; ++i)
 #pragma unroll
-            for (int w = 0; w < W; ++w) g[i][w] = c0[i] >= 0 && on[w] ? __ldg(xin + gather[w] + c0[i]) : X(0);
+            for (int w = 0; w < W; ++w) g[i][w] = c0[i] >= 0 ? __ldg(xin + gather[w] + c0[i]) : X(0);
         rows.load(a, heads, lq0, lq1, p.cols, lane);
 #pragma unroll
         for (int i = 0; i < kAtOnce; ++i)
@@ -194,27 +197,33 @@ __global__ void __launch_bounds__(kPanelThreads, 2) k_panel(const PanelMat<T> a,
     for (int i = tid + kAtOnce * kPanelThreads; i < p.cols; i += kPanelThreads) {
         const int c = __ldg(list + i);
 #pragma unroll
-        for (int w = 0; w < W; ++w) xs[i * W + w] = on[w] ? __ldg(xin + gather[w] + c) : X(0);
+        for (int w = 0; w < W; ++w) xs[i * W + w] = __ldg(xin + gather[w] + c);
     }
     if (tid < W) xs[p.cols * W + tid] = X(0);
     __syncthreads();
     // long rows: R at a time, four sums per lane
     for (int q0 = lq0; q0 < lq1; q0 += R) {
-        LongRows<T, R, STRIDES> now = rows;
+        const LongRows<T, R, STRIDES> now = rows;
         rows.load(a, heads, q0 + R, lq1, p.cols, lane);  // the next rows' entries, while these are summed
         double v[4] = {0, 0, 0, 0};
-        int longest = 0;
+        auto add = [&](const LongRows<T, R, STRIDES>& x, int left) {  // left: entries of the longest row from here on
 #pragma unroll
-        for (int r = 0; r < R; ++r) longest = max(longest, q0 + r < lq1 ? heads[q0 + r].y : 0);
-        for (int k = lane;; now.load(a, heads, q0, lq1, p.cols, k)) {
-#pragma unroll
-            for (int e = 0; e < STRIDES; ++e)
+            for (int e = 0; e < STRIDES; ++e) {
+                if (32 * e >= left) break;  // the same for the whole warp
 #pragma unroll
                 for (int r = 0; r < R; ++r)
 #pragma unroll
-                    for (int w = 0; w < W; ++w) v[r * W + w] += double(mul_rn(P(now.m[r][e]), P(xs[now.place(r, e) * W + w])));
-            k += 32 * STRIDES;
-            if (k - lane >= longest) break;
+                    for (int w = 0; w < W; ++w) v[r * W + w] += double(mul_rn(P(x.m[r][e]), P(xs[x.place(r, e) * W + w])));
+            }
+        };
+        int longest = 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) longest = max(longest, q0 + r < lq1 ? heads[q0 + r].y : 0);
+        add(now, longest);
+        for (int k = 32 * STRIDES; k < longest; k += 32 * STRIDES) {
+            LongRows<T, R, STRIDES> more;
+            more.load(a, heads, q0, lq1, p.cols, k + lane);
+            add(more, longest - k);
         }
         // each lane keeps two of the four sums, then one; a sum's tree is that of xor 16, 8, 4, 2, 1
         const bool hi = lane & 16, odd = lane & 8;
@@ -266,8 +275,7 @@ __global__ void __launch_bounds__(kPanelThreads, 2) k_panel(const PanelMat<T> a,
     for (int t = tid; t < p.rows; t += kPanelThreads) {
         typename E::Ops ops[W];
 #pragma unroll
-        for (int w = 0; w < W; ++w)
-            if (on[w]) ops[w] = epi.load(shift[w] + t);
+        for (int w = 0; w < W; ++w) ops[w] = epi.load(shift[w] + t);  // of every slot: no branch between the loads
 #pragma unroll
         for (int w = 0; w < W; ++w)
             if (on[w]) epi.apply(shift[w] + t, sums[w * p.rows + t], scale[w], ops[w]);
