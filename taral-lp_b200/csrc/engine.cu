@@ -122,32 +122,30 @@ int forced_row_split() {
     return e ? std::max(0, std::min(kPolicies - 1, std::atoi(e))) : -1;
 }
 
-std::vector<int4> build_row_blocks(const int64_t* ptr, int rows, int tile, int rows_max) {
+// End of the block that starts at row r: rows while they fit, or one longer row.
+template <class I>
+static int block_end(const I* ptr, int rows, int r, int tile, int rows_max) {
+    const int last = int(std::min<int64_t>(rows, int64_t(r) + rows_max));
+    const I* e = std::upper_bound(ptr + r + 1, ptr + last + 1, I(ptr[r] + tile)) - 1;
+    return std::max(r + 1, int(e - ptr));
+}
+template <class I>
+static std::vector<int4> row_blocks(const I* ptr, int rows, int tile, int rows_max) {
     std::vector<int4> out;
     // y: rows | kUniformCandidate when no row is much longer than the mean | kLongRows when one exceeds kShort
-    auto close = [&](int r0, int r1) {
-        int64_t mx = 0;
-        for (int r = r0; r < r1; ++r) mx = std::max<int64_t>(mx, ptr[r + 1] - ptr[r]);
+    for (int r0 = 0, r1; r0 < rows; r0 = r1) {
+        r1 = block_end(ptr, rows, r0, tile, rows_max);
+        I mx = 0;
+        for (int r = r0; r < r1; ++r) mx = std::max<I>(mx, ptr[r + 1] - ptr[r]);
         const int64_t nz = ptr[r1] - ptr[r0], mean = (nz + (r1 - r0) - 1) / (r1 - r0);
         const bool uniform = r1 - r0 > 1 && mx > kShort && mx <= 2 * mean + 8;
         out.push_back(make_int4(r0, (r1 - r0) | (uniform ? kUniformCandidate : 0) | (mx > kShort ? kLongRows : 0),
                                 int(ptr[r0]), int(ptr[r1])));
-    };
-    int start = 0, cur_rows = 0;
-    int64_t cur_nnz = 0;
-    for (int r = 0; r < rows; ++r) {
-        int64_t L = ptr[r + 1] - ptr[r];
-        if (L > tile) {  // a long row is a block of its own
-            if (cur_rows) close(start, r);
-            close(r, r + 1);
-            start = r + 1, cur_rows = 0, cur_nnz = 0;
-            continue;
-        }
-        if (cur_rows == rows_max || cur_nnz + L > tile) close(start, r), start = r, cur_rows = 0, cur_nnz = 0;
-        ++cur_rows, cur_nnz += L;
     }
-    if (cur_rows) close(start, rows);
     return out;
+}
+std::vector<int4> build_row_blocks(const int64_t* ptr, int rows, int tile, int rows_max) {
+    return row_blocks(ptr, rows, tile, rows_max);
 }
 
 static int grid_for(int64_t k) {  // elementwise kernels: grid-stride, at most 8 CTAs of 256 per SM
@@ -702,13 +700,17 @@ struct Engine final : EngineBase {
         const int teams = sms * kTeams;
         d.rblk = d.blk, d.rnblk = d.nblk;
         if (d.nblk > teams) return;
-        const std::vector<int64_t> p(d.hptr.begin(), d.hptr.end());
+        const int* p = d.hptr.data();
         std::vector<int4> list;
         for (double grow = 1;; grow *= 1.1) {
             const int tile = int(std::min<double>(kTile, std::max<double>(256, grow * double(d.nnz) / teams)));
             const int rows = int(std::min<double>(kRowsMax, std::max<double>(64, grow * d.rows / teams)));
-            list = build_row_blocks(p.data(), d.rows, tile, rows);
-            if (int(list.size()) <= teams) break;
+            int count = 0;
+            for (int r = 0; r < d.rows && count <= teams; ++count) r = block_end(p, d.rows, r, tile, rows);
+            if (count <= teams) {
+                list = row_blocks(p, d.rows, tile, rows);
+                break;
+            }
             if (tile == kTile && rows == kRowsMax) return;
         }
         d.rblk = alloc<int4>(list.size()), d.rnblk = int(list.size());
