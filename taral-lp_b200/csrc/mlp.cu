@@ -32,6 +32,7 @@
 
 #include "../../include/taral_pdhg.h"
 #include "mlp.cuh"
+#include "staging.hpp"
 
 namespace taral {
 namespace tc {
@@ -361,6 +362,7 @@ struct Mlp {
     int64_t steps = 0;
     cudaStream_t s = nullptr;
     std::vector<void*> allocs;
+    Staging host;  // large transfers from and to the caller's arrays
     std::string err;
 
     template <class U>
@@ -409,6 +411,9 @@ struct Mlp {
         MK(cudaMemsetAsync(d_err, 0, sizeof(int), s));
         ws_count = size_t(64) * mb * hid;  // split-K partials of dH = dZ W^T (K = out)
         ws = alloc<float>(ws_count);
+        size_t largest = size_t(mb) * out;
+        for (const Layer& y : L) largest = std::max(largest, size_t(y.in) * y.out);
+        host.prepare(largest * sizeof(float));
         MK(cudaStreamSynchronize(s));
     }
 
@@ -584,11 +589,11 @@ extern "C" int taral_mlp_set_params(taral_mlp* h, const float* params) {
         const float* p = params;
         for (auto& y : m.L) {
             size_t nw = size_t(y.in) * y.out;
-            MK(cudaMemcpyAsync(y.gW, p, nw * sizeof(float), cudaMemcpyHostToDevice, m.s));  // gW: the row-major form
+            MK(m.host.copy(y.gW, p, nw * sizeof(float), cudaMemcpyHostToDevice, m.s));  // gW: the row-major form
             taral::mlp::k_set_weights<<<m.grid2(y), 256, 0, m.s>>>(y.in, y.out, y.fused ? taral::mlp::blocked_groups(y.out) : 0,
                                                                    y.ldw, y.gW, y.W, y.Wb);
             p += nw;
-            MK(cudaMemcpyAsync(y.b, p, y.out * sizeof(float), cudaMemcpyHostToDevice, m.s));
+            MK(m.host.copy(y.b, p, y.out * sizeof(float), cudaMemcpyHostToDevice, m.s));
             p += y.out;
         }
         MK(cudaStreamSynchronize(m.s));
@@ -604,9 +609,9 @@ extern "C" int taral_mlp_get_params(taral_mlp* h, float* params) {
             size_t nw = size_t(y.in) * y.out;
             if (y.fused)
                 taral::mlp::k_get_weights<<<m.grid2(y), 256, 0, m.s>>>(y.in, y.out, taral::mlp::blocked_groups(y.out), y.W, y.gW);
-            MK(cudaMemcpyAsync(p, y.fused ? y.gW : y.W, nw * sizeof(float), cudaMemcpyDeviceToHost, m.s));
+            MK(m.host.copy(p, y.fused ? y.gW : y.W, nw * sizeof(float), cudaMemcpyDeviceToHost, m.s));
             p += nw;
-            MK(cudaMemcpyAsync(p, y.b, y.out * sizeof(float), cudaMemcpyDeviceToHost, m.s));
+            MK(m.host.copy(p, y.b, y.out * sizeof(float), cudaMemcpyDeviceToHost, m.s));
             p += y.out;
         }
         MK(cudaStreamSynchronize(m.s));
@@ -619,7 +624,7 @@ extern "C" int taral_mlp_forward(taral_mlp* h, int batch, const float* x, float*
         Mlp& m = h->m;
         m.load_input(batch, x);
         m.forward(batch);
-        MK(cudaMemcpyAsync(y, m.L[m.depth].Z, size_t(batch) * m.out_dim * sizeof(float), cudaMemcpyDeviceToHost, m.s));
+        MK(m.host.copy(y, m.L[m.depth].Z, size_t(batch) * m.out_dim * sizeof(float), cudaMemcpyDeviceToHost, m.s));
         MK(cudaStreamSynchronize(m.s));
         m.check_tc();
     })
@@ -631,7 +636,7 @@ extern "C" int taral_mlp_gradients(taral_mlp* h, int batch, const float* x, cons
     MLP_GUARD(h, {
         Mlp& m = h->m;
         m.load_input(batch, x);
-        MK(cudaMemcpyAsync(m.Tf, target, size_t(batch) * m.out_dim * sizeof(float), cudaMemcpyHostToDevice, m.s));
+        MK(m.host.copy(m.Tf, target, size_t(batch) * m.out_dim * sizeof(float), cudaMemcpyHostToDevice, m.s));
         m.forward(batch);
         m.backward(batch, m.Tf, nullptr, nullptr);
         const double l = m.loss(batch);
@@ -641,9 +646,9 @@ extern "C" int taral_mlp_gradients(taral_mlp* h, int batch, const float* x, cons
             float* p = grads;
             for (auto& y : m.L) {
                 size_t nw = size_t(y.in) * y.out;
-                MK(cudaMemcpyAsync(p, y.gW, nw * sizeof(float), cudaMemcpyDeviceToHost, m.s));
+                MK(m.host.copy(p, y.gW, nw * sizeof(float), cudaMemcpyDeviceToHost, m.s));
                 p += nw;
-                MK(cudaMemcpyAsync(p, y.gb, y.out * sizeof(float), cudaMemcpyDeviceToHost, m.s));
+                MK(m.host.copy(p, y.gb, y.out * sizeof(float), cudaMemcpyDeviceToHost, m.s));
                 p += y.out;
             }
             MK(cudaStreamSynchronize(m.s));
@@ -657,8 +662,8 @@ extern "C" int taral_mlp_set_dataset(taral_mlp* h, int count, const float* x, co
         Mlp& m = h->m;
         if (m.DX) throw MlpError{"dataset already set"};
         m.DX = m.alloc<float>(size_t(count) * m.in_dim), m.DT = m.alloc<float>(size_t(count) * m.out_dim);
-        MK(cudaMemcpyAsync(m.DX, x, size_t(count) * m.in_dim * sizeof(float), cudaMemcpyHostToDevice, m.s));
-        MK(cudaMemcpyAsync(m.DT, target, size_t(count) * m.out_dim * sizeof(float), cudaMemcpyHostToDevice, m.s));
+        MK(m.host.copy(m.DX, x, size_t(count) * m.in_dim * sizeof(float), cudaMemcpyHostToDevice, m.s));
+        MK(m.host.copy(m.DT, target, size_t(count) * m.out_dim * sizeof(float), cudaMemcpyHostToDevice, m.s));
         m.d_perm = m.alloc<int>(size_t(count));
         MK(cudaStreamSynchronize(m.s));
         m.dcount = count;

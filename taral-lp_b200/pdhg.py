@@ -515,23 +515,21 @@ class Mlp:
         self._err(lib().taral_mlp_set_params(self.h, p.ctypes.data_as(_fp)))
 
     def get_params(self):
-        p = np.zeros(self.param_count, np.float32)
+        p = np.empty(self.param_count, np.float32)
         self._err(lib().taral_mlp_get_params(self.h, p.ctypes.data_as(_fp)))
         return p
 
     def forward(self, x):
         x = _f32(np.atleast_2d(x))
-        y = np.zeros((x.shape[0], self.dims[3]), np.float32)
+        y = np.empty((x.shape[0], self.dims[3]), np.float32)
         for b0 in range(0, x.shape[0], self.max_batch):
-            xb = _f32(x[b0:b0 + self.max_batch])
-            yb = np.zeros((xb.shape[0], self.dims[3]), np.float32)
+            xb, yb = x[b0:b0 + self.max_batch], y[b0:b0 + self.max_batch]  # rows of C-contiguous arrays
             self._err(lib().taral_mlp_forward(self.h, xb.shape[0], xb.ctypes.data_as(_fp), yb.ctypes.data_as(_fp)))
-            y[b0:b0 + xb.shape[0]] = yb
         return y
 
     def gradients(self, x, t):
         x, t = _f32(x), _f32(t)
-        g = np.zeros(self.param_count, np.float32)
+        g = np.empty(self.param_count, np.float32)
         loss = C.c_double()
         self._err(lib().taral_mlp_gradients(self.h, x.shape[0], x.ctypes.data_as(_fp), t.ctypes.data_as(_fp),
                                             C.byref(loss), g.ctypes.data_as(_fp)))

@@ -101,3 +101,32 @@ def test_mlp_training_step_is_adam_on_the_gradients(engine_lib, dims, batch):
         # at most lr * 1e-5 * max|g| / (|g| + eps)
         slack = lr * np.minimum(2.0, 1e-5 * np.max(np.abs(g)) / (np.abs(g) + 1e-8))
         assert np.all(np.abs(w - expected) <= lr * 1e-4 + slack + 1.3e-7 * np.abs(expected)), step
+
+
+@pytest.mark.parametrize("entries", [(1 << 20) - 1, 1 << 20, (1 << 20) + 1, 20 * (1 << 17) - 3, 33 * (1 << 17) + 5])
+def test_mlp_large_transfers(engine_lib, entries, monkeypatch):
+    """Transfers below, at and above the size from which several threads share them, with ragged last chunks and fewer or
+    more chunks than threads: the same bytes as the runtime's own copies give, also into pinned memory."""
+    import torch
+    rng = np.random.default_rng(entries)
+    p = rng.standard_normal(2 * entries).astype(np.float32)  # one layer of 1 x entries: weights and biases
+    x = rng.standard_normal((1, 1)).astype(np.float32)
+    t = rng.standard_normal((1, entries)).astype(np.float32)
+    got = {}
+    for threads in ("0", "16", None):
+        if threads is None:
+            monkeypatch.delenv("TARAL_STAGING")
+        else:
+            monkeypatch.setenv("TARAL_STAGING", threads)
+        net = pdhg.Mlp(1, 8, 0, entries, max_batch=1)
+        net.set_params(p)
+        assert np.array_equal(net.get_params(), p)
+        pinned = torch.zeros(2 * entries, dtype=torch.float32, pin_memory=True)
+        net._err(pdhg.lib().taral_mlp_get_params(net.h, C.cast(pinned.data_ptr(), C.POINTER(C.c_float))))
+        assert np.array_equal(pinned.numpy(), p)
+        loss, g = net.gradients(x, t)
+        got[threads] = (net.forward(x), np.float64(loss), g)
+        net.close()
+    for threads in ("16", None):
+        for a, b in zip(got["0"], got[threads]):
+            assert np.array_equal(a, b)
