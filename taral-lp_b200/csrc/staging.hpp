@@ -36,7 +36,8 @@ public:
     // Slots for transfers of up to `largest` bytes; none where they cannot be had, and copy() then leaves it to the runtime.
     void prepare(size_t largest) {
         if (largest < kLeast || cudaGetDevice(&dev) != cudaSuccess) return;
-        int want = std::min<int>(kThreadsMax, int(std::thread::hardware_concurrency()));
+        // a slot for every 2 MB, so that pinning them (0.5 ms a MB) stays well below what one transfer of that size takes
+        int want = int(std::min<size_t>(largest >> 21, std::min<unsigned>(kThreadsMax, std::thread::hardware_concurrency())));
         if (const char* e = std::getenv("TARAL_STAGING")) want = std::min(kThreadsMax, std::atoi(e));  // 0: none (tests)
         if (want < 2 || cudaHostAlloc(reinterpret_cast<void**>(&pinned), size_t(want) * kChunk, cudaHostAllocDefault) != cudaSuccess) {
             cudaGetLastError();
