@@ -489,8 +489,9 @@ __global__ void __launch_bounds__(kThreads) k_warp_pow_part(int blocks, const in
 // The first instances' start vectors (k_power_start for all of them).
 template <class T>
 __global__ void k_power_starts(const int4* __restrict__ first, const int2* __restrict__ range, const int* __restrict__ width,
-                               const double* __restrict__ norm, T* __restrict__ v) {
+                               const double* __restrict__ norm, T* __restrict__ v, double* scale) {
     const int2 r = range[blockIdx.y];
+    if (blockIdx.x == 0 && threadIdx.x == 0) scale[first[blockIdx.y].z] = 1;
     const int W = width[blockIdx.y], slot = first[blockIdx.y].y;
     const double nrm = norm[blockIdx.y];
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < r.y; j += gridDim.x * blockDim.x)
@@ -1434,7 +1435,8 @@ struct Batch final : BatchBase {
                 if (npw_ev && single) k_warp_pow_part<T><<<(npw_ev + 7) / 8, kThreads, 0, s>>>(npw_ev, pw_ev, pwe_ev, slot_inst, pactive, b, partT);
                 else if (npw_ev) k_pack_pow_part<T><<<npw_ev, kThreads, 0, s>>>(pw_ev, pwe_ev, slot_inst, pactive, b, partT);
                 k_pow_update<<<distinct, kFinishThreads, 0, s>>>(pw_first, pw_range, partT, est, pscale, pactive, pw_taken);
-                if (npw_ev && single)
+                if (npanels[0]) --launches;  // panels scale the vector as they gather it
+                else if (npw_ev && single)
                     k_flat_pow_scale<T><<<dim3(unsigned(std::max(1, std::min(64, 592 / distinct))), unsigned(distinct)), kThreads, 0, s>>>(pw_first, pw_cols, pactive, pscale, b);
                 else if (npw_ev) k_pack_pow_scale<T><<<npw_ev, kThreads, 0, s>>>(pw_ev, pwe_ev, slot_inst, pactive, pscale, b);
                 launches += 3;
@@ -1467,8 +1469,11 @@ struct Batch final : BatchBase {
     int64_t per_pgraph = 0;
     void power_spmv(int phase, const T* xin, T* y) {
         if (npanels[0]) {
-            BK(launch_panels(panels[phase], npanels[phase], panel_most[phase], xin, (const PanelWork<1>*)panel_first[phase],
-                             (const int*)pactive, PanelStore<T>{y}, s));
+            const auto* work = (const PanelWork<1>*)panel_first[phase];
+            if (phase == 0)
+                BK(launch_panels(panels[0], npanels[0], panel_most[0], xin, work, (const int*)pactive, PanelScaled<T>{{y}, pscale}, s));
+            else
+                BK(launch_panels(panels[1], npanels[1], panel_most[1], xin, work, (const int*)pactive, PanelStore<T>{y}, s));
             ++launches;
             return;
         }
@@ -1493,7 +1498,7 @@ struct Batch final : BatchBase {
         BK(cudaEventCreate(&e1));
         BK(cudaEventRecord(e0, s));
         // power iteration per instance (gpu/pdhg.cu:416-436)
-        k_power_starts<T><<<dim3(unsigned(std::max(1, std::min(64, 592 / distinct))), unsigned(distinct)), 256, 0, s>>>(pw_first, pw_cols, pw_width, pw_norm, pv);
+        k_power_starts<T><<<dim3(unsigned(std::max(1, std::min(64, 592 / distinct))), unsigned(distinct)), 256, 0, s>>>(pw_first, pw_cols, pw_width, pw_norm, pv, pscale);
         // One estimate per distinct matrix: instances that share a matrix share its scaled copy, its row blocks and
         // the deterministic start vector, so their power iterations are the same numbers; only the first instance
         // of each matrix iterates, the others take its estimate.

@@ -757,8 +757,8 @@ struct Engine final : EngineBase {
 
     // ------------------------------------------------------------------ backend concept
     double power_norm(int iters) override {
-        k_power_start<T><<<grid_for(n), 256, 0, st>>>(n, std::sqrt(power_norm2(0.0, 0, n)), pv);
         CK(cudaMemsetAsync(pst, 0, 4 * sizeof(double), st));
+        k_power_start<T><<<grid_for(n), 256, 0, st>>>(n, std::sqrt(power_norm2(0.0, 0, n)), pv, pst);
         CK(cudaMemsetAsync(pdone, 0, sizeof(int), st));
         launches += 1;
         if (cluster_ctas > 0) {
@@ -780,12 +780,17 @@ struct Engine final : EngineBase {
         // the vectors in the same roles and a chunk captured once replays as a CUDA graph
         const int chunk = 8;
         auto step = [&] {
-            spmv(A, a, pw, pdone);
+            if (npanels[0]) {  // these scale the vector as they gather it
+                const PanelWork<1>* whole = nullptr;
+                CK(launch_panels(panels[0], npanels[0], panel_most[0], (const T*)a, whole, nullptr, PanelScaled<T>{{pw}, pst + 2}, st));
+                ++launches;
+            } else {
+                spmv(A, a, pw, pdone);
+            }
             spmv(AT, pw, b, pdone);
-            k_power_sumsq<T><<<red_grid(n), kRedThreads, 0, st>>>(n, b, part, tickets + 2, out + 24, pdone);
-            k_power_update<<<1, 1, 0, st>>>(out + 24, pst, pdone);
-            k_power_scale<T><<<grid_for(n), 256, 0, st>>>(n, b, pst, pdone);
-            launches += 3;
+            k_power_sumsq<T><<<red_grid(n), kRedThreads, 0, st>>>(n, b, part, tickets + 2, out + 24, pst, pdone);
+            if (!npanels[0]) k_power_scale<T><<<grid_for(n), 256, 0, st>>>(n, b, pst, pdone), ++launches;
+            ++launches;
             std::swap(a, b);
         };
         for (int it = 0; it < iters;) {
@@ -802,7 +807,7 @@ struct Engine final : EngineBase {
                     launches = before;
                 }
                 CK(cudaGraphLaunch(pgraph, st));
-                launches += 5 * chunk;  // two SpMVs and three small kernels per step
+                launches += (npanels[0] ? 3 : 4) * chunk;  // two products and one or two small kernels per step
                 it = end;
             } else {
                 for (; it < end; ++it) step();

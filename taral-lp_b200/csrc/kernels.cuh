@@ -596,9 +596,9 @@ __global__ void k_xupd(int n, T* __restrict__ x, const T* __restrict__ ATz, cons
 
 // ------------------------------------------------------------------------------------------ reductions
 // Sum K doubles over the CTA; the last CTA to finish (ticket) adds the per-CTA partials in CTA order.
-// Deterministic for a fixed grid size; no CTA waits on another.
+// Deterministic for a fixed grid size; no CTA waits on another. True in the CTA that finished last.
 template <int K>
-__device__ __forceinline__ void reduce_finish(double (&v)[K], double* part, unsigned* ticket, double* out) {
+__device__ __forceinline__ bool reduce_finish(double (&v)[K], double* part, unsigned* ticket, double* out) {
     __shared__ double sh[K][kRedThreads / 32];
     __shared__ bool last;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -633,6 +633,7 @@ __device__ __forceinline__ void reduce_finish(double (&v)[K], double* part, unsi
         }
         if (threadIdx.x == 0) *ticket = 0;
     }
+    return last;
 }
 
 constexpr int kEvalBatch = 4;  // elements whose loads a KKT-evaluation thread issues before summing them
@@ -732,23 +733,23 @@ __global__ void __launch_bounds__(kRedThreads) k_eval_col(int n, double f, const
 // steps taken} (the step count lives on the device, so that a captured chunk of steps can be replayed);
 // *done is set once the estimate has converged (after step 10, |est - prev| <= 1e-7 est) or when ||v||^2 <= 0,
 // and every later kernel of the queued steps returns at once.
-template <class T>
-__global__ void __launch_bounds__(kRedThreads) k_power_sumsq(int n, const T* __restrict__ v, double* part,
-                                                             unsigned* ticket, double* out, const int* done) {
-    if (*done) return;
-    double a[1] = {0};
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) a[0] += double(v[j]) * double(v[j]);
-    reduce_finish<1>(a, part, ticket, out);
-}
-
-static __global__ void k_power_update(const double* out, double* st, int* done) {  // one thread
-    if (*done) return;
-    const double s = out[0], prev = st[0], it = st[3];
+// The estimate after a step from |v|^2: st = {estimate, the one before, factor of the next vector, steps}.
+static __device__ __forceinline__ void power_update(double s, double* st, int* done) {
+    const double prev = st[0], it = st[3];
     st[3] = it + 1;
     if (s <= 0) { st[0] = 0, *done = 1; return; }
     double est = sqrt(sqrt(s));
     st[0] = est, st[1] = prev, st[2] = 1 / sqrt(s);
     if (it >= 10 && fabs(est - prev) <= 1e-7 * est) *done = 2;
+}
+
+template <class T>
+__global__ void __launch_bounds__(kRedThreads) k_power_sumsq(int n, const T* __restrict__ v, double* part,
+                                                             unsigned* ticket, double* out, double* st, int* done) {
+    if (*done) return;
+    double a[1] = {0};
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) a[0] += double(v[j]) * double(v[j]);
+    if (reduce_finish<1>(a, part, ticket, out) && threadIdx.x == 0) power_update(out[0], st, done);
 }
 
 template <class T>
@@ -814,7 +815,8 @@ inline double power_norm2(double nn, int from, int to) {
     return nn;
 }
 template <class T>
-__global__ void k_power_start(int n, double norm, T* __restrict__ v) {
+__global__ void k_power_start(int n, double norm, T* __restrict__ v, double* st) {  // st zeroed; the factor is one
+    if (blockIdx.x == 0 && threadIdx.x == 0) st[2] = 1;
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) v[j] = T(power_entry(unsigned(j)) / norm);
 }
 

@@ -18,6 +18,7 @@
 #pragma once
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 #include <vector>
 
 #include "host.hpp"
@@ -73,6 +74,18 @@ struct PanelStore {
     __device__ __forceinline__ Ops load(int) const { return {}; }
     __device__ __forceinline__ void apply(int r, double s, double2, const Ops&) const { y[r] = Y(s); }
 };
+// The gathered vector times f, rounded as if it had been scaled in memory: a power step then needs no launch to scale it
+// (refinery LP of 3.4M nonzeros FP64, a step: 2 products and 3 launches 36.5 us, 2 products and 1 launch 33).
+template <class Y>
+struct PanelScaled : PanelStore<Y> {
+    static constexpr bool kScaled = true;
+    const double* f;  // per instance
+    __device__ __forceinline__ double2 scale(int inst) const { return make_double2(f[inst], 0); }
+};
+template <class E, class = void>
+struct ScalesGather : std::false_type {};
+template <class E>
+struct ScalesGather<E, std::void_t<decltype(E::kScaled)>> : std::true_type {};
 template <class T>
 struct PanelRow {  // EpiRow, the division by sigma as in dual_prox
     T *Ax, *z;
@@ -180,6 +193,10 @@ __global__ void __launch_bounds__(kPanelThreads, 2) k_panel(const PanelMat<T> a,
         if (tid == 0) scale[0] = epi.scale(0);
     }
     __syncthreads();
+    auto entry = [&](X v, int w) {
+        if constexpr (ScalesGather<E>::value) return X(double(v) * scale[w].x);
+        else return v;
+    };
     {
         X g[kAtOnce][W];
 #pragma unroll
@@ -191,13 +208,13 @@ __global__ void __launch_bounds__(kPanelThreads, 2) k_panel(const PanelMat<T> a,
         for (int i = 0; i < kAtOnce; ++i)
             if (c0[i] >= 0)
 #pragma unroll
-                for (int w = 0; w < W; ++w) xs[(tid + i * kPanelThreads) * W + w] = g[i][w];
+                for (int w = 0; w < W; ++w) xs[(tid + i * kPanelThreads) * W + w] = entry(g[i][w], w);
     }
 #pragma unroll 4
     for (int i = tid + kAtOnce * kPanelThreads; i < p.cols; i += kPanelThreads) {
         const int c = __ldg(list + i);
 #pragma unroll
-        for (int w = 0; w < W; ++w) xs[i * W + w] = __ldg(xin + gather[w] + c);
+        for (int w = 0; w < W; ++w) xs[i * W + w] = entry(__ldg(xin + gather[w] + c), w);
     }
     if (tid < W) xs[p.cols * W + tid] = X(0);
     __syncthreads();
