@@ -264,10 +264,11 @@ struct Engine final : EngineBase {
         CK(cudaStreamSynchronize(st));  // the plans are released
         finish_init(hc_ptr, hl, hu, hrl_ptr, hru_ptr, hDr, hDc);
     }
-    // Panels (panels.cuh) for A and A^T, both or neither, from 1.5M nonzeros in FP64 and 3M in FP32: a panel's latency is
-    // about 7 us. Refinery LPs, us an iteration with row blocks / panels: 1.1M nonzeros FP64 15.1 / 14.7, FP32 11.7 / 13.6;
-    // 2.3M FP64 31.3 / 19.5, FP32 16.1 / 17.2; 3.4M FP64 42.0 / 27.3, FP32 22.9 / 19.8. Panels of half an SM's share of the nonzeros, 8,192 to 16,384: smaller ones
-    // reread too many columns, larger ones leave SMs idle. TARAL_PANELS=0: none (tests).
+    // Panels (panels.cuh) for A and A^T, both or neither, from 1.5M nonzeros in FP64 and 2M in FP32: a panel's latency is
+    // about 6 us. Refinery LPs, us an iteration with row blocks / panels: 1.1M nonzeros FP64 15.1 / 14.8, FP32 11.0 / 12.7;
+    // 2.3M FP64 31.3 / 17.5, FP32 16.1 / 14.6; 3.4M FP64 42.0 / 26.1, FP32 22.9 / 18.0; a power step of the last 55.8 / 35.4,
+    // 36.2 / 27.2. Panels of half an SM's share of the nonzeros, 8,192 to 16,384: smaller ones reread too many columns,
+    // larger ones leave SMs idle. TARAL_PANELS=0: none (tests).
     PanelMat<T> panels[2];
     int npanels[2] = {0, 0};
     PanelSize panel_most[2];
@@ -275,7 +276,7 @@ struct Engine final : EngineBase {
         const char* e = std::getenv("TARAL_PANELS");
         const bool forced = e && std::atoi(e) > 0;  // whatever the size
         if ((e && !forced) || (flags & TARAL_FLAG_NO_GRAPH) || std::getenv("TARAL_PDL") || forced_row_split() >= 0 ||
-            std::getenv("TARAL_ROWTHREAD") || (a.nnz() < (sizeof(T) == 4 ? 3000000 : 1500000) && !forced))
+            std::getenv("TARAL_ROWTHREAD") || (a.nnz() < (sizeof(T) == 4 ? 2000000 : 1500000) && !forced))
             return;
         const int target = int(std::min<int64_t>(16384, std::max<int64_t>(8192, a.nnz() / (148 * 2) * 21 / 20)));
         pa = build_panels(a.ptr, a.idx, a.rows, at.rows, target, kPanelCols, host_threads());
@@ -788,7 +789,7 @@ struct Engine final : EngineBase {
                 spmv(A, a, pw, pdone);
             }
             spmv(AT, pw, b, pdone);
-            k_power_sumsq<T><<<red_grid(n), kRedThreads, 0, st>>>(n, b, part, tickets + 2, out + 24, pst, pdone);
+            CK(launch_early(k_power_sumsq<T>, red_grid(n), kRedThreads, 0, st, n, b, part, tickets + 2, out + 24, pst, pdone));
             if (!npanels[0]) k_power_scale<T><<<grid_for(n), 256, 0, st>>>(n, b, pst, pdone), ++launches;
             ++launches;
             std::swap(a, b);

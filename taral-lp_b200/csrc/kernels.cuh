@@ -76,6 +76,22 @@ __device__ __forceinline__ void pdl_acquire() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// Chains on panels (launch_early): a kernel lets the next one start at once (launch_next) and waits for the one before
+// (wait_previous) only where it first touches what launches write. The early part reads only lists that no launch writes
+// and that copies change between chains (a copy waits for the whole chain), so the release need not follow the wait.
+// Every CTA waits, also one that then returns: a kernel that has ended means that those before it have.
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... Args>
+cudaError_t launch_early(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(grid)), cfg.blockDim = dim3(unsigned(block)), cfg.dynamicSmemBytes = smem, cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr, cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 // Products rounded on their own (never fused into a following add), as the staged paths round them.
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
@@ -746,6 +762,7 @@ static __device__ __forceinline__ void power_update(double s, double* st, int* d
 template <class T>
 __global__ void __launch_bounds__(kRedThreads) k_power_sumsq(int n, const T* __restrict__ v, double* part,
                                                              unsigned* ticket, double* out, double* st, int* done) {
+    launch_next(), wait_previous();
     if (*done) return;
     double a[1] = {0};
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) a[0] += double(v[j]) * double(v[j]);
