@@ -9,6 +9,9 @@
 // restart rule, primal-weight update -- runs per instance on the device (k_decide, FP64), so a block of
 // eval_freq iterations plus its evaluation, decisions and restarts is one CUDA graph replayed until every
 // instance has stopped; finished instances' blocks return at once.
+// Small instances run a block of iterations on one cluster each (cluster.cuh); instances that share a matrix whose rows
+// share columns run on panels (panels.cuh), several instances to a CTA. The power iterations run on the first instance of
+// every distinct matrix only.
 #include <cuda_runtime.h>
 
 #include <algorithm>

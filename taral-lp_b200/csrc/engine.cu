@@ -6,6 +6,9 @@
 //   data   c, l, u, Dc : T[n]        rl, ru, Dr : T[m]        par : T[2] = {tau, sigma}
 //   state  x, ATz, xlast : T[n]      z, Ax, zlast : T[m]      xs : f64[n]  zs : f64[m]  (running sums)
 //   eval   tmp_n f64[n], tmp_m f64[m] (products of the sums), partials, tickets, 20 result doubles
+// How a block of iterations runs: on one thread-block cluster with the whole LP in shared memory (cluster.cuh), in one
+// cooperative launch with a tile of A and A^T per team (resident.cuh), or a launch per phase, on panels (panels.cuh) where
+// rows share columns and on row blocks elsewhere. All give the same bits; choose_resident and plan_panels have the rules.
 // The running sums of A x and A^T z that the reference keeps (gpu/pdhg.cu:188, :200) are not stored: the
 // average's products are formed once per evaluation as A xs and A^T zs, which saves 16 bytes of state traffic
 // per row and per column every iteration.

@@ -765,7 +765,10 @@ __global__ void __launch_bounds__(kRedThreads) k_power_sumsq(int n, const T* __r
     launch_next(), wait_previous();
     if (*done) return;
     double a[1] = {0};
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) a[0] += double(v[j]) * double(v[j]);
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        const double t = double(__ldcg(v + j));  // past L1: the kernel started before v was complete
+        a[0] += t * t;
+    }
     if (reduce_finish<1>(a, part, ticket, out) && threadIdx.x == 0) power_update(out[0], st, done);
 }
 
