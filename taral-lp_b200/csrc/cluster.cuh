@@ -395,8 +395,7 @@ template <class T, class... P, class... Args>
 cudaError_t launch_cluster(void (*many)(const ClusterLp<T>*, int, P...), void (*one)(const ClusterLp<T>*, int, P...),
                            const ClusterLp<T>* lps, int count, int ctas, size_t smem, cudaStream_t st, Args... args) {
     auto kernel = ctas > 1 ? many : one;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (e == cudaSuccess && ctas > 8) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    const cudaError_t e = allow_launches(reinterpret_cast<const void*>(kernel), kClusterSmem, ctas > 1);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(count * ctas)), cfg.blockDim = dim3(kClusterThreads);

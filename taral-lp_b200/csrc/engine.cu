@@ -729,8 +729,8 @@ struct Engine final : EngineBase {
         return {mat(A), mat(AT), m, n, x, z, Ax, ATz, xs, zs, c, l, u, rl, ru, Dr, Dc, xlast, zlast, par, tmp_m, tmp_n,
                 part, to, nullptr, nullptr, tickets + 3, rerr};
     }
-    // `per_team`, `least`: bytes of shared memory per team and at least. The barrier counters alternate: a launch counts on one, which the
-    // launch before it has zeroed, and zeroes the other.
+    // `per_team`, `least`: bytes of shared memory per team and at least. The barrier counters alternate: a launch counts
+    // on one, which the launch before it has zeroed, and zeroes the other.
     template <class... P, class... Args>
     void launch_resident(void (*kernel)(const ResidentArgs<T>, P...), size_t per_team, size_t least, ResidentArgs<T> ra, Args... args) {
         ra.bar = rbar + rparity * (kBarrierStride / 2), ra.other_bar = rbar + (1 - rparity) * (kBarrierStride / 2);
@@ -738,7 +738,7 @@ struct Engine final : EngineBase {
         const int blocks = std::max(A.rnblk, AT.rnblk);
         const int teams = std::min(kTeams, (blocks + resident_ctas - 1) / resident_ctas);
         const size_t smem = std::max(per_team * size_t(teams), least);
-        CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        CK(allow_launches(reinterpret_cast<const void*>(kernel), std::max(per_team * size_t(kTeams), least)));
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(unsigned(resident_ctas)), cfg.blockDim = dim3(unsigned(kThreads * teams));
         cfg.dynamicSmemBytes = smem, cfg.stream = st;

@@ -14,8 +14,12 @@
 //                stream without holding registers across it.
 // The summation order depends only on the matrix, so results are bit-reproducible run to run.
 #pragma once
+#include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <mutex>
+#include <utility>
+#include <vector>
 
 namespace taral {
 
@@ -91,6 +95,25 @@ cudaError_t launch_early(void (*kernel)(P...), int grid, int block, size_t smem,
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr, cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// Lets `kernel` be launched with up to `most` bytes of dynamic shared memory and, for a cluster kernel, in clusters of more
+// than 8 CTAs, on the current device. These are attributes of the kernel, shared by all contexts and threads of the
+// process: they are set once per kernel and device, to the most that any launch asks for, and never lowered, so that no
+// thread takes away what another is about to launch with.
+inline cudaError_t allow_launches(const void* kernel, size_t most, bool wide_clusters = false) {
+    static std::mutex mu;
+    static std::vector<std::pair<const void*, int>> done;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mu);
+    const auto key = std::make_pair(kernel, dev);
+    if (std::find(done.begin(), done.end(), key) != done.end()) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most));
+    if (e == cudaSuccess && wide_clusters) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) done.push_back(key);
+    return e;
 }
 
 // Products rounded on their own (never fused into a following add), as the staged paths round them.

@@ -496,7 +496,8 @@ template <class T, int W, class E>
 cudaError_t launch_panels(const PanelMat<T>& a, int ctas, const PanelSize& most, const T* xin, const PanelWork<W>* work,
                           const int* active, const E& step, cudaStream_t st) {
     const size_t smem = panel_smem<T, W>(most.cols, most.rows, most.nlong);
-    const cudaError_t e = cudaFuncSetAttribute(k_panel<T, T, W, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    const cudaError_t e = allow_launches(reinterpret_cast<const void*>(&k_panel<T, T, W, E>),
+                                         panel_smem<T, W>(kPanelCols, kPanelRows, kPanelRows));
     if (e != cudaSuccess) return e;
     return launch_early(k_panel<T, T, W, E>, ctas, kPanelThreads, smem, st, a, xin, work, active, step);
 }

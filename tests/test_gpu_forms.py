@@ -1,0 +1,62 @@
+"""The forms in which a context or a batch runs its iterations (clusters, a cooperative grid, panels, a launch per phase)
+beside one another, at the limits of what they accept and where one of them gives up."""
+import threading
+
+import numpy as np
+import pytest
+
+import lpgen
+import pdhg
+
+pytestmark = pytest.mark.gpu
+
+
+def _drive(eng, reps, out, errors):
+    try:
+        norm = eng.power_norm(20)
+        eng.set_steps(0.7 / norm, 0.9 / norm)
+        eng.start()
+        for k in range(reps):
+            eng.iterate(1)  # a launch or two per call: as many chances as possible to meet the other thread's
+            if k % 16 == 15:
+                eng.eval_pair(1.0 / (k + 1))
+        out += [np.array([norm])] + list(eng.eval_pair(1.0 / reps)) + list(eng.download(0, 1.0))
+    except Exception as e:  # noqa: BLE001 -- reported by the test's own thread
+        errors.append(e)
+
+
+@pytest.mark.parametrize("form,small,large", [
+    ("one_cta", lambda: lpgen.general(30, 70, seed=1), lambda: lpgen.general(300, 700, seed=3)),
+    ("cluster", lambda: lpgen.planted(900, 2300, 5, seed=2), lambda: lpgen.planted(2000, 5000, 5, seed=2)),
+    ("grid", lambda: lpgen.general(30, 70, seed=1), lambda: lpgen.planted(60_000, 150_000, 6, seed=2)),
+    ("panels", lambda: lpgen.RefineryBase(1, seed=5).instance(1), lambda: lpgen.RefineryBase(3, seed=5).instance(3)),
+], ids=["one_cta", "cluster", "grid", "panels"])
+def test_contexts_of_two_threads(engine_lib, monkeypatch, form, small, large):
+    """Contexts are independent of each other: two threads, each with its own context of another size, get the bits that
+    they get one after the other."""
+    monkeypatch.setenv("TARAL_TUNE", "0")
+    if form == "grid":
+        monkeypatch.setenv("TARAL_RESIDENT", "1")
+    if form == "panels":
+        monkeypatch.setenv("TARAL_PANELS", "1")
+    lps = [small(), large()]
+    alone = []
+    for lp in lps:
+        eng, out, errors = pdhg.Engine.from_model(lp), [], []
+        _drive(eng, 400, out, errors)
+        eng.close()
+        assert not errors, errors
+        alone.append(out)
+    for _ in range(3):
+        engines = [pdhg.Engine.from_model(lp) for lp in lps]
+        outs, errors = [[], []], []
+        threads = [threading.Thread(target=_drive, args=(e, 400, o, errors)) for e, o in zip(engines, outs)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        for e in engines:
+            e.close()
+        assert not errors, errors
+        for a, b in zip(alone, outs):
+            assert len(a) == len(b) and all(np.array_equal(p, q) for p, q in zip(a, b))
