@@ -470,7 +470,8 @@ __global__ void k_pack_pow_scale(const int4* __restrict__ blk, const int4* __res
     for (int q = threadIdx.x; q < (nrows << lw); q += blockDim.x) v[vbase + q] = T(double(v[vbase + q]) * sc);
 }
 // Both where every pack has one slot: the partial sums by a warp per block (as k_warp_eval), the scaling over the
-// instances' whole vectors (range {first entry, entries} per first instance, blockIdx.y).
+// instances' whole vectors (range {first entry, entries} per first instance, `per` CTAs each; a batch may hold more
+// distinct matrices than a grid's second dimension).
 template <class T>
 __global__ void __launch_bounds__(kThreads) k_warp_pow_part(int blocks, const int4* __restrict__ blk, const int4* __restrict__ ext,
                                                              const int* __restrict__ slot_inst, const int* __restrict__ active,
@@ -492,22 +493,23 @@ __global__ void __launch_bounds__(kThreads) k_warp_pow_part(int blocks, const in
 // The first instances' start vectors (k_power_start for all of them).
 template <class T>
 __global__ void k_power_starts(const int4* __restrict__ first, const int2* __restrict__ range, const int* __restrict__ width,
-                               const double* __restrict__ norm, T* __restrict__ v, double* scale) {
-    const int2 r = range[blockIdx.y];
-    if (blockIdx.x == 0 && threadIdx.x == 0) scale[first[blockIdx.y].z] = 1;
-    const int W = width[blockIdx.y], slot = first[blockIdx.y].y;
-    const double nrm = norm[blockIdx.y];
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < r.y; j += gridDim.x * blockDim.x)
+                               const double* __restrict__ norm, T* __restrict__ v, double* scale, int per) {
+    const int k = blockIdx.x / per, part = blockIdx.x % per;
+    const int2 r = range[k];
+    if (part == 0 && threadIdx.x == 0) scale[first[k].z] = 1;
+    const int W = width[k], slot = first[k].y;
+    const double nrm = norm[k];
+    for (int j = part * blockDim.x + threadIdx.x; j < r.y; j += per * blockDim.x)
         v[size_t(r.x) + size_t(j) * W + slot] = T(power_entry(unsigned(j)) / nrm);
 }
 template <class T>
 __global__ void k_flat_pow_scale(const int4* __restrict__ first, const int2* __restrict__ range, const int* __restrict__ active,
-                                 const double* __restrict__ scale, T* __restrict__ v) {
-    const int inst = first[blockIdx.y].z;
+                                 const double* __restrict__ scale, T* __restrict__ v, int per) {
+    const int k = blockIdx.x / per, part = blockIdx.x % per, inst = first[k].z;
     if (!active[inst]) return;
     const double sc = scale[inst];
-    const int2 r = range[blockIdx.y];
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < r.y; j += gridDim.x * blockDim.x) v[r.x + j] = T(double(v[r.x + j]) * sc);
+    const int2 r = range[k];
+    for (int j = part * blockDim.x + threadIdx.x; j < r.y; j += per * blockDim.x) v[r.x + j] = T(double(v[r.x + j]) * sc);
 }
 
 // Download: out = (avg ? sum * f : point) for every used slot.
@@ -1425,6 +1427,7 @@ struct Batch final : BatchBase {
         launches += 7;
     }
 
+    int matrix_ctas() const { return std::max(1, std::min(64, 592 / distinct)); }  // of the kernels over every first instance
     // Up to 200 power steps on the first instance of every distinct matrix, 8 at a time between looks at the device-side
     // stop flags; with graphs a chunk is captured once for the batch's lifetime (its lists never change).
     void power_iteration() {
@@ -1440,7 +1443,7 @@ struct Batch final : BatchBase {
                 k_pow_update<<<distinct, kFinishThreads, 0, s>>>(pw_first, pw_range, partT, est, pscale, pactive, pw_taken);
                 if (npanels[0]) --launches;  // panels scale the vector as they gather it
                 else if (npw_ev && single)
-                    k_flat_pow_scale<T><<<dim3(unsigned(std::max(1, std::min(64, 592 / distinct))), unsigned(distinct)), kThreads, 0, s>>>(pw_first, pw_cols, pactive, pscale, b);
+                    k_flat_pow_scale<T><<<matrix_ctas() * distinct, kThreads, 0, s>>>(pw_first, pw_cols, pactive, pscale, b, matrix_ctas());
                 else if (npw_ev) k_pack_pow_scale<T><<<npw_ev, kThreads, 0, s>>>(pw_ev, pwe_ev, slot_inst, pactive, pscale, b);
                 launches += 3;
                 std::swap(a, b);
@@ -1501,7 +1504,8 @@ struct Batch final : BatchBase {
         BK(cudaEventCreate(&e1));
         BK(cudaEventRecord(e0, s));
         // power iteration per instance (gpu/pdhg.cu:416-436)
-        k_power_starts<T><<<dim3(unsigned(std::max(1, std::min(64, 592 / distinct))), unsigned(distinct)), 256, 0, s>>>(pw_first, pw_cols, pw_width, pw_norm, pv, pscale);
+        k_power_starts<T><<<matrix_ctas() * distinct, 256, 0, s>>>(pw_first, pw_cols, pw_width, pw_norm, pv, pscale, matrix_ctas());
+        BK(cudaGetLastError());
         // One estimate per distinct matrix: instances that share a matrix share its scaled copy, its row blocks and
         // the deterministic start vector, so their power iterations are the same numbers; only the first instance
         // of each matrix iterates, the others take its estimate.

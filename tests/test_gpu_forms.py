@@ -60,3 +60,25 @@ def test_contexts_of_two_threads(engine_lib, monkeypatch, form, small, large):
         assert not errors, errors
         for a, b in zip(alone, outs):
             assert len(a) == len(b) and all(np.array_equal(p, q) for p, q in zip(a, b))
+
+
+def test_batch_of_more_matrices_than_a_grid_dimension(engine_lib):
+    """65,537 LPs of a matrix each, beyond the 65,535 CTAs of a grid's second dimension: every one gets the answer that it
+    gets in a batch of a few."""
+    count = (1 << 16) + 1
+    ptr, idx = np.array([0, 1, 2], np.int64), np.array([0, 0], np.int32)
+    cost, lo, up, rhs = np.array([1.0, 2.0]), np.zeros(2), np.full(2, 5.0), np.array([3.0])
+
+    def lp(k):  # min x0 + 2 x1, (1 + k / count) x0 + x1 = 3
+        return lpgen.LP(f"two_{k}", 1, 2, ptr, idx, np.array([1.0 + k / count, 1.0]), cost, lo, up, rhs, rhs)
+    picked = [0, 1, 40_000, 65_534, 65_535, 65_536]
+    few = pdhg.Batch([lp(k) for k in picked], tol=1e-8, max_iter=128)
+    r0, x0, y0 = few.solve()
+    few.close()
+    many = pdhg.Batch([lp(k) for k in range(count)], tol=1e-8, max_iter=128)
+    assert many.info()["distinct_matrices"] == count
+    r1, x1, y1 = many.solve()
+    many.close()
+    for i, k in enumerate(picked):
+        assert (r0[i]["status"], r0[i]["iterations"], r0[i]["norm_a"]) == (r1[k]["status"], r1[k]["iterations"], r1[k]["norm_a"])
+        assert np.array_equal(x0[i], x1[k]) and np.array_equal(y0[i], y1[k])
