@@ -488,7 +488,8 @@ struct Engine final : EngineBase {
         pst = zeros<double>(4);
         tickets = zeros<unsigned>(4);
         pdone = zeros<int>(1);
-        rbar = zeros<unsigned>(kBarrierStride + 1), rerr = zeros<int>(1);
+        rbar = zeros<unsigned>(kBarrierStride + 1);
+        rerr = reinterpret_cast<int*>(out + kResidentDone);  // beside the scalars, so that one copy brings both
         hc.assign(hc_ptr, hc_ptr + n), hrl.assign(hrl_ptr, hrl_ptr + m), hru.assign(hru_ptr, hru_ptr + m);
         h_out = static_cast<double*>(pinned_block());
         if (!h_out) throw CudaError{"cudaMallocHost: no pinned host memory for the status reads"};
@@ -654,7 +655,9 @@ struct Engine final : EngineBase {
     // ------------------------------------------------------------------ resident launches (resident.cuh)
     static constexpr int kBarrierStride = 64;  // the two barrier counters and the ticket on lines of their own
     unsigned* rbar = nullptr;
-    int* rerr = nullptr;
+    int* rerr = nullptr;     // a resident launch gave up a wait since the last start
+    bool lost = false;       // seen by the host: there is no point until the next start
+    int barrier_polls = kBarrierPolls;
     int resident_ctas = 0;  // CTAs of a resident launch, 0: the phase kernels
     bool resident_iterates = false;  // iteration blocks too (every tile has a team of its own), not only evaluations
     int cluster_ctas = 0;   // CTAs of the LP's cluster (cluster.cuh), 0: not on one cluster
@@ -670,6 +673,7 @@ struct Engine final : EngineBase {
         CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
         if (const char* e = std::getenv("TARAL_RESIDENT")) mode = std::atoi(e);
         if (mode == 0 || !coop) return;
+        if (const char* e = std::getenv("TARAL_BARRIER_POLLS")) barrier_polls = std::max(0, std::atoi(e));  // tests
         resident_blocks(A, sms), resident_blocks(AT, sms);
         resident_ctas = std::min(sms, std::max(A.rnblk, AT.rnblk));
         cluster_ctas = 0;
@@ -727,7 +731,7 @@ struct Engine final : EngineBase {
             return ResidentMat<T>{d.ptr, d.idx, static_cast<const T*>(d.val), d.rblk, d.rnblk};
         };
         return {mat(A), mat(AT), m, n, x, z, Ax, ATz, xs, zs, c, l, u, rl, ru, Dr, Dc, xlast, zlast, par, tmp_m, tmp_n,
-                part, to, nullptr, nullptr, tickets + 3, rerr};
+                part, to, nullptr, nullptr, tickets + 3, rerr, barrier_polls};
     }
     // `per_team`, `least`: bytes of shared memory per team and at least. The barrier counters alternate: a launch counts
     // on one, which the launch before it has zeroed, and zeroes the other.
@@ -748,15 +752,28 @@ struct Engine final : EngineBase {
         cfg.attrs = attr, cfg.numAttrs = 1;
         CK(cudaLaunchKernelEx(&cfg, kernel, ra, static_cast<P>(args)...));
     }
+    // A wait that gave up leaves a half-done iterate: every call that would use or return it fails until the next start.
+    void check_point() const {
+        if (lost) throw CudaError{"resident kernel: a grid barrier timed out, and there is no point until the next start"};
+    }
+    void check_waits(bool gave_up) {
+        if (!gave_up) return;
+        lost = true;
+        CK(cudaMemsetAsync(rerr, 0, sizeof(int), st));
+        CK(cudaMemsetAsync(rbar, 0, (kBarrierStride + 1) * sizeof(unsigned), st));
+        CK(cudaMemsetAsync(tickets, 0, 4 * sizeof(unsigned), st));
+        check_point();
+    }
     void check_resident() {  // after the synchronisation that waits for a launch writing to h_out
         CK(cudaGetLastError());
         const bool done = h_out[kResidentDone] == 1.0;
         h_out[kResidentDone] = 0;
-        if (done) return;
-        CK(cudaMemsetAsync(rerr, 0, sizeof(int), st));
-        CK(cudaMemsetAsync(rbar, 0, (kBarrierStride + 1) * sizeof(unsigned), st));
-        CK(cudaMemsetAsync(tickets, 0, 4 * sizeof(unsigned), st));
-        throw CudaError{"resident kernel: a grid barrier timed out"};
+        check_waits(!done);
+    }
+    bool rerr_of(const double* scalars) const {  // from a copy of `out` up to rerr
+        int e;
+        std::memcpy(&e, scalars + kResidentDone, sizeof e);
+        return e != 0;
     }
 
     // ------------------------------------------------------------------ backend concept
@@ -831,6 +848,8 @@ struct Engine final : EngineBase {
         CK(cudaGetLastError());
     }
     void start(const double* x0, const double* z0) override {
+        CK(cudaMemsetAsync(rerr, 0, sizeof(int), st));
+        lost = false;
         if (x0) {
             CK(cudaMemcpyAsync(d_in, x0, size_t(n) * sizeof(double), cudaMemcpyHostToDevice, st));
             k_set_point<T><<<grid_for(n), 256, 0, st>>>(n, d_in, x, xlast, xs);
@@ -861,6 +880,7 @@ struct Engine final : EngineBase {
         }
     }
     void iterate(int steps) override {
+        check_point();
         if (steps <= 0) return;
         if (cluster_ctas > 0) {
             CK(launch_cluster(k_cluster_iterate<T, true>, k_cluster_iterate<T, false>, d_lp, 1, cluster_ctas, cluster_smem, st, steps));
@@ -904,13 +924,18 @@ struct Engine final : EngineBase {
         launches += 2;
     }
     void eval(bool avg, double f, double* o10) override {
+        check_point();
         queue_eval(avg, f, out);
-        CK(cudaMemcpyAsync(h_out, out, 10 * sizeof(double), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(h_out, out, (kResidentDone + 1) * sizeof(double), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         CK(cudaGetLastError());
+        const bool gave_up = rerr_of(h_out);
+        h_out[kResidentDone] = 0;
+        check_waits(gave_up);
         std::memcpy(o10, h_out, 10 * sizeof(double));
     }
     void eval_pair(double f, double* cur, double* avg) override {
+        check_point();
         if (resident_ctas > 0) {  // the scalars go straight to the pinned status block
             launch_resident(k_resident_eval<T>,
                             sizeof(RowSmem<double>), 20 * kEvalCtas * sizeof(double), resident_args(h_out), f, red_grid(m), red_grid(n));
@@ -926,7 +951,8 @@ struct Engine final : EngineBase {
         std::memcpy(cur, h_out, 10 * sizeof(double));
         std::memcpy(avg, h_out + 10, 10 * sizeof(double));
     }
-    void restart(bool avg, double f) override {
+    void restart(bool avg, double f) override {  // of a block that gave up: reported by the next call that reads
+        check_point();
         k_restart<T><<<grid_for(n), 256, 0, st>>>(n, avg ? 1 : 0, f, x, xs, xlast);
         k_restart<T><<<grid_for(m), 256, 0, st>>>(m, avg ? 1 : 0, f, z, zs, zlast);
         launches += 2;
@@ -934,11 +960,11 @@ struct Engine final : EngineBase {
         CK(cudaGetLastError());
     }
     void download(bool avg, double f, double* hx, double* hz) override {
+        check_point();
         if (resident_ctas > 0) {  // a block whose barrier gave up leaves no point to return
             CK(cudaMemcpyAsync(h_flag, rerr, sizeof(int), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
-            h_out[kResidentDone] = *h_flag ? 0 : 1;
-            check_resident();
+            check_waits(*h_flag != 0);
         }
         if (n) {
             if (avg) k_scale_out<double><<<grid_for(n), 256, 0, st>>>(n, f, xs, hbuf);

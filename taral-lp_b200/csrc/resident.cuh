@@ -24,7 +24,7 @@ namespace taral {
 // Teams per CTA: 2 teams of 256 threads leave 128 registers a thread, which hold a tile in flight beside the step's
 // FP64 operands and the interleaved sums of long rows; 3 or 4 teams spill them to local memory.
 constexpr int kTeams = 2;
-constexpr int kBarrierPolls = 1 << 22;  // bound of a barrier wait (seconds); the launch is cooperative, so it ends at once
+constexpr int kBarrierPolls = 1 << 22;  // bound of a barrier wait (seconds); the launch is cooperative, so it ends sooner
 
 template <class T>
 struct ResidentMat {
@@ -44,7 +44,8 @@ struct ResidentArgs {
     const double* par;
     double *tmp_m, *tmp_n, *part, *out;
     unsigned *bar, *other_bar, *ticket;  // grid barrier's counter (zero at launch) and the next launch's, zeroed here
-    int* err;
+    int* err;   // set when a wait gave up: the launch left its work half done
+    int polls;  // after which a wait gives up
 };
 
 // ------------------------------------------------------------------------------------------ barriers
@@ -52,11 +53,13 @@ struct ResidentArgs {
 struct GridBarrier {
     unsigned *bar, target = 0;
     int* err;
+    int polls;
     bool* ok;  // shared
-    __device__ GridBarrier(unsigned* b, unsigned* other, int* e, bool* shared_ok) : bar(b), err(e), ok(shared_ok) {
+    template <class T>
+    __device__ GridBarrier(const ResidentArgs<T>& a, bool* shared_ok) : bar(a.bar), err(a.err), polls(a.polls), ok(shared_ok) {
         if (threadIdx.x == 0) {
             *ok = true;
-            if (blockIdx.x == 0) *other = 0;
+            if (blockIdx.x == 0) *a.other_bar = 0;
         }
     }
     __device__ __forceinline__ void arrive() {
@@ -67,12 +70,13 @@ struct GridBarrier {
     }
     __device__ __forceinline__ bool wait() {
         if (threadIdx.x == 0) {
-            unsigned v;
-            int i = 0;
-            do {
+            bool there = false;
+            for (int i = 0; i < polls && !there; ++i) {
+                unsigned v;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-            } while (int(v - target) < 0 && ++i < kBarrierPolls);
-            if (int(v - target) < 0) *ok = false, atomicExch(err, 1);
+                there = int(v - target) >= 0;
+            }
+            if (!there) *ok = false, atomicExch(err, 1);
         }
         __syncthreads();
         return *ok;
@@ -289,7 +293,7 @@ __global__ void __launch_bounds__(kThreads * kTeams, 1) k_resident_iterate(const
     __shared__ int held[2][kTeams][kRowsMax + 1];
     const Team t;
     RowSmem<T>& sm = reinterpret_cast<RowSmem<T>*>(raw)[t.id];
-    GridBarrier barrier(a.bar, a.other_bar, a.err, &ok);
+    GridBarrier barrier(a, &ok);
     const int first = t.id * int(gridDim.x) + int(blockIdx.x), teams = int(gridDim.x) * (int(blockDim.x) / kThreads);
     const FirstTile fa = first_tile(a.A, t, first, held[0][t.id]), ft = first_tile(a.AT, t, first, held[1][t.id]);
     const double tau = a.par[0], sigma = a.par[1];
@@ -346,7 +350,7 @@ __global__ void __launch_bounds__(kThreads * kTeams, 1) k_resident_eval(const Re
     __shared__ double sh[kTeams][5 * (kThreads / 32)];
     const Team t;
     RowSmem<double>& sm = reinterpret_cast<RowSmem<double>*>(raw)[t.id];
-    GridBarrier barrier(a.bar, a.other_bar, a.err, &ok);
+    GridBarrier barrier(a, &ok);
     const int first = t.id * int(gridDim.x) + int(blockIdx.x), teams = int(gridDim.x) * (int(blockDim.x) / kThreads);
     auto products = [&](const ResidentMat<T>& mat, const double* in, double* to) {
         for (int b = first; b < mat.nblk; b += teams) {
@@ -414,7 +418,7 @@ __global__ void __launch_bounds__(kThreads * kTeams, 1) k_resident_power(const R
     __shared__ double sh[kTeams][kThreads / 32], parts[kEvalCtas], total;
     const Team t;
     RowSmem<T>& sm = reinterpret_cast<RowSmem<T>*>(raw)[t.id];
-    GridBarrier barrier(a.bar, a.other_bar, a.err, &ok);
+    GridBarrier barrier(a, &ok);
     const int first = t.id * int(gridDim.x) + int(blockIdx.x), teams = int(gridDim.x) * (int(blockDim.x) / kThreads);
     const FirstTile fa = first_tile(a.A, t, first, held[0][t.id]), ft = first_tile(a.AT, t, first, held[1][t.id]);
     double est = 0, f = 0;

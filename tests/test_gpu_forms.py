@@ -82,3 +82,41 @@ def test_batch_of_more_matrices_than_a_grid_dimension(engine_lib):
     for i, k in enumerate(picked):
         assert (r0[i]["status"], r0[i]["iterations"], r0[i]["norm_a"]) == (r1[k]["status"], r1[k]["iterations"], r1[k]["norm_a"])
         assert np.array_equal(x0[i], x1[k]) and np.array_equal(y0[i], y1[k])
+
+
+@pytest.mark.parametrize("call", ["eval_current", "eval_average", "eval_pair", "download", "restart_then_eval", "power_norm"])
+def test_barrier_that_gives_up_is_reported(engine_lib, monkeypatch, call):
+    """A block of iterations whose grid barrier gives up its wait (here: at once) leaves a half-done iterate. The first
+    call that would return numbers of it fails, so do the others, and a new start makes the context usable again."""
+    lp = lpgen.planted(4000, 10_000, 5, seed=2)  # several CTAs
+    monkeypatch.setenv("TARAL_RESIDENT", "1")
+    good = pdhg.Engine.from_model(lp)
+    good.set_steps(0.1, 0.1)
+    good.start()
+    expected, point = good.eval(0, 1.0), good.download(0, 1.0)
+    good.close()
+    monkeypatch.setenv("TARAL_BARRIER_POLLS", "0")
+    eng = pdhg.Engine.from_model(lp)
+    eng.set_steps(0.1, 0.1)
+    calls = {"eval_current": lambda: eng.eval(0, 1.0), "eval_average": lambda: eng.eval(1, 1.0 / 8),
+             "eval_pair": lambda: eng.eval_pair(1.0 / 8), "download": lambda: eng.download(0, 1.0),
+             "restart_then_eval": lambda: (eng.restart(False, 1.0), eng.eval(0, 1.0)),
+             "power_norm": lambda: eng.power_norm(20)}
+    for _ in range(2):
+        eng.start()
+        assert np.array_equal(eng.eval(0, 1.0), expected)
+        assert all(np.array_equal(a, b) for a, b in zip(eng.download(0, 1.0), point))
+        eng.iterate(8)
+        with pytest.raises(pdhg.TaralError) as e:
+            calls[call]()
+        assert "timed out" in str(e.value)
+        for other in calls.values():
+            with pytest.raises(pdhg.TaralError):
+                other()
+        with pytest.raises(pdhg.TaralError):
+            eng.iterate(8)
+    with pytest.raises(pdhg.TaralError):
+        eng.solve(eng.bnorm, eng.cnorm, tol=1e-4, max_iter=64)
+    eng.start()
+    assert np.array_equal(eng.eval(0, 1.0), expected)
+    eng.close()
