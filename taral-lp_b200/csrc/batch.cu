@@ -43,6 +43,7 @@ namespace {
 struct BatchError {
     std::string msg;
 };
+struct BatchNoMemory : BatchError {};  // of the device
 #define BK(call)                                                                                            \
     do {                                                                                                    \
         cudaError_t e_ = (call);                                                                            \
@@ -661,14 +662,28 @@ struct Batch final : BatchBase {
         void* p = nullptr;
         const size_t bytes = std::max<size_t>(n, 1) * sizeof(U);
         if (!alloc_allowed(alloc_bytes, bytes))
-            throw BatchError{"cudaMalloc: the device allocation limit (taral_set_device_alloc_limit) is reached"};
+            throw BatchNoMemory{{"cudaMalloc: the device allocation limit (taral_set_device_alloc_limit) is reached"}};
         cudaError_t e = cudaMallocAsync(&p, bytes, s);
-        if (e != cudaSuccess) throw BatchError{std::string("cudaMalloc: ") + cudaGetErrorString(e)};
+        if (e != cudaSuccess) throw BatchNoMemory{{std::string("cudaMalloc: ") + cudaGetErrorString(e)}};
         allocs.push_back(p);
         alloc_bytes += bytes;
         return static_cast<U*>(p);
     }
     size_t alloc_bytes = 0;
+    // make() allocates what the batch can do without: false, with its allocations given back, where memory is short.
+    template <class F>
+    bool if_memory(F make) {
+        const size_t kept = allocs.size(), bytes = alloc_bytes;
+        try {
+            make();
+            return true;
+        } catch (const BatchNoMemory&) {
+            cudaGetLastError();
+            for (; allocs.size() > kept; allocs.pop_back()) cudaFreeAsync(allocs.back(), s);
+            alloc_bytes = bytes;
+            return false;
+        }
+    }
     template <class U>
     U* put(const std::vector<U>& h) {
         U* p = alloc<U>(h.size());
@@ -827,7 +842,6 @@ struct Batch final : BatchBase {
                 k_narrow<T><<<g, 256, 0, s>>>(nzb, va, Aval);
                 k_narrow<T><<<g, 256, 0, s>>>(nzb, vt, Tval);
             }
-            put_panels();
             std::vector<double> hdr(static_cast<size_t>(drn)), hdc(static_cast<size_t>(dcn));
             if (drn) BK(cudaMemcpyAsync(hdr.data(), dr, size_t(drn) * sizeof(double), cudaMemcpyDeviceToHost, s));
             if (dcn) BK(cudaMemcpyAsync(hdc.data(), dc, size_t(dcn) * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -950,7 +964,6 @@ struct Batch final : BatchBase {
         h_ae1 = ae1_it, h_ae = ae_it, h_te1 = te1_it, h_te = te_it;
         slot_inst = put(hslot), d_where = put(where);
         power_lists(t_ev, te_ev, hcr);
-        panel_lists(std::vector<int>(size_t(count), 1));
         // 5. upload
         A_it = put(a_it), Ae_it = put(ae_it), T_it = put(t_it), Te_it = put(te_it);
         A_ev = put(a_ev), Ae_ev = put(ae_ev), T_ev = put(t_ev), Te_ev = put(te_ev);
@@ -985,6 +998,11 @@ struct Batch final : BatchBase {
         BK(cudaHostGetDevicePointer(&dc, h_cancel, 0));
         d_cancel = static_cast<const int*>(dc);
         BK(cudaStreamSynchronize(s));
+        // after all that the batch cannot do without; the row blocks stay and give the same numbers
+        if (!if_memory([&] { put_panels(), panel_lists(std::vector<int>(size_t(count), 1)); }))
+            for (int k = 0; k < 2; ++k) npanels[k] = 0, panel_work[k] = nullptr, h_panels[k].clear(), first_panel[k].clear();
+        for (auto& sh : mats)
+            for (PanelPlan& p : sh->panels) p = PanelPlan();
         mem_used = alloc_bytes;
         nnz_total = 0;
         for (int i = 0; i < count; ++i) nnz_total += mats[mat_of[i]]->nnz;
@@ -1032,7 +1050,6 @@ struct Batch final : BatchBase {
                 PanelPlan& p = sh.panels[k];
                 first_panel[k].push_back(int(all.panels.size()));
                 all.append(p, k ? sh.pbaseT : sh.pbaseA);
-                p = PanelPlan();
             }
             first_panel[k].push_back(int(all.panels.size()));
             Four<T>* val = alloc<Four<T>>(size_t(all.groups) * 32);
@@ -1045,6 +1062,7 @@ struct Batch final : BatchBase {
                                                             panels[k].longrow, k ? Tptr : Aptr, k ? Tidx : Aidx, k ? Tval : Aval, val,
                                                             place, lval, lplace);
             BK(cudaGetLastError());
+            BK(cudaStreamSynchronize(s));
         }
     }
     // The CTAs of the instances with live[i], matrix by matrix: a panel, then the groups of instances that use it.
@@ -1163,7 +1181,11 @@ struct Batch final : BatchBase {
             }
             if (need > kClusterSmem) continue;
             std::vector<int*> d_plan;
-            for (const auto& p : plans) d_plan.push_back(put(p));
+            if (!if_memory([&] {
+                    for (const auto& p : plans) d_plan.push_back(put(p));
+                    d_lps = alloc<ClusterLp<T>>(size_t(ninst)), d_first_lps = alloc<ClusterLp<T>>(mats.size()), d_norms = alloc<double>(2 * mats.size());
+                }))
+                return;
             std::vector<ClusterLp<T>> lps, firsts;
             for (int i = 0; i < ninst; ++i) {
                 const Shared& sh = *mats[size_t(mat_of[size_t(i)])];
@@ -1176,7 +1198,9 @@ struct Batch final : BatchBase {
                 lp.active = nullptr;
                 if (first_inst[size_t(mat_of[size_t(i)])] == i) firsts.push_back(lp);  // in the order of the matrices
             }
-            d_lps = put(lps), d_first_lps = put(firsts), d_norms = alloc<double>(2 * mats.size());
+            BK(cudaMemcpyAsync(d_lps, lps.data(), lps.size() * sizeof(lps[0]), cudaMemcpyHostToDevice, s));
+            BK(cudaMemcpyAsync(d_first_lps, firsts.data(), firsts.size() * sizeof(firsts[0]), cudaMemcpyHostToDevice, s));
+            BK(cudaStreamSynchronize(s));
             cluster_ctas = q, cluster_smem = need;
             mem_used = alloc_bytes;
             return;

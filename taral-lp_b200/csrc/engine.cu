@@ -161,6 +161,7 @@ static int red_grid(int64_t k) {  // reductions: fixed grid per size, so the par
 struct CudaError {
     std::string msg;
 };
+struct NoMemory : CudaError {};  // of the device
 #define CK(call)                                                                                           \
     do {                                                                                                   \
         cudaError_t e_ = (call);                                                                           \
@@ -207,14 +208,28 @@ struct Engine final : EngineBase {
         void* p = nullptr;
         const size_t bytes = std::max<size_t>(count, 1) * sizeof(U);
         if (!alloc_allowed(alloc_bytes, bytes))
-            throw CudaError{"cudaMalloc: the device allocation limit (taral_set_device_alloc_limit) is reached"};
+            throw NoMemory{{"cudaMalloc: the device allocation limit (taral_set_device_alloc_limit) is reached"}};
         cudaError_t e = cudaMallocAsync(&p, bytes, st);
-        if (e != cudaSuccess) throw CudaError{std::string("cudaMalloc: ") + cudaGetErrorString(e)};
+        if (e != cudaSuccess) throw NoMemory{{std::string("cudaMalloc: ") + cudaGetErrorString(e)}};
         allocs.push_back(p);
         alloc_bytes += bytes;
         return static_cast<U*>(p);
     }
     size_t alloc_bytes = 0;
+    // make() allocates what the context can do without: false, with its allocations given back, where memory is short.
+    template <class F>
+    bool if_memory(F make) {
+        const size_t kept = allocs.size(), bytes = alloc_bytes;
+        try {
+            make();
+            return true;
+        } catch (const NoMemory&) {
+            cudaGetLastError();
+            for (; allocs.size() > kept; allocs.pop_back()) cudaFreeAsync(allocs.back(), st);
+            alloc_bytes = bytes;
+            return false;
+        }
+    }
     T* upload(const double* v, size_t k) {
         std::vector<T> h(v, v + k);
         T* p = alloc<T>(k);
@@ -263,9 +278,7 @@ struct Engine final : EngineBase {
         nnz = hA.nnz;
         PanelPlan panels_a, panels_t;
         plan_panels({hA.rows, hA.ptr, hA.idx, hA.val}, {hAT.rows, hAT.ptr, hAT.idx, hAT.val}, flags, panels_a, panels_t);
-        put_panels(0, A, panels_a), put_panels(1, AT, panels_t);
-        CK(cudaStreamSynchronize(st));  // the plans are released
-        finish_init(hc_ptr, hl, hu, hrl_ptr, hru_ptr, hDr, hDc);
+        finish_init(hc_ptr, hl, hu, hrl_ptr, hru_ptr, hDr, hDc, panels_a, panels_t);
     }
     // Panels (panels.cuh) for A and A^T, both or neither, from 1.5M nonzeros in FP64 and 2M in FP32: a panel's latency is
     // about 6 us. Refinery LPs, us an iteration with row blocks / panels: 1.1M nonzeros FP64 15.1 / 14.8, FP32 11.0 / 12.7;
@@ -448,7 +461,6 @@ struct Engine final : EngineBase {
             k_narrow<T><<<g, 256, 0, st>>>(nz, va, static_cast<T*>(A.val));
             k_narrow<T><<<g, 256, 0, st>>>(nz, vt, static_cast<T*>(AT.val));
         }
-        put_panels(0, A, panels_a), put_panels(1, AT, panels_t);
         if (m) CK(cudaMemcpyAsync(P.Dr.data(), dr, size_t(m) * sizeof(double), cudaMemcpyDeviceToHost, st));
         if (n) CK(cudaMemcpyAsync(P.Dc.data(), dc, size_t(n) * sizeof(double), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
@@ -465,15 +477,16 @@ struct Engine final : EngineBase {
         if (host_s) *host_s = hs;
         if (reorder) {
             const std::vector<double> rl_i = to_internal(P.rl), ru_i = to_internal(P.ru), dr_i = to_internal(P.Dr);
-            finish_init(P.c.data(), P.l.data(), P.u.data(), rl_i.data(), ru_i.data(), dr_i.data(), P.Dc.data());
+            finish_init(P.c.data(), P.l.data(), P.u.data(), rl_i.data(), ru_i.data(), dr_i.data(), P.Dc.data(), panels_a, panels_t);
             hrl = P.rl, hru = P.ru;  // the driver's host copies stay in the model's order
         } else {
-            finish_init(P.c.data(), P.l.data(), P.u.data(), P.rl.data(), P.ru.data(), P.Dr.data(), P.Dc.data());
+            finish_init(P.c.data(), P.l.data(), P.u.data(), P.rl.data(), P.ru.data(), P.Dr.data(), P.Dc.data(), panels_a, panels_t);
         }
         nnz = nz;
     }
     void finish_init(const double* hc_ptr, const double* hl, const double* hu, const double* hrl_ptr,
-                     const double* hru_ptr, const double* hDr, const double* hDc) {
+                     const double* hru_ptr, const double* hDr, const double* hDc, const PanelPlan& panels_a,
+                     const PanelPlan& panels_t) {
         c = upload(hc_ptr, n), l = upload(hl, n), u = upload(hu, n), Dc = upload(hDc, n);
         rl = upload(hrl_ptr, m), ru = upload(hru_ptr, m), Dr = upload(hDr, m);
         par = zeros<double>(2);
@@ -496,6 +509,9 @@ struct Engine final : EngineBase {
         h_flag = reinterpret_cast<int*>(h_out + 32);
         h_out[kResidentDone] = 0;
         CK(cudaStreamSynchronize(st));
+        // after all that the context cannot do without; the row blocks stay and give the same numbers
+        if (!if_memory([&] { put_panels(0, A, panels_a), put_panels(1, AT, panels_t); })) npanels[0] = npanels[1] = 0;
+        CK(cudaStreamSynchronize(st));  // the plans are released
         mem_used = alloc_bytes;
         tune();
         choose_resident();
@@ -690,12 +706,12 @@ struct Engine final : EngineBase {
             std::vector<int> plan;
             const size_t need = cluster_plan<T>(A.hptr.data(), AT.hptr.data(), m, n, q, plan);
             if (need > kClusterSmem) continue;
+            int* d_plan = nullptr;
+            if (!if_memory([&] { d_plan = alloc<int>(plan.size()), d_lp = alloc<ClusterLp<T>>(1); })) return;
             cluster_ctas = q, cluster_smem = need;
-            int* d_plan = alloc<int>(plan.size());
             CK(cudaMemcpyAsync(d_plan, plan.data(), plan.size() * sizeof(int), cudaMemcpyHostToDevice, st));
             const ClusterLp<T> lp{A.ptr, A.idx, AT.ptr, AT.idx, static_cast<const T*>(A.val), static_cast<const T*>(AT.val),
                                   m, n, x, z, Ax, ATz, xs, zs, c, l, u, rl, ru, par, pv, d_plan, nullptr};
-            d_lp = alloc<ClusterLp<T>>(1);
             CK(cudaMemcpyAsync(d_lp, &lp, sizeof lp, cudaMemcpyHostToDevice, st));
             CK(cudaStreamSynchronize(st));
             mem_used = alloc_bytes;
@@ -721,7 +737,7 @@ struct Engine final : EngineBase {
             }
             if (tile == kTile && rows == kRowsMax) return;
         }
-        d.rblk = alloc<int4>(list.size()), d.rnblk = int(list.size());
+        if (!if_memory([&] { d.rblk = alloc<int4>(list.size()), d.rnblk = int(list.size()); })) return;
         CK(cudaMemcpyAsync(d.rblk, list.data(), list.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
         CK(cudaStreamSynchronize(st));
         mem_used = alloc_bytes;

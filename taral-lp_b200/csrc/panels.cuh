@@ -18,6 +18,7 @@
 #pragma once
 #include <algorithm>
 #include <cstdint>
+#include <new>
 #include <type_traits>
 #include <vector>
 
@@ -451,7 +452,7 @@ PanelPlan panels_of(const I* ptr, const int32_t* idx, int first, int last, int c
 // lists must hold at most a third as many columns as the panels hold nonzeros (a list and its entries of x cost about as
 // much to read as they save otherwise), and padding at most 40 % of the nonzeros.
 template <class I>
-PanelPlan build_panels(const I* ptr, const int32_t* idx, int rows, int cols, int target, int max_cols, int threads) {
+PanelPlan plan_of_panels(const I* ptr, const int32_t* idx, int rows, int cols, int target, int max_cols, int threads) {
     PanelPlan plan;
     if (rows == 0 || ptr[rows] == ptr[0]) return plan;
     for (int r = 0; r < rows; ++r)
@@ -478,13 +479,26 @@ PanelPlan build_panels(const I* ptr, const int32_t* idx, int rows, int cols, int
             auto cut = [&](int64_t k) {
                 return k >= threads ? rows : int(std::lower_bound(ptr, ptr + rows, ptr[0] + I(all * k / threads)) - ptr);
             };
-            part[size_t(q)] = panels_of(ptr, idx, cut(q), cut(q + 1), cols, target, max_cols);
+            try {
+                part[size_t(q)] = panels_of(ptr, idx, cut(q), cut(q + 1), cols, target, max_cols);
+            } catch (const std::bad_alloc&) {  // no exception leaves a thread: its rows are not covered, and there are no panels
+                part[size_t(q)] = PanelPlan();
+            }
         }
     });
     for (const PanelPlan& p : part) plan.append(p, 0);
     int covered = 0;
     for (const Panel& p : plan.panels) covered += p.rows;
     return covered == rows && pays(plan, all) ? plan : PanelPlan();
+}
+// The same; none either where the host has no memory for the plan.
+template <class I>
+PanelPlan build_panels(const I* ptr, const int32_t* idx, int rows, int cols, int target, int max_cols, int threads) {
+    try {
+        return plan_of_panels(ptr, idx, rows, cols, target, max_cols, threads);
+    } catch (const std::bad_alloc&) {
+        return PanelPlan();
+    }
 }
 
 // The panel counterparts of the row blocks' fused steps.

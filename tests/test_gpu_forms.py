@@ -1,5 +1,6 @@
 """The forms in which a context or a batch runs its iterations (clusters, a cooperative grid, panels, a launch per phase)
 beside one another, at the limits of what they accept and where one of them gives up."""
+import dataclasses
 import threading
 
 import numpy as np
@@ -120,3 +121,59 @@ def test_barrier_that_gives_up_is_reported(engine_lib, monkeypatch, call):
     eng.start()
     assert np.array_equal(eng.eval(0, 1.0), expected)
     eng.close()
+
+
+def _engine_numbers(lp, precision):
+    eng = pdhg.Engine.from_model(lp, precision=precision)
+    norm = eng.power_norm(30)
+    eng.set_steps(0.7 / norm, 0.9 / norm)
+    eng.start()
+    eng.iterate(64)
+    out = [np.array([norm])] + list(eng.eval_pair(1 / 64)) + list(eng.download(0, 1.0))
+    mem = eng.info()[1]
+    eng.close()
+    return mem, out
+
+
+def _batch_numbers(lps, precision):
+    b = pdhg.Batch(lps, tol=1e-12, max_iter=128, precision=precision)
+    res, xs, ys = b.solve()
+    mem = b.info()["device_mem_bytes"]
+    b.close()
+    return mem, [np.array([r["norm_a"], r["rel_primal"], r["rel_dual"]]) for r in res] + xs + ys
+
+
+@pytest.mark.parametrize("precision", [pdhg.FP64, pdhg.FP32], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("form", ["panels", "batch_panels", "cluster", "batch_cluster"])
+def test_forms_give_way_where_memory_is_short(engine_lib, monkeypatch, form, precision):
+    """What panels and clusters hold on the device is extra: a context or a batch for whose plain form the memory suffices
+    is created all the same, and gives the same numbers."""
+    monkeypatch.setenv("TARAL_TUNE", "0")
+    monkeypatch.setenv("TARAL_ROWORDER", "0")
+    base = lpgen.RefineryBase(2, seed=5)
+    pert = lpgen.perturbations(6, seed=8)
+    small = lpgen.general(200, 450, seed=5)
+    if form.startswith("batch"):
+        lps = [base.instance(2, p) for p in pert] if form == "batch_panels" else [
+            dataclasses.replace(small, cost=small.cost * (1 + k / 10)) for k in range(4)]
+        numbers = lambda: _batch_numbers(lps, precision)  # noqa: E731
+    else:
+        lp = base.instance(2, pert[0]) if form == "panels" else small
+        numbers = lambda: _engine_numbers(lp, precision)  # noqa: E731
+    switch, off, on = ("TARAL_PANELS", "0", "1") if "panels" in form else ("TARAL_RESIDENT", "0", "2")
+    monkeypatch.setenv(switch, off)
+    plain, expected = numbers()
+    monkeypatch.setenv(switch, on)
+    full, got = numbers()
+    assert full > plain  # the form is there
+    for a, b in zip(expected, got):
+        assert np.array_equal(a, b)
+    try:
+        for limit in (plain, plain + (full - plain) // 3, plain + 2 * (full - plain) // 3, full - 1, full):
+            pdhg.set_device_alloc_limit(limit)
+            mem, got = numbers()
+            assert mem <= limit and (mem == full) == (limit == full)
+            for a, b in zip(expected, got):
+                assert np.array_equal(a, b)
+    finally:
+        pdhg.set_device_alloc_limit(0)
