@@ -774,10 +774,7 @@ struct Batch final : BatchBase {
                 });
             for (auto& t : th) t.join();
         };
-        // panels (panels.cuh) for every matrix, both ways, or for none
-        nnz_total = 0;
-        for (int i = 0; i < count; ++i) nnz_total += md[i].col_ptr[md[i].n];
-        const bool panels_ok = panels_allowed();
+        std::atomic<bool> panels_ok{panels_allowed(md)};  // panels (panels.cuh) for every matrix, both ways, or for none
         par_for(distinct, [&](int k) {
             Shared& sh = *mats[k];
             const taral_model& mk = md[first_inst[k]];
@@ -785,6 +782,7 @@ struct Batch final : BatchBase {
             if (panels_ok) {
                 sh.panels[0] = build_panels(sh.S.A.ptr.data(), sh.S.A.idx.data(), mk.m, mk.n, kPanelTarget, kBatchPanelCols, 1);
                 if (!sh.panels[0].empty()) sh.panels[1] = build_panels(sh.S.AT.ptr.data(), sh.S.AT.idx.data(), mk.n, mk.m, kPanelTarget, kBatchPanelCols, 1);
+                if (sh.panels[1].empty()) panels_ok = false;
             }
             sh.S.m = mk.m, sh.S.n = mk.n, sh.nnz = int64_t(sh.S.A.idx.size());
         });
@@ -1022,7 +1020,13 @@ struct Batch final : BatchBase {
     // ------------------------------------------------------------------ panels
     // Every phase of a batch on panels of the distinct matrices, kPW instances that share a matrix to a CTA. On 48
     // refinery scenarios of 12 matrices (22.6M products a phase, FP32) a row phase takes 42 us (row blocks 72), a column
-    // phase 33 (55). From a million nonzeros over the instances, where panels fill the SMs. TARAL_PANELS=0: none.
+    // phase 33 (55). TARAL_PANELS=0: none, 1: at any size (tests).
+    //
+    // Only where the CTAs whose slots are all used fill the SMs (FP64: two thirds of them), and rows of at least 8 (see
+    // panels_suit). Measured, us an iteration with row blocks / panels by those CTAs: refinery scenarios FP32 69: 45.5 /
+    // 57.3, 92: 56.3 / 59.9, 104: 63.6 / 61.9, 112: 72.1 / 78.9, 168: 101 / 88, 184: 103 / 69, 207: 115 / 73; FP64 69: 44.3 /
+    // 49.3, 92: 48.9 / 49.7, 104: 59 / 50, 112: 70 / 69, 138: 71 / 53; bands of 8 FP32 78: 23 / 30, 156: 36.6 / 35.0; bands of 6
+    // FP32 320: 50.7 / 61.4, FP64 640: 66.5 / 78.0.
     static constexpr int kPW = sizeof(T) == 4 ? 4 : 2;
     static constexpr int kPanelTarget = 24576, kBatchPanelCols = 4096;
     PanelMat<T> panels[2];
@@ -1033,12 +1037,25 @@ struct Batch final : BatchBase {
     PanelWork<kPW>* panel_work[2] = {nullptr, nullptr};    // the running instances' CTAs
     PanelWork<1>* panel_first[2] = {nullptr, nullptr};     // the power iteration's
     int npanel_work[2] = {0, 0};
-    bool panels_allowed() const {
+    bool panels_allowed(const taral_model* md) const {
         const char* e = std::getenv("TARAL_PANELS");
         const char* pack = std::getenv("TARAL_BATCH_PACK");
         if ((e && std::atoi(e) == 0) || (pack && std::atoi(pack) > 1) || pdl || std::getenv("TARAL_ROWSPLIT") || std::getenv("TARAL_ROWTHREAD"))
             return false;
-        return nnz_total >= (int64_t(1) << 20) || (e && std::atoi(e) > 0);
+        if (e && std::atoi(e) > 0) return true;
+        int dev, sms;
+        BK(cudaGetDevice(&dev));
+        BK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        double ctas[2] = {0, 0}, rows[2] = {0, 0}, nnz = 0;
+        for (int i = 0; i < ninst; ++i) {
+            const double size[2] = {double(md[i].m), double(md[i].n)}, entries = double(md[i].col_ptr[md[i].n]);
+            for (int k = 0; k < 2; ++k) {
+                ctas[k] += std::max(size[k] / kPanelRows, entries / kPanelTarget) / kPW;
+                rows[k] += size[k];
+            }
+            nnz += entries;
+        }
+        return std::min(ctas[0], ctas[1]) >= (sizeof(T) == 4 ? 1.0 : 2.0 / 3) * sms && nnz >= 8 * std::max(rows[0], rows[1]);
     }
     void put_panels() {  // the plans of all matrices one after another, filled from the scaled values
         for (const auto& sh : mats)

@@ -284,7 +284,7 @@ struct Engine final : EngineBase {
     // about 6 us. Refinery LPs, us an iteration with row blocks / panels: 1.1M nonzeros FP64 15.1 / 14.8, FP32 11.0 / 12.7;
     // 2.3M FP64 31.3 / 17.5, FP32 16.1 / 14.6; 3.4M FP64 42.0 / 26.1, FP32 22.9 / 18.0; a power step of the last 55.8 / 35.4,
     // 36.2 / 27.2. Panels of half an SM's share of the nonzeros, 8,192 to 16,384: smaller ones reread too many columns,
-    // larger ones leave SMs idle. TARAL_PANELS=0: none (tests).
+    // larger ones leave SMs idle. Which matrices: panels_suit. TARAL_PANELS=0: none, 1: at any size (tests).
     PanelMat<T> panels[2];
     int npanels[2] = {0, 0};
     PanelSize panel_most[2];
@@ -294,10 +294,17 @@ struct Engine final : EngineBase {
         if ((e && !forced) || (flags & TARAL_FLAG_NO_GRAPH) || std::getenv("TARAL_PDL") || forced_row_split() >= 0 ||
             std::getenv("TARAL_ROWTHREAD") || (a.nnz() < (sizeof(T) == 4 ? 2000000 : 1500000) && !forced))
             return;
-        const int target = int(std::min<int64_t>(16384, std::max<int64_t>(8192, a.nnz() / (148 * 2) * 21 / 20)));
+        int dev, sms;
+        CK(cudaGetDevice(&dev));
+        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        const int target = int(std::min<int64_t>(16384, std::max<int64_t>(8192, a.nnz() / (sms * 2) * 21 / 20)));
+        auto suit = [&](int64_t panels_a, int64_t panels_t) {
+            return forced || panels_suit(a.nnz(), a.rows, at.rows, panels_a, panels_t, sms, sizeof(T) == 8);
+        };
+        if (!suit(least_panels(a.nnz(), a.rows, target), least_panels(a.nnz(), at.rows, target))) return;
         pa = build_panels(a.ptr, a.idx, a.rows, at.rows, target, kPanelCols, host_threads());
         if (!pa.empty()) pt = build_panels(at.ptr, at.idx, at.rows, a.rows, target, kPanelCols, host_threads());
-        if (pa.empty() || pt.empty()) pa = PanelPlan(), pt = PanelPlan();
+        if (pa.empty() || pt.empty() || !suit(int64_t(pa.panels.size()), int64_t(pt.panels.size()))) pa = PanelPlan(), pt = PanelPlan();
     }
     void put_panels(int which, const DevMat& d, const PanelPlan& p) {
         if (p.empty()) return;

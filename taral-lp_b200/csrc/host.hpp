@@ -88,15 +88,23 @@ inline CsrRef ref(const Csr& a) { return {a.rows, a.ptr.data(), a.idx.data(), a.
 Csr transpose_par(const int64_t* ptr, const int32_t* idx, const double* val, int rows, int cols, int threads);
 int host_threads();
 // work(q, begin, end) over [0, count) cut into `parts` contiguous ranges of about equal length, range 0 on the
-// calling thread and every other one on a thread of its own.
+// calling thread and every other one on a thread of its own (on the calling thread where no more can be started).
 template <class F>
 void split_ranges(int64_t count, int parts, F work) {
     parts = int(std::max<int64_t>(1, std::min<int64_t>(parts, count)));
-    std::vector<std::thread> pool;
-    for (int q = 1; q < parts; ++q)
-        pool.emplace_back([&work, q, count, parts] { work(q, count * q / parts, count * (q + 1) / parts); });
+    struct Pool {
+        std::vector<std::thread> threads;
+        ~Pool() { for (std::thread& t : threads) t.join(); }  // also where the calling thread's work throws
+    } pool;
+    int q = 1;
+    try {
+        pool.threads.reserve(size_t(parts - 1));
+        for (; q < parts; ++q)
+            pool.threads.emplace_back([&work, q, count, parts] { work(q, count * q / parts, count * (q + 1) / parts); });
+    } catch (const std::exception&) {
+    }
     work(0, int64_t(0), count / parts);
-    for (std::thread& t : pool) t.join();
+    for (; q < parts; ++q) work(q, count * q / parts, count * (q + 1) / parts);
 }
 
 // Scaled problem (gpu/pdhg.cu:72-78): A_s = diag(Dr) A diag(Dc).

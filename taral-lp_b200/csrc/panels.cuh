@@ -370,6 +370,7 @@ struct PanelPlan {
     int groups = 0;             // entry groups of 32 lanes x 4
     int long_entries = 0;
     int64_t padded = 0;         // entries stored
+    int64_t listed = 0;         // columns in the panels' lists
     PanelSize most;
     bool empty() const { return panels.empty(); }
     void append(const PanelPlan& p, int row_shift) {
@@ -381,18 +382,26 @@ struct PanelPlan {
         for (int4 q : p.longrow) longrow.push_back(make_int4(q.x + long_entries, q.y, q.z, 0));
         order.insert(order.end(), p.order.begin(), p.order.end());
         cols.insert(cols.end(), p.cols.begin(), p.cols.end());
-        groups += p.groups, long_entries += p.long_entries, padded += p.padded;
+        groups += p.groups, long_entries += p.long_entries, padded += p.padded, listed += p.listed;
         most.cover(p.most);
     }
 };
 
+// Marks of the columns that a panel has used, kept from panel to panel.
+struct PanelMarks {
+    std::vector<int> seen;
+    int stamp = 0;
+    explicit PanelMarks(int cols) : seen(size_t(cols), 0) {}
+};
 // Panels of about `target` nonzeros and at most max_cols columns for the rows [first, last); empty where a single row uses
-// more columns than that.
+// more columns than that. lists = false: their sizes only, without the column lists in order.
 template <class I>
-PanelPlan panels_of(const I* ptr, const int32_t* idx, int first, int last, int cols, int target, int max_cols) {
+PanelPlan panels_of(const I* ptr, const int32_t* idx, int first, int last, int cols, int target, int max_cols, PanelMarks& marks,
+                    bool lists = true) {
     PanelPlan plan;
-    std::vector<int> seen(size_t(cols), 0), list;
-    int stamp = 0, low = 0, high = 0;
+    std::vector<int>& seen = marks.seen;
+    std::vector<int> list;
+    int &stamp = marks.stamp, low = 0, high = 0;
     auto unique = [&](int r0, int r1) {  // columns of the rows [r0, r1) into list, unsorted, all of them in [low, high]
         list.clear(), ++stamp, low = cols, high = -1;
         for (I k = ptr[r0]; k < ptr[r1]; ++k) {
@@ -412,7 +421,9 @@ PanelPlan panels_of(const I* ptr, const int32_t* idx, int first, int last, int c
         Panel p{};
         p.row0 = r0, p.rows = r1 - r0, p.slice0 = int(plan.slice.size()), p.col0 = int(plan.cols.size()), p.cols = int(list.size());
         p.long0 = int(plan.longrow.size());
-        if (int64_t(high) - low < 16 * int64_t(list.size())) {  // in column order: the marks of the range
+        plan.listed += int64_t(list.size());
+        if (!lists) {
+        } else if (int64_t(high) - low < 16 * int64_t(list.size())) {  // in column order: the marks of the range
             for (int c = low; c <= high; ++c)
                 if (seen[size_t(c)] == stamp) plan.cols.push_back(c);
         } else {
@@ -448,6 +459,27 @@ PanelPlan panels_of(const I* ptr, const int32_t* idx, int first, int last, int c
     return plan;
 }
 
+// Whether an LP's products are faster on panels than on row blocks, by the number of panels of A and of A^T (a lower bound
+// refuses before they are planned). A panel kernel has 2 CTAs an SM: a second wave of panels costs what a first does (a
+// tenth of one starts as the first panels end), and a panel of short rows is bound by its 1,024 rows, not by its nonzeros.
+// Measured (us an iteration, row blocks / panels):
+//   up to 2.2 an SM: refinery of 64 periods (304 panels) FP32 29.8 / 25.6, FP64 52.3 / 40.1; band of 8 (280,000 rows) 12.7 /
+//              10.0 and 21.9 / 12.8; band of 20 (4.4M nonzeros) 20.4 / 14.8 and 42.3 / 26.0; blocks of 50 x 60 16.3 / 14.2,
+//              33.5 / 17.4; random in blocks of 300 x 500 (5M, 320 panels) 30.8 / 25.1 and 54.4 / 43.7
+//   more, FP32: refinery of 96 41.7 / 50.1, band of 20 (6M) 26.5 / 32.9, band of 100 (9M) 41.2 / 46.2, blocks of 150 x 200
+//              (6M) 33.2 / 30.5, (9.9M) 49.0 / 58.7, band of 8 (1M rows) 37.7 / 58.6
+//   more, FP64, full panels: refinery of 96 73.7 / 60.4, band of 100 (9M) 83.9 / 56.2, band of 20 (6M) 46.9 / 45.4; filled by
+//              their rows: band of 10 (400,000 rows) 33.5 / 39.7, band of 7 (600,000) 35.6 / 38.1
+//   rows of fewer than 8: band of 6 (350,000 rows) 10.8 / 17.7 and 13.8 / 24.5, band of 7 (304 panels) 10.8 / 14.9
+constexpr int kFullPanel = 15000;  // of the largest target, 16,384
+inline bool panels_suit(int64_t nnz, int64_t m, int64_t n, int64_t panels_a, int64_t panels_t, int sms, bool fp64) {
+    const int64_t most = std::max(panels_a, panels_t);
+    return nnz >= 8 * std::max(m, n) && (5 * most <= 11 * int64_t(sms) || (fp64 && nnz >= kFullPanel * most));
+}
+inline int64_t least_panels(int64_t nnz, int64_t rows, int target) {
+    return std::max((nnz + target - 1) / target, (rows + kPanelRows - 1) / kPanelRows);
+}
+
 // Panels for the CSR rows on `threads` host threads (max_cols <= kPanelCols), or none where they do not pay: the column
 // lists must hold at most a third as many columns as the panels hold nonzeros (a list and its entries of x cost about as
 // much to read as they save otherwise), and padding at most 40 % of the nonzeros.
@@ -458,32 +490,35 @@ PanelPlan plan_of_panels(const I* ptr, const int32_t* idx, int rows, int cols, i
     for (int r = 0; r < rows; ++r)
         if (ptr[r + 1] - ptr[r] > I(kTile)) return plan;  // summed by a whole CTA in the row blocks
     const int64_t all = int64_t(ptr[rows] - ptr[0]);
-    auto pays = [](const PanelPlan& p, int64_t nnz) { return nnz >= 3 * int64_t(p.cols.size()) && 10 * p.padded <= 14 * nnz; };
+    auto pays = [](const PanelPlan& p, int64_t nnz) { return nnz >= 3 * p.listed && 10 * p.padded <= 14 * nnz; };
     {  // a look at a few rows first: most matrices without shared columns are refused here
+        PanelMarks marks(cols);
         PanelPlan look;
         int64_t nnz = 0;
         for (int q = 0; q < 4; ++q) {
             const int r0 = int(int64_t(rows) * q / 4);
             int r1 = r0;
             while (r1 < rows && ptr[r1] - ptr[r0] < I(target)) ++r1;
-            const PanelPlan p = panels_of(ptr, idx, r0, r1, cols, target, max_cols);
+            const PanelPlan p = panels_of(ptr, idx, r0, r1, cols, target, max_cols, marks, false);
             if (p.empty()) return plan;
             look.append(p, 0), nnz += int64_t(ptr[r1] - ptr[r0]);
         }
         if (!pays(look, nnz)) return plan;
     }
-    threads = int(std::max<int64_t>(1, std::min<int64_t>(threads, all / (8 * int64_t(target)))));
-    std::vector<PanelPlan> part(static_cast<size_t>(threads));
-    split_ranges(threads, threads, [&](int, int64_t q0, int64_t q1) {
-        for (int64_t q = q0; q < q1; ++q) {
-            auto cut = [&](int64_t k) {
-                return k >= threads ? rows : int(std::lower_bound(ptr, ptr + rows, ptr[0] + I(all * k / threads)) - ptr);
-            };
-            try {
-                part[size_t(q)] = panels_of(ptr, idx, cut(q), cut(q + 1), cols, target, max_cols);
-            } catch (const std::bad_alloc&) {  // no exception leaves a thread: its rows are not covered, and there are no panels
-                part[size_t(q)] = PanelPlan();
+    // parts planned on their own (each ends with a panel that is not full), the same on every host
+    const int parts = int(std::max<int64_t>(1, std::min<int64_t>(16, all / (8 * int64_t(target)))));
+    std::vector<PanelPlan> part(static_cast<size_t>(parts));
+    split_ranges(parts, threads, [&](int, int64_t q0, int64_t q1) {
+        try {
+            PanelMarks marks(cols);
+            for (int64_t q = q0; q < q1; ++q) {
+                auto cut = [&](int64_t k) {
+                    return k >= parts ? rows : int(std::lower_bound(ptr, ptr + rows, ptr[0] + I(all * k / parts)) - ptr);
+                };
+                part[size_t(q)] = panels_of(ptr, idx, cut(q), cut(q + 1), cols, target, max_cols, marks);
             }
+        } catch (const std::bad_alloc&) {  // no exception leaves a thread
+            for (int64_t q = q0; q < q1; ++q) part[size_t(q)] = PanelPlan();
         }
     });
     for (const PanelPlan& p : part) plan.append(p, 0);
