@@ -94,9 +94,11 @@ int pdhg_restart(pdhg_ctx* ctx, int avg, double f);
 int pdhg_download(pdhg_ctx* ctx, int avg, double f, double* x, double* z);
 /* Gpu::name / Gpu::mem_used. name_out receives at most cap bytes (NUL-terminated). */
 int pdhg_info(pdhg_ctx* ctx, char* name_out, size_t cap, size_t* mem_used);
-/* Total kernels this context has launched: graph replays count their kernels, and a launch that takes a whole block of
- * iterations, an evaluation or the power iteration counts the phases it takes. */
+/* The steps this context has queued, counted as kernels of one phase each: 1 + 2 * steps for a block of iterations, 6 for
+ * pdhg_eval_pair, whether each phase was a launch of its own or one launch took several. */
 int64_t pdhg_kernel_launches(const pdhg_ctx* ctx);
+/* The kernels this context has launched (graph replays count theirs). */
+int64_t pdhg_device_launches(const pdhg_ctx* ctx);
 const char* pdhg_last_error(const pdhg_ctx* ctx);
 void pdhg_destroy(pdhg_ctx* ctx);
 
@@ -146,7 +148,7 @@ typedef struct {
     double max_row_violation, max_bound_violation; /* original model, absolute */
     double scale_s, device_init_s, transfer_s, solve_s, power_iter_s;
     size_t device_mem_bytes;
-    int64_t kernel_launches;
+    int64_t kernel_launches; /* kernels launched, as pdhg_device_launches counts them */
     int64_t nnz;
     double device_s;        /* pdhg_solve_ctx: CUDA-event time of the solve on the context stream */
 } taral_outcome;

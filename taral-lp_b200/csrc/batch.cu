@@ -1446,7 +1446,7 @@ struct Batch final : BatchBase {
     void block(int steps) {
         if (cluster_ctas > 0) {
             BK(launch_cluster(k_cluster_iterate<T, true>, k_cluster_iterate<T, false>, d_lps, ninst, cluster_ctas, cluster_smem, s, steps));
-            launches += 1 + 2 * int64_t(steps);  // the phases, as when each is a launch of its own
+            ++launches;
         } else {
             if (nT) k_pack_xupd<T><<<nT, kThreads, 0, s>>>(T_ev, Te_ev, slot_inst, running, x, ATz, c, l, u, par, xs), ++launches;
             for (int k = 0; k < steps; ++k) {
@@ -1547,6 +1547,7 @@ struct Batch final : BatchBase {
         // power iteration per instance (gpu/pdhg.cu:416-436)
         k_power_starts<T><<<matrix_ctas() * distinct, 256, 0, s>>>(pw_first, pw_cols, pw_width, pw_norm, pv, pscale, matrix_ctas());
         BK(cudaGetLastError());
+        ++launches;
         // One estimate per distinct matrix: instances that share a matrix share its scaled copy, its row blocks and
         // the deterministic start vector, so their power iterations are the same numbers; only the first instance
         // of each matrix iterates, the others take its estimate.
@@ -1562,10 +1563,8 @@ struct Batch final : BatchBase {
             std::vector<double> got(2 * size_t(distinct));
             BK(cudaMemcpyAsync(got.data(), d_norms, got.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
             BK(cudaStreamSynchronize(s));
-            for (int k = 0; k < distinct; ++k) {
-                norms[size_t(first_inst[size_t(k)])] = got[2 * size_t(k)];
-                launches += 2 * int64_t(got[2 * size_t(k) + 1]);  // the products, as when each is a launch of its own
-            }
+            for (int k = 0; k < distinct; ++k) norms[size_t(first_inst[size_t(k)])] = got[2 * size_t(k)];
+            ++launches;
         } else {
             power_iteration();
             BK(cudaMemcpyAsync(norms.data(), est, ninst * sizeof(double), cudaMemcpyDeviceToHost, s));

@@ -808,7 +808,7 @@ struct Engine final : EngineBase {
         if (cluster_ctas > 0) {
             CK(launch_cluster(k_cluster_power<T, true>, k_cluster_power<T, false>, d_lp, 1, cluster_ctas, cluster_smem, st, iters, h_out));
             CK(cudaStreamSynchronize(st));
-            launches += 2 * int64_t(h_out[1]);  // the products, as when each is a launch of its own
+            launches += 2 * int64_t(h_out[1]), folded += 2 * int64_t(h_out[1]) - 1;
             return h_out[0];
         }
         if (resident_ctas > 0 && npanels[0] == 0) {
@@ -816,7 +816,7 @@ struct Engine final : EngineBase {
                             resident_args(h_out), pv, pw, iters, red_grid(n));
             CK(cudaStreamSynchronize(st));
             check_resident();
-            launches += 2 * int64_t(h_out[1]);  // the products, as when each is a launch of its own
+            launches += 2 * int64_t(h_out[1]), folded += 2 * int64_t(h_out[1]) - 1;
             return h_out[0];
         }
         T *a = pv, *b = pu;
@@ -907,11 +907,11 @@ struct Engine final : EngineBase {
         if (steps <= 0) return;
         if (cluster_ctas > 0) {
             CK(launch_cluster(k_cluster_iterate<T, true>, k_cluster_iterate<T, false>, d_lp, 1, cluster_ctas, cluster_smem, st, steps));
-            launches += 1 + 2 * int64_t(steps);  // the phases, as when each is a launch of its own
+            launches += 1 + 2 * int64_t(steps), folded += 2 * int64_t(steps);
         } else if (resident_iterates) {
             launch_resident(k_resident_iterate<T>, sizeof(RowSmem<T>), 0,
                             resident_args(out), steps);
-            launches += 1 + 2 * int64_t(steps);  // the phases, as when each is a launch of its own
+            launches += 1 + 2 * int64_t(steps), folded += 2 * int64_t(steps);
         } else if (use_graph && steps == eval_freq) {
             if (!graph) {
                 cudaGraph_t g;
@@ -962,7 +962,7 @@ struct Engine final : EngineBase {
         if (resident_ctas > 0) {  // the scalars go straight to the pinned status block
             launch_resident(k_resident_eval<T>,
                             sizeof(RowSmem<double>), 20 * kEvalCtas * sizeof(double), resident_args(h_out), f, red_grid(m), red_grid(n));
-            launches += 6;  // the phases, as when each is a launch of its own
+            launches += 6, folded += 5;
         } else {
             queue_eval(false, 1.0, out);
             queue_eval(true, f, out + 10);
@@ -1243,7 +1243,7 @@ extern "C" int pdhg_solve_ctx(pdhg_ctx* ctx, double bnorm, double cnorm, const t
     EngineBase& e = *ctx->e;
     taral::DriverData P{int(e.hrl.size()), int(e.hc.size()), e.hc.data(), e.hrl.data(), e.hru.data(), bnorm, cnorm};
     GUARD(ctx, {
-        int64_t l0 = e.launches;
+        const int64_t l0 = e.device_launches();
         auto t0 = taral::Clock::now();
         e.mark();
         taral::Outcome r = taral::run(e, P, op, op.time_limit, x0, z0);
@@ -1254,7 +1254,7 @@ extern "C" int pdhg_solve_ctx(pdhg_ctx* ctx, double bnorm, double cnorm, const t
         out->from_average = r.from_average ? 1 : 0;
         out->rel_primal = r.rel_primal, out->rel_dual = r.rel_dual, out->rel_gap = r.rel_gap;
         out->norm_a = r.norm_a, out->primal_weight = r.omega, out->power_iter_s = r.power_s;
-        out->device_mem_bytes = e.mem_used, out->kernel_launches = e.launches - l0;
+        out->device_mem_bytes = e.mem_used, out->kernel_launches = e.device_launches() - l0;
         if (x) std::memcpy(x, r.x.data(), r.x.size() * sizeof(double));
         if (z) std::memcpy(z, r.z.data(), r.z.size() * sizeof(double));
     })
@@ -1279,6 +1279,7 @@ extern "C" int pdhg_scaled_problem(pdhg_ctx* ctx, double* Dr, double* Dc, double
     GUARD(ctx, ctx->e->scaled_values(Dr, Dc, A_val, AT_val))
 }
 extern "C" int64_t pdhg_kernel_launches(const pdhg_ctx* ctx) { return ctx ? ctx->e->launches : 0; }
+extern "C" int64_t pdhg_device_launches(const pdhg_ctx* ctx) { return ctx ? ctx->e->device_launches() : 0; }
 extern "C" const char* pdhg_last_error(const pdhg_ctx* ctx) { return ctx ? ctx->err.c_str() : "NULL context"; }
 extern "C" void pdhg_destroy(pdhg_ctx* ctx) { delete ctx; }
 extern "C" void taral_set_device_alloc_limit(size_t bytes) { taral::g_alloc_limit.store(bytes); }

@@ -15,7 +15,9 @@ namespace taral {
 struct EngineBase {
     std::string name;
     size_t mem_used = 0;
-    int64_t launches = 0;
+    int64_t launches = 0;  // kernels, with the phases that one launch takes counted as when each is a launch of its own
+    int64_t folded = 0;    // phases that were not launches of their own
+    int64_t device_launches() const { return launches - folded; }
     int64_t nnz = 0;  // nonzeros of A
     int tuned[2] = {0, 0};  // row-split policy chosen by the autotuner for A and A^T
     bool per_thread[2] = {false, false};  // A, A^T use the one-thread-per-row SpMV kernel

@@ -107,7 +107,7 @@ int solve_model(const taral_model& md, const Options& o, SolveResult& res, const
         return TARAL_ERR_CUDA;
     }
     res.solve_s = since(t);
-    res.kernel_launches = e->launches;
+    res.kernel_launches = e->device_launches();
     res.nnz = e->nnz;
     const int tuned_a = e->tuned[0] + (e->per_thread[0] ? 10 : 0), tuned_t = e->tuned[1] + (e->per_thread[1] ? 10 : 0);
     t = Clock::now();

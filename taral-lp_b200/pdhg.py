@@ -89,6 +89,7 @@ SIGNATURES = {
     "pdhg_solve_ctx": (C.c_int, [C.c_void_p, C.c_double, C.c_double, C.c_void_p, _dp, _dp, C.c_void_p, _dp, _dp]),
     "pdhg_profile_phases": (C.c_int, [C.c_void_p, C.c_int, _dp, _dp]),
     "pdhg_kernel_launches": (C.c_int64, [C.c_void_p]),
+    "pdhg_device_launches": (C.c_int64, [C.c_void_p]),
     "pdhg_last_error": (C.c_char_p, [C.c_void_p]),
     "pdhg_destroy": (None, [C.c_void_p]),
     "taral_options_default": (None, [C.POINTER(OptionsT)]),
@@ -301,6 +302,10 @@ class Engine:
     @property
     def kernel_launches(self):
         return lib().pdhg_kernel_launches(self.h)
+
+    @property
+    def device_launches(self):
+        return lib().pdhg_device_launches(self.h)
 
     def close(self):
         if getattr(self, "h", None):

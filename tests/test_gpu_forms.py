@@ -123,6 +123,31 @@ def test_barrier_that_gives_up_is_reported(engine_lib, monkeypatch, call):
     eng.close()
 
 
+@pytest.mark.parametrize("resident,block,pair", [("0", 1 + 2 * 64, 6), ("1", 1, 1), ("2", 1, 1)], ids=["phases", "grid", "cluster"])
+def test_launches_are_counted(engine_lib, monkeypatch, resident, block, pair):
+    """device_launches and a solve's kernel_launches are what the device was given; kernel_launches of a context counts the
+    phases, the same in every form."""
+    monkeypatch.setenv("TARAL_RESIDENT", resident)
+    eng = pdhg.Engine.from_model(lpgen.packing(2000, seed=3))
+    eng.set_steps(0.5, 0.5)
+    eng.start()
+
+    def counted(call):
+        before = eng.device_launches, eng.kernel_launches
+        call()
+        return eng.device_launches - before[0], eng.kernel_launches - before[1]
+    assert counted(lambda: eng.iterate(64)) == (block, 129)
+    assert counted(lambda: eng.iterate(1)) == (1 + 2 if resident == "0" else 1, 3)
+    assert counted(lambda: eng.eval_pair(1 / 64)) == (pair, 6)
+    launched, _ = counted(lambda: eng.power_norm(50))
+    # the start vector, and chunks of 8 steps of 4 launches or all steps in one
+    assert launched >= 1 + 8 * 4 if resident == "0" else launched == 2
+    before = eng.device_launches
+    r, _, _ = eng.solve(eng.bnorm, eng.cnorm, tol=1e-12, max_iter=128)
+    assert r["kernel_launches"] == eng.device_launches - before
+    eng.close()
+
+
 def _engine_numbers(lp, precision):
     eng = pdhg.Engine.from_model(lp, precision=precision)
     norm = eng.power_norm(30)
