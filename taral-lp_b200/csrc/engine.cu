@@ -683,12 +683,13 @@ struct Engine final : EngineBase {
     int barrier_polls = kBarrierPolls;
     int resident_ctas = 0;  // CTAs of a resident launch, 0: the phase kernels
     bool resident_iterates = false;  // iteration blocks too (every tile has a team of its own), not only evaluations
+    bool resident_powers = false;    // the power iteration too
     int cluster_ctas = 0;   // CTAs of the LP's cluster (cluster.cuh), 0: not on one cluster
     size_t cluster_smem = 0;
     ClusterLp<T>* d_lp = nullptr;
     int rparity = 0;
     void choose_resident() {
-        resident_ctas = 0, resident_iterates = false;
+        resident_ctas = 0, resident_iterates = resident_powers = false;
         if (!use_graph || pdl || A.nblk == 0 || AT.nblk == 0) return;
         int dev, sms, coop, mode = -1;
         CK(cudaGetDevice(&dev));
@@ -700,6 +701,13 @@ struct Engine final : EngineBase {
         resident_blocks(A, sms), resident_blocks(AT, sms);
         resident_ctas = std::min(sms, std::max(A.rnblk, AT.rnblk));
         cluster_ctas = 0;
+        // The power iteration: 4 grid barriers a step against 4 launches, but 2 teams an SM where the phases have 5 to 8
+        // CTAs; a row of many tiles is one team's work. Measured (us a step, phases / resident): 528 tiles FP32 25.0 / 21.6,
+        // FP64 29.4 / 24.0; 735 29.1 / 28.2, 33.7 / 30.8; 980 planted 35.8 / 35.5, 45.9 / 40.2, power-law 35.1 / 41.2, 44.4 /
+        // 42.6; 1,800 55.9 / 56.6, 71.6 / 63.4; 2,450 power-law 63.7 / 89.2, 77.7 / 93.8; 3,906 80 / 100, 100 / 105; one row of
+        // 20,000 nonzeros 20.7 / 22.0, 22.0 / 20.7, of 100,000 57.6 / 81.6, 58.9 / 75.4.
+        const int tiles = std::max(A.rnblk, AT.rnblk), per_team = sizeof(T) == 4 ? 2 : 8;
+        resident_powers = npanels[0] == 0 && ((tiles <= per_team * kTeams * sms && std::max(A.maxrow, AT.maxrow) <= 16 * kTile) || mode >= 1);
         // the tuner's choice for the phases, or panels
         if (A.per_thread || AT.per_thread || tuned[0] == 2 || tuned[1] == 2 || npanels[0]) return;
         resident_iterates = mode >= 1 || std::max(A.rnblk, AT.rnblk) <= kTeams * sms;
@@ -811,7 +819,7 @@ struct Engine final : EngineBase {
             launches += 2 * int64_t(h_out[1]), folded += 2 * int64_t(h_out[1]) - 1;
             return h_out[0];
         }
-        if (resident_ctas > 0 && npanels[0] == 0) {
+        if (resident_powers) {
             launch_resident(k_resident_power<T>, sizeof(RowSmem<T>), 0,
                             resident_args(h_out), pv, pw, iters, red_grid(n));
             CK(cudaStreamSynchronize(st));

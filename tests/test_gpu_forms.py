@@ -148,6 +148,37 @@ def test_launches_are_counted(engine_lib, monkeypatch, resident, block, pair):
     eng.close()
 
 
+@pytest.mark.parametrize("precision,tiles,long,resident", [
+    (pdhg.FP32, 560, 0, True), (pdhg.FP32, 640, 0, False), (pdhg.FP64, 640, 0, True), (pdhg.FP64, 2300, 0, True),
+    (pdhg.FP64, 2450, 0, False), (pdhg.FP64, 560, 33_000, False), (pdhg.FP32, 100, 25_600, True),
+])
+def test_power_iteration_form(engine_lib, monkeypatch, precision, tiles, long, resident):
+    """One launch for the whole power iteration up to the sizes where it is the faster one, a launch per phase beyond and
+    where a row is many tiles long; the same norm bit for bit."""
+    monkeypatch.setenv("TARAL_TUNE", "0")
+    n = 256 * tiles  # columns of 5: a tile of A^T holds 256 of them
+    lp = lpgen.planted(max(n // 3, 100), n, 5, seed=1)
+    if long:  # one row more, over the first columns: longer than 16 tiles of 2,044 nonzeros or not
+        rows = np.split(lp.row_idx, lp.col_ptr[1:-1])
+        vals = np.split(lp.val, lp.col_ptr[1:-1])
+        rows = [np.append(r, lp.m) if j < long else r for j, r in enumerate(rows)]
+        vals = [np.append(v, 0.01) if j < long else v for j, v in enumerate(vals)]
+        ptr = np.concatenate([[0], np.cumsum([r.size for r in rows])]).astype(np.int64)
+        lp = dataclasses.replace(lp, m=lp.m + 1, col_ptr=ptr, row_idx=np.concatenate(rows).astype(np.int32), val=np.concatenate(vals),
+                                 row_lo=np.append(lp.row_lo, -np.inf), row_up=np.append(lp.row_up, np.inf))
+    norms = {}
+    for mode in (None, "0"):
+        if mode is not None:
+            monkeypatch.setenv("TARAL_RESIDENT", mode)
+        eng = pdhg.Engine.from_model(lp, precision=precision)
+        before = eng.device_launches
+        norms[mode] = eng.power_norm(24)
+        if mode is None:
+            assert (eng.device_launches - before == 2) == resident
+        eng.close()
+    assert norms[None] == norms["0"]
+
+
 def _engine_numbers(lp, precision):
     eng = pdhg.Engine.from_model(lp, precision=precision)
     norm = eng.power_norm(30)
