@@ -561,6 +561,7 @@ struct Shared {  // one distinct scaled matrix
     int dr_off = 0, dc_off = 0;  // offsets of this matrix's Dr / Dc in the device scaling scratch
     int maxrowA = 0, maxrowT = 0;  // longest row of A and of A^T
     PanelPlan panels[2];           // of A and of A^T, until they are uploaded
+    int looked = 0, adjacent = 0;  // of A's first entries, those whose column follows the one before
 };
 
 uint64_t fnv(const void* p, size_t n, uint64_t h) {  // FNV-1a over 8-byte words, then the tail bytes
@@ -785,6 +786,8 @@ struct Batch final : BatchBase {
                 if (sh.panels[1].empty()) panels_ok = false;
             }
             sh.S.m = mk.m, sh.S.n = mk.n, sh.nnz = int64_t(sh.S.A.idx.size());
+            sh.looked = int(std::min<int64_t>(sh.nnz, 4096));
+            for (int e = 1; e < sh.looked; ++e) sh.adjacent += sh.S.A.idx[size_t(e)] == sh.S.A.idx[size_t(e) - 1] + 1;
         });
         mark("transposes");
         // 3. concatenated matrices (int32 offsets), uploaded unscaled and scaled on the device (scaling.cuh:
@@ -1169,37 +1172,69 @@ struct Batch final : BatchBase {
         pw_ev = put(ev), pwe_ev = put(eve), pw_first = put(first), pw_range = put(range), pw_cols = put(cols_of), pw_width = put(widths), pw_norm = put(norms), pw_taken = alloc<int>(size_t(distinct));
     }
 
-    // Small instances on one cluster each (cluster.cuh): where the launch's waves of clusters, at about 0.9 us an iteration
-    // + 0.33 us a thousand nonzeros of a CTA (+ 1 us for the cluster's barriers and exchange), take less than the phase
-    // kernels' 7.5 us + 8 us a million products. Measured, FP64: 40 instances of 151 x 347 (1,400 nonzeros) 1.4 against 9 us.
+    // Small instances on one cluster each (cluster.cuh): where the waves of clusters that fit the GPU at the same time, at the
+    // plan's estimate for the slowest matrix, take less than the phase kernels. Those are estimated at 7 us (9 with rows of
+    // more than 32 on average) + a us a million products + b us a million rows and columns, where neighbouring entries are
+    // neighbours in memory (a 2.8, b 4; FP64 4.5, 9) or not (3.2, 8; 7, 10), on panels 0.6 times that. Beyond 3 waves the phase
+    // kernels fill the GPU: a margin of 0.8 there (FP64 0.85, one CTA 0.95), 0.9 before. Measured, FP32 and FP64, us an
+    // iteration with phases / clusters: 40 of 150 x 350 7.5 / 1.4, 7.5 / 1.3; 400 of them 9.7 / 4.2, 12.1 / 3.8; 100 of 700 x 1,633
+    // 10.2 / 9.0, 12.0 / 9.2; 200 14.0 / 15.8, 17.4 / 16.0; 40 of 1,500 x 3,500 9.7 / 8.2, 11.2 / 9.0; 100 15.6 / 18.8, 19.0 / 20.9;
+    // 200 bands of 8 (1,000 rows) 11.7 / 13.8, 17.1 / 14.3; 16 of dense 200 x 200 9.4 / 7.7, 10.3 / 7.4; 100 11.9 / 27.0, 25.5 /
+    // 25.7; 16 of 600 x 800 in dense blocks of 150 x 200 FP32 12.9 / 25.0 (more than 65,536 nonzeros: longer than estimated).
     void choose_cluster() {
         const char* res = std::getenv("TARAL_RESIDENT");
         if (pdl || (res && std::atoi(res) == 0) || forced_row_split() > 0 || std::getenv("TARAL_ROWTHREAD")) return;
         if (std::getenv("TARAL_ROWSPLIT") || packs.size() != size_t(ninst)) return;
-        int64_t most = 0;
-        for (const auto& sh : mats) {
-            if (sh->maxrowA > kTile || sh->maxrowT > kTile || sh->S.m > kClusterRows || sh->S.n > kClusterRows) return;
-            if (sh->S.m == 0 || sh->S.n == 0) return;
-            most = std::max(most, sh->nnz);
+        size_t largest = 0;
+        for (size_t k = 0; k < mats.size(); ++k) {
+            const Shared& sh = *mats[k];
+            if (sh.maxrowA > kTile || sh.maxrowT > kTile || sh.S.m > kClusterRows || sh.S.n > kClusterRows) return;
+            if (sh.S.m == 0 || sh.S.n == 0) return;
+            if (sh.nnz > mats[largest]->nnz) largest = k;
         }
         int dev, sms;
         BK(cudaGetDevice(&dev));
         BK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        std::vector<std::vector<int>> plans(mats.size());
-        for (int q = cluster_size(most); q <= 8; q *= 2) {
-            const double waves = std::ceil(double(ninst) * q / double(q > 1 ? 128 : sms));
-            const double cluster = waves * (0.9 + 0.33e-3 * double(most) / q + (q > 1 ? 1.0 : 0.0));
-            if (cluster > 7.5 + 8e-6 * double(nnz_total)) return;
+        if (mats[largest]->nnz > 65536) return;
+        const bool near = 2 * mats[largest]->adjacent > mats[largest]->looked, fp32 = sizeof(T) == 4;
+        const double product = near ? (fp32 ? 2.8e-6 : 4.5e-6) : (fp32 ? 3.2e-6 : 7e-6), row = near ? (fp32 ? 4e-6 : 9e-6) : (fp32 ? 8e-6 : 1e-5);
+        const double phases = ((nnz_total > 32 * int64_t(std::max(M, N)) ? 9 : 7) + product * double(nnz_total) + row * (double(M) + double(N))) *
+                              (npanels[0] ? 0.6 : 1.0);
+        for (int q = cluster_size(mats[largest]->nnz); q <= 8; q *= 2) {
+            auto pays = [&](double us, int at_once) {
+                const double waves = double(ninst) / at_once;
+                const double margin = q == 1 ? 0.95 : waves <= 3 ? 0.9 : fp32 ? 0.8 : 0.85;
+                return waves <= 8 && (waves <= 3 ? std::ceil(waves) : waves) * us <= margin * phases;
+            };
+            if (!pays(q > 1 ? 1.9 : 1.0, std::max(1, sms / q))) return;  // the least that a plan comes to
             size_t need = 0;
-            for (size_t k = 0; k < mats.size() && need <= kClusterSmem; ++k) {
+            double us = 0;
+            int at_once = 0;
+            std::vector<int> all, one;  // the plans, one after another
+            std::vector<size_t> start(mats.size());
+            auto plan = [&](size_t k) {
                 const Shared& sh = *mats[k];
                 const std::vector<int> ap(sh.S.A.ptr.begin(), sh.S.A.ptr.end()), tp(sh.S.AT.ptr.begin(), sh.S.AT.ptr.end());
-                need = std::max(need, cluster_plan<T>(ap.data(), tp.data(), sh.S.m, sh.S.n, q, plans[k]));
-            }
-            if (need > kClusterSmem) continue;
-            std::vector<int*> d_plan;
+                double t;
+                need = std::max(need, cluster_plan<T>(ap.data(), tp.data(), sh.S.m, sh.S.n, q, one, &t));
+                us = std::max(us, t);
+                start[k] = all.size();
+                all.insert(all.end(), one.begin(), one.end());
+                return need <= kClusterSmem;
+            };
+            auto go = [&] {  // with what has been planned so far
+                BK(clusters_at_once<T>(q, need, &at_once));
+                return at_once > 0 && pays(us, at_once);
+            };
+            bool fits = plan(largest);
+            if (fits && !go()) return;
+            for (size_t k = 0; k < mats.size() && fits; ++k)
+                if (k != largest) fits = plan(k);
+            if (!fits) continue;
+            if (!go()) return;
+            int* d_plan = nullptr;
             if (!if_memory([&] {
-                    for (const auto& p : plans) d_plan.push_back(put(p));
+                    d_plan = put(all);
                     d_lps = alloc<ClusterLp<T>>(size_t(ninst)), d_first_lps = alloc<ClusterLp<T>>(mats.size()), d_norms = alloc<double>(2 * mats.size());
                 }))
                 return;
@@ -1210,7 +1245,7 @@ struct Batch final : BatchBase {
                 const int rb = pk.rbase, cb = pk.cbase;
                 ClusterLp<T> lp{Aptr + sh.pbaseA, Aidx, Tptr + sh.pbaseT, Tidx, Aval, Tval, sh.S.m, sh.S.n, x + cb, z + rb, Ax + rb,
                                 ATz + cb, xs + cb, zs + rb, c + cb, l + cb, u + cb, rl + rb, ru + rb, par + 2 * i, pv + cb,
-                                d_plan[size_t(mat_of[size_t(i)])], running + i};
+                                d_plan + start[size_t(mat_of[size_t(i)])], running + i};
                 lps.push_back(lp);
                 lp.active = nullptr;
                 if (first_inst[size_t(mat_of[size_t(i)])] == i) firsts.push_back(lp);  // in the order of the matrices

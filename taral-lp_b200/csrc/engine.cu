@@ -712,15 +712,18 @@ struct Engine final : EngineBase {
         if (A.per_thread || AT.per_thread || tuned[0] == 2 || tuned[1] == 2 || npanels[0]) return;
         resident_iterates = mode >= 1 || std::max(A.rnblk, AT.rnblk) <= kTeams * sms;
         if (mode == 1 || A.maxrow > kTile || AT.maxrow > kTile || m > kClusterRows || n > kClusterRows) return;
-        // One cluster where its time, about 1 us an iteration + 41 ns a KB of x and z + 40 ns a thousand nonzeros, is below
-        // the grid's 5 us. Measured (grid / cluster, us an iteration): planted 2,000 x 5,000 (25,000 nonzeros) FP32 5.4 /
-        // 3.6, FP64 4.9 / 4.2; 3,000 x 7,500 (37,500) FP32 5.4 / 4.3, FP64 5.1 / 5.9; 4,000 x 10,000 FP64 5.1 / 7.6.
+        // One cluster where its time is below the grid's, which is 4.5 to 6 us an iteration whatever the LP. Measured (grid /
+        // cluster): planted 2,000 x 5,000 (25,000 nonzeros) FP32 5.4 / 3.6, FP64 4.9 / 4.2; 3,000 x 7,500 FP32 5.4 / 4.3, FP64 5.1
+        // / 5.9; band of 60, 1,200 rows, FP32 5.9 / 15.5 (75 rows for a warp to take one after another). Beyond 90,000 bytes of x
+        // and z and nonzeros no plan comes below it.
         const char* cl = std::getenv("TARAL_CLUSTER");
         if (!cl && int64_t(m + n) * int64_t(sizeof(T)) + A.nnz > 90000) return;
         for (int q = cl ? std::atoi(cl) : cluster_size(A.nnz); q <= kClusterMax; q *= 2) {
             std::vector<int> plan;
-            const size_t need = cluster_plan<T>(A.hptr.data(), AT.hptr.data(), m, n, q, plan);
+            double us;
+            const size_t need = cluster_plan<T>(A.hptr.data(), AT.hptr.data(), m, n, q, plan, &us);
             if (need > kClusterSmem) continue;
+            if (!cl && us > 5) return;
             int* d_plan = nullptr;
             if (!if_memory([&] { d_plan = alloc<int>(plan.size()), d_lp = alloc<ClusterLp<T>>(1); })) return;
             cluster_ctas = q, cluster_smem = need;

@@ -179,6 +179,51 @@ def test_power_iteration_form(engine_lib, monkeypatch, precision, tiles, long, r
     assert norms[None] == norms["0"]
 
 
+def _blocks(count, rows, cols, seed=0):
+    """A block-diagonal LP of dense blocks."""
+    rng = np.random.default_rng(seed)
+    m, n = count * rows, count * cols
+    idx = ((np.arange(n) // cols * rows)[:, None] + np.arange(rows)).ravel().astype(np.int32)
+    val, x = rng.standard_normal(n * rows), rng.uniform(0, 1, n)
+    b = np.zeros(m)
+    np.add.at(b, idx, val * np.repeat(x, rows))
+    return lpgen.LP(f"blocks_{count}", m, n, np.arange(n + 1, dtype=np.int64) * rows, idx, val, rng.standard_normal(n), np.zeros(n),
+                    np.full(n, 10.0), b, b.copy())
+
+
+@pytest.mark.parametrize("lp,precision,cluster", [
+    (lambda: lpgen.planted(2000, 5000, 5, seed=1), pdhg.FP64, True), (lambda: lpgen.general(307, 701, seed=1), pdhg.FP32, True),
+    (lambda: _blocks(4, 100, 100), pdhg.FP32, False), (lambda: _blocks(12, 70, 80), pdhg.FP32, False),
+], ids=["planted", "general", "long_rows", "many_long_rows"])
+def test_cluster_choice(engine_lib, monkeypatch, lp, precision, cluster):
+    """One LP runs on a cluster where the plan's estimate is below the grid's time, not where a warp would take many long
+    rows one after another."""
+    lp, mem = lp(), {}
+    for mode in ("1", "2"):  # 1: never a cluster
+        monkeypatch.setenv("TARAL_RESIDENT", mode)
+        eng = pdhg.Engine.from_model(lp, precision=precision)
+        mem[mode] = eng.info()[1]
+        eng.close()
+    assert (mem["2"] > mem["1"]) == cluster
+
+
+@pytest.mark.parametrize("lps,precision,cluster", [
+    (lambda: [lpgen.general(151, 347, seed=k) for k in range(40)], pdhg.FP64, True),
+    (lambda: [lpgen.general(1500, 3500, seed=1)] * 14, pdhg.FP32, True),
+    (lambda: [lpgen.general(1500, 3500, seed=1)] * 128, pdhg.FP32, False),   # more waves of clusters than they are worth
+    (lambda: [_blocks(4, 150, 200)] * 16, pdhg.FP32, False),                 # long rows
+    (lambda: [_blocks(2, 100, 100)] * 100, pdhg.FP32, False),
+], ids=["small", "a_wave", "many_waves", "large", "long_rows"])
+def test_batch_cluster_choice(engine_lib, monkeypatch, lps, precision, cluster):
+    lps, mem = lps(), {}
+    for mode in ("0", "2"):
+        monkeypatch.setenv("TARAL_RESIDENT", mode)
+        b = pdhg.Batch(lps, precision=precision)
+        mem[mode] = b.info()["device_mem_bytes"]
+        b.close()
+    assert (mem["2"] > mem["0"]) == cluster
+
+
 def _engine_numbers(lp, precision):
     eng = pdhg.Engine.from_model(lp, precision=precision)
     norm = eng.power_norm(30)
