@@ -31,14 +31,15 @@ def _drive(eng, reps, out, errors):
     ("cluster", lambda: lpgen.planted(900, 2300, 5, seed=2), lambda: lpgen.planted(2000, 5000, 5, seed=2)),
     ("grid", lambda: lpgen.general(30, 70, seed=1), lambda: lpgen.planted(60_000, 150_000, 6, seed=2)),
     ("panels", lambda: lpgen.RefineryBase(1, seed=5).instance(1), lambda: lpgen.RefineryBase(3, seed=5).instance(3)),
-], ids=["one_cta", "cluster", "grid", "panels"])
+    ("grid_beside_panels", lambda: lpgen.planted(10_000, 25_000, 5, seed=2), lambda: lpgen.RefineryBase(3, seed=5).instance(3)),
+], ids=["one_cta", "cluster", "grid", "panels", "grid_beside_panels"])
 def test_contexts_of_two_threads(engine_lib, monkeypatch, form, small, large):
     """Contexts are independent of each other: two threads, each with its own context of another size, get the bits that
     they get one after the other."""
     monkeypatch.setenv("TARAL_TUNE", "0")
     if form == "grid":
         monkeypatch.setenv("TARAL_RESIDENT", "1")
-    if form == "panels":
+    if "panels" in form:
         monkeypatch.setenv("TARAL_PANELS", "1")
     lps = [small(), large()]
     alone = []
@@ -278,3 +279,78 @@ def test_forms_give_way_where_memory_is_short(engine_lib, monkeypatch, form, pre
                 assert np.array_equal(a, b)
     finally:
         pdhg.set_device_alloc_limit(0)
+
+
+def _band(rows, k, extra=0, seed=0):
+    """A square LP whose column j has the rows j .. j + k - 1, with `extra` empty rows and columns at the end."""
+    rng = np.random.default_rng(seed)
+    m = n = rows + k - 1 + extra
+    lens = np.where(np.arange(n) < rows, k, 0)
+    idx = np.concatenate([np.arange(j, j + k) for j in range(rows)]).astype(np.int32)
+    val, x = rng.standard_normal(idx.size), rng.uniform(0, 1, n)
+    b = np.zeros(m)
+    np.add.at(b, idx, val * np.repeat(x, lens))
+    return lpgen.LP(f"band_{rows}_{k}", m, n, np.concatenate([[0], np.cumsum(lens)]).astype(np.int64), idx, val, rng.standard_normal(n),
+                    np.zeros(n), np.full(n, 10.0), b, b.copy())
+
+
+def _column_limit():
+    """A band of 24 and, at its end, rows of 10 with columns of their own: more than 6,144 columns in one panel's nonzeros, so
+    that its rows are halved. Those columns lie where the plan does not look first."""
+    base, rows, per, at = _band(24_000, 24), 700, 10, 8200
+    rng = np.random.default_rng(5)
+    cut = base.col_ptr[at]
+    idx = np.concatenate([base.row_idx[:cut], np.repeat(base.m + np.arange(rows), per), base.row_idx[cut:]]).astype(np.int32)
+    val = np.concatenate([base.val[:cut], rng.uniform(0.5, 1.5, rows * per), base.val[cut:]])
+    ptr = np.concatenate([base.col_ptr[:at], cut + np.arange(rows * per), base.col_ptr[at:] + rows * per])
+    n, pad = base.n + rows * per, np.full(rows, 3.0)
+    return lpgen.LP("column_limit", base.m + rows, n, ptr.astype(np.int64), idx, val, rng.standard_normal(n), np.zeros(n), np.full(n, 10.0),
+                    np.concatenate([base.row_lo, pad]), np.concatenate([base.row_up, pad]))
+
+
+PANELS = {
+    "full_panels_of_1024_rows": lambda: _band(3000, 8),
+    "empty_rows": lambda: _band(2500, 12, extra=300),
+    "long_rows_only": lambda: _band(1500, 60),
+    "blocks": lambda: _blocks(6, 70, 90),
+    "column_limit": _column_limit,
+    "refinery": lambda: lpgen.RefineryBase(3, seed=5).instance(3, lpgen.perturbations(1, 3)[0]),
+}
+
+
+@pytest.mark.parametrize("precision", [pdhg.FP64, pdhg.FP32], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("case", sorted(PANELS))
+def test_panels_and_one_launch_evaluations(engine_lib, monkeypatch, case, precision):
+    """Panels as they run (with the one-launch evaluation) against a launch per phase on row blocks, both in the model's row
+    order: the same bits, also for points that are not finite."""
+    lp = PANELS[case]()
+    monkeypatch.setenv("TARAL_TUNE", "0")
+    monkeypatch.setenv("TARAL_ROWORDER", "0")
+    got, mem = [], []
+    for panels, resident in (("0", "0"), ("1", None)):
+        monkeypatch.setenv("TARAL_PANELS", panels)
+        if resident is None:
+            monkeypatch.delenv("TARAL_RESIDENT")
+        else:
+            monkeypatch.setenv("TARAL_RESIDENT", resident)
+        eng = pdhg.Engine.from_model(lp, precision=precision)
+        mem.append(eng.info()[1])
+        out = [np.array([eng.power_norm(40)])]
+        eng.set_steps(0.02, 0.03)
+        for x0 in (None, np.where(np.arange(lp.n) % 97 == 5, np.inf, 0.25), np.where(np.arange(lp.n) % 89 == 3, np.nan, -1.0)):
+            eng.start(x0, None if x0 is None else np.linspace(-1, 1, lp.m))
+            for steps in (64, 64, 3):
+                eng.iterate(steps)
+                out += list(eng.eval_pair(1.0 / steps))
+                eng.restart(steps == 64, 1.0 / steps)
+            out += [eng.eval(0, 1.0)] + [v for avg in (0, 1) for v in eng.download(avg, 0.5)]
+        got.append(out)
+        if resident is None:  # a launch per phase, so these are the panels
+            before = eng.device_launches
+            eng.iterate(5)
+            assert eng.device_launches - before == 11
+        eng.close()
+    size = 8 if precision == pdhg.FP64 else 4
+    assert mem[1] - mem[0] >= 2 * lp.nnz * (size + 2)  # both matrices' values and positions once more
+    for k, (a, b) in enumerate(zip(*got)):
+        assert np.array_equal(a, b, equal_nan=True), (k, a, b)
