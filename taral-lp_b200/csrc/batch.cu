@@ -782,7 +782,8 @@ struct Batch final : BatchBase {
             model_matrices(mk, sh.S.A, sh.S.AT, 1);
             if (panels_ok) {
                 sh.panels[0] = build_panels(sh.S.A.ptr.data(), sh.S.A.idx.data(), mk.m, mk.n, kPanelTarget, kBatchPanelCols, 1);
-                if (!sh.panels[0].empty()) sh.panels[1] = build_panels(sh.S.AT.ptr.data(), sh.S.AT.idx.data(), mk.n, mk.m, kPanelTarget, kBatchPanelCols, 1);
+                if (!sh.panels[0].empty())
+                    sh.panels[1] = build_panels(sh.S.AT.ptr.data(), sh.S.AT.idx.data(), mk.n, mk.m, kPanelTarget, kBatchPanelCols, 1);
                 if (sh.panels[1].empty()) panels_ok = false;
             }
             sh.S.m = mk.m, sh.S.n = mk.n, sh.nnz = int64_t(sh.S.A.idx.size());
@@ -1043,8 +1044,8 @@ struct Batch final : BatchBase {
     bool panels_allowed(const taral_model* md) const {
         const char* e = std::getenv("TARAL_PANELS");
         const char* pack = std::getenv("TARAL_BATCH_PACK");
-        if ((e && std::atoi(e) == 0) || (pack && std::atoi(pack) > 1) || pdl || std::getenv("TARAL_ROWSPLIT") || std::getenv("TARAL_ROWTHREAD"))
-            return false;
+        if ((e && std::atoi(e) == 0) || (pack && std::atoi(pack) > 1) || pdl) return false;
+        if (std::getenv("TARAL_ROWSPLIT") || std::getenv("TARAL_ROWTHREAD")) return false;
         if (e && std::atoi(e) > 0) return true;
         int dev, sms;
         BK(cudaGetDevice(&dev));
@@ -1140,15 +1141,17 @@ struct Batch final : BatchBase {
     void power_lists(const std::vector<int4>& t_ev, const std::vector<int4>& te_ev, const std::vector<int>& hcr) {
         std::vector<char> first_of(size_t(ninst), 0), pack_of(packs.size(), 0);
         for (int i : first_inst) first_of[size_t(i)] = 1, pack_of[size_t(where[size_t(i)].x)] = 1;
-        auto pick = [&](const std::vector<int4>& blk, const std::vector<int4>& ext, const std::vector<char>& keep, int4*& db, int4*& de) {
+        auto pick = [&](const std::vector<int4>& blk, const std::vector<int4>& ext, const std::vector<char>& keep, int4*& db,
+                        int4*& de) {
             std::vector<int4> b, e;
             for (size_t k = 0; k < blk.size(); ++k)
                 if (keep[size_t(ext[k].x)]) b.push_back(blk[k]), e.push_back(ext[k]);
             db = put(b), de = put(e);
             return int(b.size());
         };
-        pw_lists[0].n1 = pick(h_a1, h_ae1, first_of, pw_lists[0].blk1, pw_lists[0].ext1), pw_lists[0].np = pick(h_ap, h_ae, pack_of, pw_lists[0].blkp, pw_lists[0].extp);
-        pw_lists[1].n1 = pick(h_t1, h_te1, first_of, pw_lists[1].blk1, pw_lists[1].ext1), pw_lists[1].np = pick(h_tp, h_te, pack_of, pw_lists[1].blkp, pw_lists[1].extp);
+        PowerLists &a = pw_lists[0], &t = pw_lists[1];
+        a.n1 = pick(h_a1, h_ae1, first_of, a.blk1, a.ext1), a.np = pick(h_ap, h_ae, pack_of, a.blkp, a.extp);
+        t.n1 = pick(h_t1, h_te1, first_of, t.blk1, t.ext1), t.np = pick(h_tp, h_te, pack_of, t.blkp, t.extp);
         std::vector<int4> ev, eve, first;
         std::vector<int2> cols_of;
         std::vector<int> widths;
@@ -1158,7 +1161,8 @@ struct Batch final : BatchBase {
         for (int k = 0; k < distinct; ++k) {
             const int i = first_inst[size_t(k)];
             const int2 at = where[size_t(i)];
-            for (int b = hcr[size_t(at.x)]; b < hcr[size_t(at.x) + 1]; ++b) ev.push_back(t_ev[size_t(b)]), eve.push_back(te_ev[size_t(b)]);
+            for (int b = hcr[size_t(at.x)]; b < hcr[size_t(at.x) + 1]; ++b)
+                ev.push_back(t_ev[size_t(b)]), eve.push_back(te_ev[size_t(b)]);
             first.push_back(make_int4(at.x, at.y, i, 0)), range.push_back(int(ev.size()));
             cols_of.push_back(make_int2(packs[size_t(at.x)].cbase, mats[size_t(k)]->S.n));
             widths.push_back(packs[size_t(at.x)].W);
@@ -1169,7 +1173,8 @@ struct Batch final : BatchBase {
         int done = 0;
         for (const auto& q : by_n) nn = power_norm2(nn, done, q.first), done = q.first, norms[size_t(q.second)] = std::sqrt(nn);
         npw_ev = int(ev.size());
-        pw_ev = put(ev), pwe_ev = put(eve), pw_first = put(first), pw_range = put(range), pw_cols = put(cols_of), pw_width = put(widths), pw_norm = put(norms), pw_taken = alloc<int>(size_t(distinct));
+        pw_ev = put(ev), pwe_ev = put(eve), pw_first = put(first), pw_range = put(range);
+        pw_cols = put(cols_of), pw_width = put(widths), pw_norm = put(norms), pw_taken = alloc<int>(size_t(distinct));
     }
 
     // Small instances on one cluster each (cluster.cuh): where the waves of clusters that fit the GPU at the same time, at the
@@ -1197,9 +1202,9 @@ struct Batch final : BatchBase {
         BK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         if (mats[largest]->nnz > 65536) return;
         const bool near = 2 * mats[largest]->adjacent > mats[largest]->looked, fp32 = sizeof(T) == 4;
-        const double product = near ? (fp32 ? 2.8e-6 : 4.5e-6) : (fp32 ? 3.2e-6 : 7e-6), row = near ? (fp32 ? 4e-6 : 9e-6) : (fp32 ? 8e-6 : 1e-5);
-        const double phases = ((nnz_total > 32 * int64_t(std::max(M, N)) ? 9 : 7) + product * double(nnz_total) + row * (double(M) + double(N))) *
-                              (npanels[0] ? 0.6 : 1.0);
+        const double product = near ? (fp32 ? 2.8e-6 : 4.5e-6) : (fp32 ? 3.2e-6 : 7e-6);
+        const double row = near ? (fp32 ? 4e-6 : 9e-6) : (fp32 ? 8e-6 : 1e-5), base = nnz_total > 32 * int64_t(std::max(M, N)) ? 9 : 7;
+        const double phases = (base + product * double(nnz_total) + row * (double(M) + double(N))) * (npanels[0] ? 0.6 : 1.0);
         for (int q = cluster_size(mats[largest]->nnz); q <= 8; q *= 2) {
             auto pays = [&](double us, int at_once) {
                 const double waves = double(ninst) / at_once;
@@ -1235,7 +1240,8 @@ struct Batch final : BatchBase {
             int* d_plan = nullptr;
             if (!if_memory([&] {
                     d_plan = put(all);
-                    d_lps = alloc<ClusterLp<T>>(size_t(ninst)), d_first_lps = alloc<ClusterLp<T>>(mats.size()), d_norms = alloc<double>(2 * mats.size());
+                    d_lps = alloc<ClusterLp<T>>(size_t(ninst)), d_first_lps = alloc<ClusterLp<T>>(mats.size());
+                    d_norms = alloc<double>(2 * mats.size());
                 }))
                 return;
             std::vector<ClusterLp<T>> lps, firsts;
@@ -1480,7 +1486,8 @@ struct Batch final : BatchBase {
 
     void block(int steps) {
         if (cluster_ctas > 0) {
-            BK(launch_cluster(k_cluster_iterate<T, true>, k_cluster_iterate<T, false>, d_lps, ninst, cluster_ctas, cluster_smem, s, steps));
+            BK(launch_cluster(k_cluster_iterate<T, true>, k_cluster_iterate<T, false>, d_lps, ninst, cluster_ctas, cluster_smem, s,
+                              steps));
             ++launches;
         } else {
             if (nT) k_pack_xupd<T><<<nT, kThreads, 0, s>>>(T_ev, Te_ev, slot_inst, running, x, ATz, c, l, u, par, xs), ++launches;
@@ -1514,12 +1521,14 @@ struct Batch final : BatchBase {
             for (int k = 0; k < chunk; ++k) {
                 power_spmv(0, a, pw), power_spmv(1, pw, b);
                 const bool single = packs.size() == size_t(ninst);  // one slot each
-                if (npw_ev && single) k_warp_pow_part<T><<<(npw_ev + 7) / 8, kThreads, 0, s>>>(npw_ev, pw_ev, pwe_ev, slot_inst, pactive, b, partT);
+                if (npw_ev && single)
+                    k_warp_pow_part<T><<<(npw_ev + 7) / 8, kThreads, 0, s>>>(npw_ev, pw_ev, pwe_ev, slot_inst, pactive, b, partT);
                 else if (npw_ev) k_pack_pow_part<T><<<npw_ev, kThreads, 0, s>>>(pw_ev, pwe_ev, slot_inst, pactive, b, partT);
                 k_pow_update<<<distinct, kFinishThreads, 0, s>>>(pw_first, pw_range, partT, est, pscale, pactive, pw_taken);
                 if (npanels[0]) --launches;  // panels scale the vector as they gather it
                 else if (npw_ev && single)
-                    k_flat_pow_scale<T><<<matrix_ctas() * distinct, kThreads, 0, s>>>(pw_first, pw_cols, pactive, pscale, b, matrix_ctas());
+                    k_flat_pow_scale<T><<<matrix_ctas() * distinct, kThreads, 0, s>>>(pw_first, pw_cols, pactive, pscale, b,
+                                                                                       matrix_ctas());
                 else if (npw_ev) k_pack_pow_scale<T><<<npw_ev, kThreads, 0, s>>>(pw_ev, pwe_ev, slot_inst, pactive, pscale, b);
                 launches += 3;
                 std::swap(a, b);
@@ -1553,7 +1562,8 @@ struct Batch final : BatchBase {
         if (npanels[0]) {
             const auto* work = (const PanelWork<1>*)panel_first[phase];
             if (phase == 0)
-                BK(launch_panels(panels[0], npanels[0], panel_most[0], xin, work, (const int*)pactive, PanelScaled<T>{{y}, pscale}, s));
+                BK(launch_panels(panels[0], npanels[0], panel_most[0], xin, work, (const int*)pactive,
+                                 PanelScaled<T>{{y}, pscale}, s));
             else
                 BK(launch_panels(panels[1], npanels[1], panel_most[1], xin, work, (const int*)pactive, PanelStore<T>{y}, s));
             ++launches;
@@ -1563,8 +1573,11 @@ struct Batch final : BatchBase {
         const int *ptr = phase ? Tptr : Aptr, *idx = phase ? Tidx : Aidx;
         const T* val = phase ? Tval : Aval;
         const EpiStore<T> e{y};
-        if (q.n1) launch(k_rowblock_batch<T, T, EpiStore<T>, true>, q.n1, false, ptr, idx, val, xin, (const int4*)q.blk1, (const int4*)q.ext1, (const int*)pactive, e);
-        if (q.np) k_pack_spmv<T, T, EpiStore<T>><<<q.np, kThreads, 0, s>>>(ptr, idx, val, xin, q.blkp, q.extp, slot_inst, pactive, e), ++launches;
+        if (q.n1)
+            launch(k_rowblock_batch<T, T, EpiStore<T>, true>, q.n1, false, ptr, idx, val, xin, (const int4*)q.blk1,
+                   (const int4*)q.ext1, (const int*)pactive, e);
+        if (q.np)
+            k_pack_spmv<T, T, EpiStore<T>><<<q.np, kThreads, 0, s>>>(ptr, idx, val, xin, q.blkp, q.extp, slot_inst, pactive, e), ++launches;
     }
 
     void cancel() override {
@@ -1580,7 +1593,8 @@ struct Batch final : BatchBase {
         BK(cudaEventCreate(&e1));
         BK(cudaEventRecord(e0, s));
         // power iteration per instance (gpu/pdhg.cu:416-436)
-        k_power_starts<T><<<matrix_ctas() * distinct, 256, 0, s>>>(pw_first, pw_cols, pw_width, pw_norm, pv, pscale, matrix_ctas());
+        k_power_starts<T><<<matrix_ctas() * distinct, 256, 0, s>>>(pw_first, pw_cols, pw_width, pw_norm, pv, pscale,
+                                                                   matrix_ctas());
         BK(cudaGetLastError());
         ++launches;
         // One estimate per distinct matrix: instances that share a matrix share its scaled copy, its row blocks and
@@ -1594,7 +1608,8 @@ struct Batch final : BatchBase {
         const int g = (ninst + 255) / 256;
         std::vector<double> norms(ninst);
         if (cluster_ctas > 0) {
-            BK(launch_cluster(k_cluster_power<T, true>, k_cluster_power<T, false>, d_first_lps, distinct, cluster_ctas, cluster_smem, s, 200, d_norms));
+            BK(launch_cluster(k_cluster_power<T, true>, k_cluster_power<T, false>, d_first_lps, distinct, cluster_ctas, cluster_smem,
+                              s, 200, d_norms));
             std::vector<double> got(2 * size_t(distinct));
             BK(cudaMemcpyAsync(got.data(), d_norms, got.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
             BK(cudaStreamSynchronize(s));

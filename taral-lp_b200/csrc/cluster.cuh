@@ -229,7 +229,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster_iterate(const Cl
     for (int s = 0; s < steps; ++s) {
         slice_phase(A, [&](int k) { return x[k]; }, [&](int t, double sum) {
             const T st = T(sum);
-            const T zn = T(dual_prox(double(zo[t]) + sigma * (2.0 * double(st) - double(rs.a[t])), double(rs.b[t]), double(rs.c[t]), sigma, inv_sigma));
+            const double v = double(zo[t]) + sigma * (2.0 * double(st) - double(rs.a[t]));
+            const T zn = T(dual_prox(v, double(rs.b[t]), double(rs.c[t]), sigma, inv_sigma));
             store_all<MANY>(zo + t, zn, ctas);
             rs.a[t] = st, rs.sum[t] += double(zn);
         });
@@ -404,10 +405,12 @@ inline int cluster_size(int64_t nnz) {
     return c;
 }
 
-// Clusters of `ctas` CTAs with `smem` bytes each that the device runs at the same time (14 or 15 of 8 CTAs on 148 SMs, 30 to 33 of 4).
+// Clusters of `ctas` CTAs with `smem` bytes each that the device runs at the same time (on 148 SMs 14 or 15 of 8 CTAs, 30
+// to 33 of 4).
 template <class T>
 cudaError_t clusters_at_once(int ctas, size_t smem, int* count) {
-    const void* kernel = ctas > 1 ? reinterpret_cast<const void*>(&k_cluster_iterate<T, true>) : reinterpret_cast<const void*>(&k_cluster_iterate<T, false>);
+    const void* kernel = ctas > 1 ? reinterpret_cast<const void*>(&k_cluster_iterate<T, true>)
+                                  : reinterpret_cast<const void*>(&k_cluster_iterate<T, false>);
     const cudaError_t e = allow_launches(kernel, kClusterSmem, ctas > 1);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};

@@ -8,7 +8,10 @@
 //   eval   tmp_n f64[n], tmp_m f64[m] (products of the sums), partials, tickets, 20 result doubles
 // How a block of iterations runs: on one thread-block cluster with the whole LP in shared memory (cluster.cuh), in one
 // cooperative launch with a tile of A and A^T per team (resident.cuh), or a launch per phase, on panels (panels.cuh) where
-// rows share columns and on row blocks elsewhere. All give the same bits; choose_resident and plan_panels have the rules.
+// rows share columns and on row blocks elsewhere; choose_resident and plan_panels have the rules. On the default row split
+// and in one row order all give the same bits. Panels keep the model's row order, and the one-launch evaluation and power
+// iteration the default split: against a context that sorted its rows, or one that tuned another split (FP32), FP64 sums
+// run in another order.
 // The running sums of A x and A^T z that the reference keeps (gpu/pdhg.cu:188, :200) are not stored: the
 // average's products are formed once per evaluation as A xs and A^T zs, which saves 16 bytes of state traffic
 // per row and per column every iteration.
@@ -129,7 +132,7 @@ int forced_row_split() {
 template <class I>
 static int block_end(const I* ptr, int rows, int r, int tile, int rows_max) {
     const int last = int(std::min<int64_t>(rows, int64_t(r) + rows_max));
-    const I* e = std::upper_bound(ptr + r + 1, ptr + last + 1, I(ptr[r] + tile)) - 1;
+    const I* e = std::upper_bound(ptr + r + 1, ptr + last + 1, int64_t(ptr[r]) + tile) - 1;
     return std::max(r + 1, int(e - ptr));
 }
 template <class I>
@@ -707,7 +710,8 @@ struct Engine final : EngineBase {
         // 42.6; 1,800 55.9 / 56.6, 71.6 / 63.4; 2,450 power-law 63.7 / 89.2, 77.7 / 93.8; 3,906 80 / 100, 100 / 105; one row of
         // 20,000 nonzeros 20.7 / 22.0, 22.0 / 20.7, of 100,000 57.6 / 81.6, 58.9 / 75.4.
         const int tiles = std::max(A.rnblk, AT.rnblk), per_team = sizeof(T) == 4 ? 2 : 8;
-        resident_powers = npanels[0] == 0 && ((tiles <= per_team * kTeams * sms && std::max(A.maxrow, AT.maxrow) <= 16 * kTile) || mode >= 1);
+        const bool faster = tiles <= per_team * kTeams * sms && std::max(A.maxrow, AT.maxrow) <= 16 * kTile;
+        resident_powers = npanels[0] == 0 && (faster || mode >= 1);
         // the tuner's choice for the phases, or panels
         if (A.per_thread || AT.per_thread || tuned[0] == 2 || tuned[1] == 2 || npanels[0]) return;
         resident_iterates = mode >= 1 || std::max(A.rnblk, AT.rnblk) <= kTeams * sms;
@@ -770,7 +774,8 @@ struct Engine final : EngineBase {
     // `per_team`, `least`: bytes of shared memory per team and at least. The barrier counters alternate: a launch counts
     // on one, which the launch before it has zeroed, and zeroes the other.
     template <class... P, class... Args>
-    void launch_resident(void (*kernel)(const ResidentArgs<T>, P...), size_t per_team, size_t least, ResidentArgs<T> ra, Args... args) {
+    void launch_resident(void (*kernel)(const ResidentArgs<T>, P...), size_t per_team, size_t least, ResidentArgs<T> ra,
+                         Args... args) {
         ra.bar = rbar + rparity * (kBarrierStride / 2), ra.other_bar = rbar + (1 - rparity) * (kBarrierStride / 2);
         rparity = 1 - rparity;
         const int blocks = std::max(A.rnblk, AT.rnblk);
@@ -817,7 +822,8 @@ struct Engine final : EngineBase {
         CK(cudaMemsetAsync(pdone, 0, sizeof(int), st));
         launches += 1;
         if (cluster_ctas > 0) {
-            CK(launch_cluster(k_cluster_power<T, true>, k_cluster_power<T, false>, d_lp, 1, cluster_ctas, cluster_smem, st, iters, h_out));
+            CK(launch_cluster(k_cluster_power<T, true>, k_cluster_power<T, false>, d_lp, 1, cluster_ctas, cluster_smem, st, iters,
+                              h_out));
             CK(cudaStreamSynchronize(st));
             launches += 2 * int64_t(h_out[1]), folded += 2 * int64_t(h_out[1]) - 1;
             return h_out[0];
@@ -837,7 +843,8 @@ struct Engine final : EngineBase {
         auto step = [&] {
             if (npanels[0]) {  // these scale the vector as they gather it
                 const PanelWork<1>* whole = nullptr;
-                CK(launch_panels(panels[0], npanels[0], panel_most[0], (const T*)a, whole, nullptr, PanelScaled<T>{{pw}, pst + 2}, st));
+                CK(launch_panels(panels[0], npanels[0], panel_most[0], (const T*)a, whole, nullptr,
+                                 PanelScaled<T>{{pw}, pst + 2}, st));
                 ++launches;
             } else {
                 spmv(A, a, pw, pdone);
@@ -917,7 +924,8 @@ struct Engine final : EngineBase {
         check_point();
         if (steps <= 0) return;
         if (cluster_ctas > 0) {
-            CK(launch_cluster(k_cluster_iterate<T, true>, k_cluster_iterate<T, false>, d_lp, 1, cluster_ctas, cluster_smem, st, steps));
+            CK(launch_cluster(k_cluster_iterate<T, true>, k_cluster_iterate<T, false>, d_lp, 1, cluster_ctas, cluster_smem, st,
+                              steps));
             launches += 1 + 2 * int64_t(steps), folded += 2 * int64_t(steps);
         } else if (resident_iterates) {
             launch_resident(k_resident_iterate<T>, sizeof(RowSmem<T>), 0,
@@ -971,8 +979,8 @@ struct Engine final : EngineBase {
     void eval_pair(double f, double* cur, double* avg) override {
         check_point();
         if (resident_ctas > 0) {  // the scalars go straight to the pinned status block
-            launch_resident(k_resident_eval<T>,
-                            sizeof(RowSmem<double>), 20 * kEvalCtas * sizeof(double), resident_args(h_out), f, red_grid(m), red_grid(n));
+            launch_resident(k_resident_eval<T>, sizeof(RowSmem<double>), 20 * kEvalCtas * sizeof(double), resident_args(h_out), f,
+                            red_grid(m), red_grid(n));
             launches += 6, folded += 5;
         } else {
             queue_eval(false, 1.0, out);

@@ -481,7 +481,8 @@ struct Mlp {
     void backward(int batch, const float* T, const int* idx, const AdamStep* step) {
         auto bias = [&](Layer& y) { return step ? BiasStep{y.b, y.mb, y.vb, *step} : BiasStep{}; };
         Layer& top = L[depth];
-        k_loss_grad<<<loss_ctas(), 256, column_smem(batch, kLossCols), s>>>(batch, top.out, ldy, top.Z, T, idx, dYb, top.gb, bias(top), part);
+        k_loss_grad<<<loss_ctas(), 256, column_smem(batch, kLossCols), s>>>(batch, top.out, ldy, top.Z, T, idx, dYb, top.gb,
+                                                                            bias(top), part);
         const bf16* dZ = dYb;
         int ldz = ldy;  // row stride of dZ
         for (int l = depth; l >= 0; --l) {
@@ -504,7 +505,8 @@ struct Mlp {
                     gemm<false, true>(batch, y.in, y.out, dZ, y.Wb, C, std::max(1, std::min(64, y.out / 2048)));
                     slices = 1, partials = C;
                 }
-                k_hidden_grad<<<(p.out + kHiddenCols - 1) / kHiddenCols, 1024, column_smem(batch, kHiddenCols), s>>>(batch, p.out, slices, partials, p.Z, next, p.gb, bias(p));
+                k_hidden_grad<<<(p.out + kHiddenCols - 1) / kHiddenCols, 1024, column_smem(batch, kHiddenCols), s>>>(
+                    batch, p.out, slices, partials, p.Z, next, p.gb, bias(p));
             }
             if (y.fused && step) {
                 tc_check(taral::tc::gemm_adam(y.in, y.out, batch, Hprev, y.in, dZ, ldz, y.W, y.mW, y.vW, y.Wb, y.ldw, *step, d_err, s));

@@ -442,7 +442,9 @@ template <class E>
 static int launch_gemm(int M, int N, int K, const void* A, int lda, int a_mn, const void* B, int ldb, int b_mn, const E& epi,
                        int* slices, int* err, cudaStream_t stream) {
     const int64_t items = int64_t((M + TM - 1) / TM) * ((N + 255) / 256) * (*slices < 1 ? 1 : *slices);
-    if (items <= 37) return launch_tiles<E, 64>(M, N, K, A, lda, a_mn, B, ldb, b_mn, epi, slices, err, stream);
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (items <= sms / 4) return launch_tiles<E, 64>(M, N, K, A, lda, a_mn, B, ldb, b_mn, epi, slices, err, stream);
     return launch_tiles<E, 256 / E::kCtas>(M, N, K, A, lda, a_mn, B, ldb, b_mn, epi, slices, err, stream);
 }
 

@@ -154,9 +154,9 @@ struct LongRows {
 // One CTA per panel (work NULL: panel blockIdx.x, one instance) or per work item. A panel's latency is what a phase of a
 // single LP takes, so every load that does not need the gathered entries is issued before the copy of those is waited for:
 // the first long rows of each warp here, and in the loop the next ones before the current are summed. (More rows in
-// flight per warp spill, and ranges prefetched into L2 compete with the loads: 10% slower each.) The lists and the first long
-// rows are read while the phase before ends (launch_early; what that phase writes is then read past L1 or by plain loads): a refinery LP of 3.4M nonzeros takes 26.1 us an iteration in FP64
-// instead of 27.3, in FP32 18.0 instead of 19.8.
+// flight per warp spill, and ranges prefetched into L2 compete with the loads: 10% slower each.) The lists and the first
+// long rows are read while the phase before ends (launch_early; what that phase writes is then read past L1 or by plain
+// loads): a refinery LP of 3.4M nonzeros takes 26.1 us an iteration in FP64 instead of 27.3, in FP32 18.0 instead of 19.8.
 template <class T, class X, int W, class E>
 __global__ void __launch_bounds__(kPanelThreads, 2) k_panel(const PanelMat<T> a, const X* __restrict__ xin,
                                                             const PanelWork<W>* __restrict__ work,

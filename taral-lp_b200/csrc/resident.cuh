@@ -9,7 +9,8 @@
 // step are left.
 //
 //   team   -- 256 threads, one row block (tile) of the block list at a time, exactly as a CTA of k_rowblock takes
-//             it: the same products, the same summation order per row, hence the same iterates bit for bit;
+//             it on the default row split: the same products, the same summation order per row, hence the same iterates
+//             bit for bit (blocks that a context tuned to kMidGroups or kSegmented are summed by the default rule here);
 //   CTA    -- kTeams teams, one CTA per SM (its teams share the CTA's arrival at the barrier);
 //   grid   -- a cooperative launch, so that every CTA is resident while others wait for it at the barrier, a counter
 //             in global memory.
@@ -132,7 +133,8 @@ __device__ __forceinline__ void load_rows(const ResidentMat<T>& a, int4 meta, co
 // row longer than a tile by the whole team. `in(k)`: entry k of the gathered vector. Every thread of the team calls
 // it; the result is meaningful where tid < rows.
 template <class P, class T, class In>
-__device__ __forceinline__ double tile_sum(const ResidentMat<T>& a, const Tile<T>& q, const Team& t, RowSmem<P>& sm, const int* rptr, In in) {
+__device__ __forceinline__ double tile_sum(const ResidentMat<T>& a, const Tile<T>& q, const Team& t, RowSmem<P>& sm,
+                                           const int* rptr, In in) {
     const int tid = t.tid, lane = tid & 31, warp = tid >> 5;
     const int nrows = q.meta.y & 0xffff, p0 = q.meta.z, p1 = q.meta.w;
     if (p1 - p0 > kTile) {
@@ -239,7 +241,8 @@ __device__ __forceinline__ FirstTile first_tile(const ResidentMat<T>& a, const T
 // One phase: every tile of the matrix with the fused step `epi`, gathering through `in`. Called after arrive(); the
 // first tile's entries and operands are loaded before the wait.
 template <class P, class T, class E, class In>
-__device__ __forceinline__ bool phase(GridBarrier& barrier, const ResidentMat<T>& a, const FirstTile& f, const Team& t, RowSmem<P>& sm, const E& epi, In in) {
+__device__ __forceinline__ bool phase(GridBarrier& barrier, const ResidentMat<T>& a, const FirstTile& f, const Team& t,
+                                      RowSmem<P>& sm, const E& epi, In in) {
     const int first = t.id * int(gridDim.x) + int(blockIdx.x), teams = int(gridDim.x) * (int(blockDim.x) / kThreads);
     Tile<T> q;
     typename E::Ops ops{};

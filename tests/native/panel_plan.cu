@@ -8,8 +8,8 @@ using namespace taral;
 
 // y = A x by the plan; sizes: panels, most columns, rows and long rows of a panel, columns listed, entries stored.
 // Returns 0 without panels, -1 where the plan is not one of this matrix, else 1.
-extern "C" int panel_product(int rows, int cols, const int64_t* ptr, const int32_t* idx, const double* val, const double* x, int target,
-                             int max_cols, int threads, int64_t allocs, double* y, int64_t* sizes) {
+extern "C" int panel_product(int rows, int cols, const int64_t* ptr, const int32_t* idx, const double* val, const double* x,
+                             int target, int max_cols, int threads, int64_t allocs, double* y, int64_t* sizes) {
     fail_allocations_after(allocs);
     const PanelPlan p = build_panels(ptr, idx, rows, cols, target, max_cols, threads);
     fail_allocations_after(-1);
@@ -20,7 +20,8 @@ extern "C" int panel_product(int rows, int cols, const int64_t* ptr, const int32
     for (const Panel& h : p.panels) {
         if (h.row0 != next || h.rows < 1 || h.rows > kPanelRows || h.cols > max_cols) return -1;
         next += h.rows;
-        most[0] = std::max<int64_t>(most[0], h.cols), most[1] = std::max<int64_t>(most[1], h.rows), most[2] = std::max<int64_t>(most[2], h.nlong);
+        const int size[3] = {h.cols, h.rows, h.nlong};
+        for (int k = 0; k < 3; ++k) most[k] = std::max<int64_t>(most[k], size[k]);
         const int* list = p.cols.data() + h.col0;
         for (int i = 1; i < h.cols; ++i)
             if (list[i - 1] >= list[i]) return -1;
@@ -38,7 +39,8 @@ extern "C" int panel_product(int rows, int cols, const int64_t* ptr, const int32
         };
         for (int q = 0; q < h.nlong; ++q) {
             const int4 r = p.longrow[size_t(h.long0 + q)];
-            if (r.y <= kShort || r.x < 0 || r.x + r.y > p.long_entries || r.y != ptr[h.row0 + r.z + 1] - ptr[h.row0 + r.z]) return -1;
+            if (r.y <= kShort || r.x < 0 || r.x + r.y > p.long_entries) return -1;
+            if (r.y != ptr[h.row0 + r.z + 1] - ptr[h.row0 + r.z]) return -1;
             if (!sum(r.z, r.y)) return -1;
         }
         for (int s = 0; s < h.slices; ++s) {
@@ -52,7 +54,8 @@ extern "C" int panel_product(int rows, int cols, const int64_t* ptr, const int32
         }
     }
     if (next != rows) return -1;
-    if (most[0] != p.most.cols || most[1] != p.most.rows || most[2] != p.most.nlong || int64_t(p.cols.size()) != p.listed) return -1;
+    if (most[0] != p.most.cols || most[1] != p.most.rows || most[2] != p.most.nlong) return -1;
+    if (int64_t(p.cols.size()) != p.listed) return -1;
     const int64_t out[6] = {int64_t(p.panels.size()), most[0], most[1], most[2], p.listed, p.padded};
     std::copy(out, out + 6, sizes);
     return 1;
