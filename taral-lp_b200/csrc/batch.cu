@@ -1026,11 +1026,13 @@ struct Batch final : BatchBase {
     // refinery scenarios of 12 matrices (22.6M products a phase, FP32) a row phase takes 42 us (row blocks 72), a column
     // phase 33 (55). TARAL_PANELS=0: none, 1: at any size (tests).
     //
-    // Only where the CTAs whose slots are all used fill the SMs (FP64: two thirds of them), and rows of at least 8 (see
-    // panels_suit). Measured, us an iteration with row blocks / panels by those CTAs: refinery scenarios FP32 69: 45.5 /
-    // 57.3, 92: 56.3 / 59.9, 104: 63.6 / 61.9, 112: 72.1 / 78.9, 168: 101 / 88, 184: 103 / 69, 207: 115 / 73; FP64 69: 44.3 /
-    // 49.3, 92: 48.9 / 49.7, 104: 59 / 50, 112: 70 / 69, 138: 71 / 53; bands of 8 FP32 78: 23 / 30, 156: 36.6 / 35.0; bands of 6
-    // FP32 320: 50.7 / 61.4, FP64 640: 66.5 / 78.0.
+    // Only where enough CTAs, counted by their used slots, are at work: two thirds of the SMs, or, where the distinct matrices
+    // alone have panels for half of them (the power iteration's), 0.55 (FP64 0.4); and rows of at least 8 (see panels_suit).
+    // Measured, us an iteration with row blocks / panels by those CTAs, refinery scenarios: of one matrix FP32 69: 45.5 / 57.3,
+    // 92: 56.3 / 59.9, 104: 63.6 / 61.9, 184: 103 / 69, 207: 115 / 73; FP64 69: 44.3 / 49.3, 92: 48.9 / 49.7, 104: 59 / 50, 138: 71 /
+    // 53; of 8 to 12 matrices FP32 56: 44.9 / 70.2, 83: 67 / 67 (a power step 39 / 30), 104: 77 / 69, 112: 72 / 79, 130: 92 / 77,
+    // 168: 101 / 88; FP64 65: 55.9 / 55.7 (57 / 45), 112: 70 / 69. Bands of 8 FP32 78: 23 / 30, 156: 36.6 / 35.0; bands of 6 FP32
+    // 320: 50.7 / 61.4, FP64 640: 66.5 / 78.0.
     static constexpr int kPW = sizeof(T) == 4 ? 4 : 2;
     static constexpr int kPanelTarget = 24576, kBatchPanelCols = 4096;
     PanelMat<T> panels[2];
@@ -1050,16 +1052,19 @@ struct Batch final : BatchBase {
         int dev, sms;
         BK(cudaGetDevice(&dev));
         BK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        double ctas[2] = {0, 0}, rows[2] = {0, 0}, nnz = 0;
+        double ctas[2] = {0, 0}, own[2] = {0, 0}, rows[2] = {0, 0}, nnz = 0;  // own: panels of the distinct matrices
         for (int i = 0; i < ninst; ++i) {
             const double size[2] = {double(md[i].m), double(md[i].n)}, entries = double(md[i].col_ptr[md[i].n]);
             for (int k = 0; k < 2; ++k) {
-                ctas[k] += std::max(size[k] / kPanelRows, entries / kPanelTarget) / kPW;
+                const double panels = std::max(size[k] / kPanelRows, entries / kPanelTarget);
+                ctas[k] += panels / kPW;
+                if (first_inst[size_t(mat_of[size_t(i)])] == i) own[k] += panels;
                 rows[k] += size[k];
             }
             nnz += entries;
         }
-        return std::min(ctas[0], ctas[1]) >= (sizeof(T) == 4 ? 1.0 : 2.0 / 3) * sms && nnz >= 8 * std::max(rows[0], rows[1]);
+        const double least = std::min(own[0], own[1]) < 0.5 * sms ? 2.0 / 3 : sizeof(T) == 4 ? 0.55 : 0.4;
+        return std::min(ctas[0], ctas[1]) >= least * sms && nnz >= 8 * std::max(rows[0], rows[1]);
     }
     void put_panels() {  // the plans of all matrices one after another, filled from the scaled values
         for (const auto& sh : mats)
@@ -1181,7 +1186,7 @@ struct Batch final : BatchBase {
     // plan's estimate for the slowest matrix, take less than the phase kernels. Those are estimated at 7 us (9 with rows of
     // more than 32 on average) + a us a million products + b us a million rows and columns, where neighbouring entries are
     // neighbours in memory (a 2.8, b 4; FP64 4.5, 9) or not (3.2, 8; 7, 10), on panels 0.6 times that. Beyond 3 waves the phase
-    // kernels fill the GPU: a margin of 0.8 there (FP64 0.85, one CTA 0.95), 0.9 before. Measured, FP32 and FP64, us an
+    // kernels fill the GPU: a margin of 0.8 there (FP64 0.85, one CTA 0.95), 0.92 before. Measured, FP32 and FP64, us an
     // iteration with phases / clusters: 40 of 150 x 350 7.5 / 1.4, 7.5 / 1.3; 400 of them 9.7 / 4.2, 12.1 / 3.8; 100 of 700 x 1,633
     // 10.2 / 9.0, 12.0 / 9.2; 200 14.0 / 15.8, 17.4 / 16.0; 40 of 1,500 x 3,500 9.7 / 8.2, 11.2 / 9.0; 100 15.6 / 18.8, 19.0 / 20.9;
     // 200 bands of 8 (1,000 rows) 11.7 / 13.8, 17.1 / 14.3; 16 of dense 200 x 200 9.4 / 7.7, 10.3 / 7.4; 100 11.9 / 27.0, 25.5 /
@@ -1208,7 +1213,7 @@ struct Batch final : BatchBase {
         for (int q = cluster_size(mats[largest]->nnz); q <= 8; q *= 2) {
             auto pays = [&](double us, int at_once) {
                 const double waves = double(ninst) / at_once;
-                const double margin = q == 1 ? 0.95 : waves <= 3 ? 0.9 : fp32 ? 0.8 : 0.85;
+                const double margin = q == 1 ? 0.95 : waves <= 3 ? 0.92 : fp32 ? 0.8 : 0.85;
                 return waves <= 8 && (waves <= 3 ? std::ceil(waves) : waves) * us <= margin * phases;
             };
             if (!pays(q > 1 ? 1.9 : 1.0, std::max(1, sms / q))) return;  // the least that a plan comes to

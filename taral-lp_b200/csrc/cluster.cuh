@@ -333,16 +333,18 @@ constexpr size_t kClusterSmem = 224 * 1024;  // dynamic shared memory a CTA may 
 // contiguous ranges of about equal cost (nonzeros plus 4 per row, the weight of a row's step). Returns the largest
 // CTA's shared memory; offsets in the headers count from the plan's start.
 //
-// *us: what an iteration takes. A phase lasts as long as the warp with the most work: 0.37 us a group of 32 short rows, 0.02
-// a step of its longest row, 0.59 a long row (a shuffle tree in FP64, and one lane's fused step), 0.12 its stride of 128;
-// several CTAs add 0.6 us of barriers and 0.028 us a KB of x and z, which every SM takes in. Within 15 % of the time
-// measured on 40 LPs of 360 to 120,000 nonzeros, FP32 and FP64, all but two of them (1,000 short rows beside 30 long ones).
+// *us: what an iteration takes. A phase lasts as long as the warp with the most work; in us, FP32 (FP64): 0.33 (0.40) a
+// group of 32 short rows, 0.027 (0.014) a step of its longest row, 0.63 (0.64) a long row (a shuffle tree in FP64, and one
+// lane's fused step), 0.12 (0.075) its stride of 128. Several CTAs add 0.56 of barriers and 0.037 (0.028) a KB of x and z,
+// which every SM takes in. Within 20 % of the time measured on 70 LPs of 360 to 60,000 nonzeros.
 template <class T>
 size_t cluster_plan(const int* a_ptr, const int* t_ptr, int m, int n, int ctas, std::vector<int>& plan, double* us) {
     constexpr int kHeader = int(sizeof(ClusterCta) / sizeof(int));
     std::vector<ClusterCta> head(static_cast<size_t>(ctas));
     plan.assign(size_t(ctas) * kHeader, 0);
-    *us = ctas > 1 ? 0.6 + 0.028e-3 * double(size_t(m + n) * sizeof(T)) : 0;
+    constexpr bool fp32 = sizeof(T) == 4;
+    constexpr double group = fp32 ? 0.33 : 0.40, step = fp32 ? 0.027 : 0.014, long_row = fp32 ? 0.63 : 0.64, stride = fp32 ? 0.12 : 0.075;
+    *us = ctas > 1 ? 0.56 + (fp32 ? 0.037e-3 : 0.028e-3) * double(size_t(m + n) * sizeof(T)) : 0;
     for (int k = 0; k < 2; ++k) {
         const int *ptr = k ? t_ptr : a_ptr, rows = k ? n : m;
         const double all = double(ptr[rows] - ptr[0]) + 4.0 * rows;
@@ -365,13 +367,13 @@ size_t cluster_plan(const int* a_ptr, const int* t_ptr, int m, int n, int ctas, 
             int at = 0;
             for (int t = nlong; t < h.rows[k]; t += 32) {
                 base.push_back(at), at += 32 * len(first[t]);
-                warp[(t - nlong) / 32 % (kClusterThreads / 32)] += 0.37 + 0.02 * ((len(first[t]) + 3) / 4 * 4);
+                warp[(t - nlong) / 32 % (kClusterThreads / 32)] += group + step * ((len(first[t]) + 3) / 4 * 4);
             }
             base.push_back(at);  // the last group's end, and the first long row
             for (int t = 0; t < nlong; ++t) {
                 if (t) base.push_back(at);
                 at += len(first[t]);
-                warp[t % (kClusterThreads / 32)] += 0.59 + 0.12 * ((len(first[t]) + 127) / 128);
+                warp[t % (kClusterThreads / 32)] += long_row + stride * ((len(first[t]) + 127) / 128);
             }
             phase = std::max(phase, *std::max_element(warp, warp + kClusterThreads / 32));
             h.entries[k] = at, h.base[k] = int(plan.size());

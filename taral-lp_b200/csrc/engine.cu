@@ -705,21 +705,24 @@ struct Engine final : EngineBase {
         resident_ctas = std::min(sms, std::max(A.rnblk, AT.rnblk));
         cluster_ctas = 0;
         // The power iteration: 4 grid barriers a step against 4 launches, but 2 teams an SM where the phases have 5 to 8
-        // CTAs; a row of many tiles is one team's work. Measured (us a step, phases / resident): 528 tiles FP32 25.0 / 21.6,
-        // FP64 29.4 / 24.0; 735 29.1 / 28.2, 33.7 / 30.8; 980 planted 35.8 / 35.5, 45.9 / 40.2, power-law 35.1 / 41.2, 44.4 /
-        // 42.6; 1,800 55.9 / 56.6, 71.6 / 63.4; 2,450 power-law 63.7 / 89.2, 77.7 / 93.8; 3,906 80 / 100, 100 / 105; one row of
-        // 20,000 nonzeros 20.7 / 22.0, 22.0 / 20.7, of 100,000 57.6 / 81.6, 58.9 / 75.4.
-        const int tiles = std::max(A.rnblk, AT.rnblk), per_team = sizeof(T) == 4 ? 2 : 8;
-        const bool faster = tiles <= per_team * kTeams * sms && std::max(A.maxrow, AT.maxrow) <= 16 * kTile;
+        // CTAs; a row of many tiles is one team's work. Measured (us a step, phases / resident, FP32 and FP64), by nonzeros: 0.72M
+        // (937 tiles) 26.4 / 25.4, 29.2 / 25.9; 1.0M (782) 28.5 / 25.7, 32.8 / 26.8; 1.08M (1,407) 32.4 / 30.7, 34.0 / 31.6; power-law
+        // 1.2M 27.4 / 28.2, 29.4 / 29.0; 1.5M 29.1 / 28.2, 33.7 / 30.8, band of 5 22.8 / 26.0, 24.5 / 27.8; 2.0M (980) 35.8 / 35.5, 45.9
+        // / 40.2, power-law 35.1 / 41.2, 44.4 / 42.6; 3.6M (1,800) 55.9 / 56.6, 71.6 / 63.4; power-law 5.0M (2,450) 63.7 / 89.2, 77.7
+        // / 93.8; 3M (3,906) 65 / 80, 73 / 83; one row of 20,000 nonzeros 20.7 / 22.0, 22.0 / 20.7, of 100,000 57.6 / 81.6, 58.9 / 75.4.
+        const int64_t tiles = std::max(A.rnblk, AT.rnblk), teams = int64_t(kTeams) * sms;
+        const bool faster = (sizeof(T) == 4 ? tiles <= 5 * teams && A.nnz <= 2 * teams * kTile : tiles <= 8 * teams) &&
+                            std::max(A.maxrow, AT.maxrow) <= 16 * kTile;
         resident_powers = npanels[0] == 0 && (faster || mode >= 1);
         // the tuner's choice for the phases, or panels
         if (A.per_thread || AT.per_thread || tuned[0] == 2 || tuned[1] == 2 || npanels[0]) return;
         resident_iterates = mode >= 1 || std::max(A.rnblk, AT.rnblk) <= kTeams * sms;
         if (mode == 1 || A.maxrow > kTile || AT.maxrow > kTile || m > kClusterRows || n > kClusterRows) return;
-        // One cluster where its time is below the grid's, which is 4.5 to 6 us an iteration whatever the LP. Measured (grid /
-        // cluster): planted 2,000 x 5,000 (25,000 nonzeros) FP32 5.4 / 3.6, FP64 4.9 / 4.2; 3,000 x 7,500 FP32 5.4 / 4.3, FP64 5.1
-        // / 5.9; band of 60, 1,200 rows, FP32 5.9 / 15.5 (75 rows for a warp to take one after another). Beyond 90,000 bytes of x
-        // and z and nonzeros no plan comes below it.
+        // One cluster where its time is below the grid's, which is 4.8 us an iteration and 1.6 ns a nonzero of the longest rows,
+        // a warp's work. Measured (grid / cluster): planted 2,000 x 5,000 (25,000 nonzeros) FP32 5.4 / 3.6, FP64 4.9 / 4.2; 3,000 x
+        // 7,500 FP32 5.4 / 4.3, FP64 5.1 / 5.9; power-law 1,996 x 3,338 with a row of 1,547 7.3 / 5.4; band of 60, 1,200 rows,
+        // FP32 5.9 / 15.5 (75 rows for a warp of the cluster to take one after another). Beyond 90,000 bytes of x and z and
+        // nonzeros no plan comes below it.
         const char* cl = std::getenv("TARAL_CLUSTER");
         if (!cl && int64_t(m + n) * int64_t(sizeof(T)) + A.nnz > 90000) return;
         for (int q = cl ? std::atoi(cl) : cluster_size(A.nnz); q <= kClusterMax; q *= 2) {
@@ -727,7 +730,7 @@ struct Engine final : EngineBase {
             double us;
             const size_t need = cluster_plan<T>(A.hptr.data(), AT.hptr.data(), m, n, q, plan, &us);
             if (need > kClusterSmem) continue;
-            if (!cl && us > 5) return;
+            if (!cl && us > 4.8 + 1.6e-3 * double(A.maxrow + AT.maxrow)) return;
             int* d_plan = nullptr;
             if (!if_memory([&] { d_plan = alloc<int>(plan.size()), d_lp = alloc<ClusterLp<T>>(1); })) return;
             cluster_ctas = q, cluster_smem = need;

@@ -150,7 +150,7 @@ def test_launches_are_counted(engine_lib, monkeypatch, resident, block, pair):
 
 
 @pytest.mark.parametrize("precision,tiles,long,resident", [
-    (pdhg.FP32, 560, 0, True), (pdhg.FP32, 640, 0, False), (pdhg.FP64, 640, 0, True), (pdhg.FP64, 2300, 0, True),
+    (pdhg.FP32, 640, 0, True), (pdhg.FP32, 900, 0, True), (pdhg.FP32, 1000, 0, False), (pdhg.FP64, 1000, 0, True), (pdhg.FP64, 2300, 0, True),
     (pdhg.FP64, 2450, 0, False), (pdhg.FP64, 560, 33_000, False), (pdhg.FP32, 100, 25_600, True),
 ])
 def test_power_iteration_form(engine_lib, monkeypatch, precision, tiles, long, resident):
@@ -194,8 +194,9 @@ def _blocks(count, rows, cols, seed=0):
 
 @pytest.mark.parametrize("lp,precision,cluster", [
     (lambda: lpgen.planted(2000, 5000, 5, seed=1), pdhg.FP64, True), (lambda: lpgen.general(307, 701, seed=1), pdhg.FP32, True),
+    (lambda: lpgen.planted(1996, 3338, 7, seed=1, zipf=1.2, cap=2000, floor=5), pdhg.FP64, True),  # the grid is slower still
     (lambda: _blocks(4, 100, 100), pdhg.FP32, False), (lambda: _blocks(12, 70, 80), pdhg.FP32, False),
-], ids=["planted", "general", "long_rows", "many_long_rows"])
+], ids=["planted", "general", "a_very_long_row", "long_rows", "many_long_rows"])
 def test_cluster_choice(engine_lib, monkeypatch, lp, precision, cluster):
     """One LP runs on a cluster where the plan's estimate is below the grid's time, not where a warp would take many long
     rows one after another."""
